@@ -1,27 +1,35 @@
 // FFT cross-correlation shift search (reference arecCCImages,
 // AREC3D/AREC3D/arecImage.cpp:384-434 = ccorr2d + speak per image pair,
-// AREC3D/AREC3D/align2dstack.cpp:480-521, 1059-1166).
+// AREC3D/AREC3D/align2dstack.cpp:480-521, 1059-1166) and the Fourier shift
+// (fshift2d, align2dstack.cpp:566-630).
 //
 //   c = IDFT2( conj(DFT2 x) * DFT2 y )   (unnormalised, [ny][nx], real)
 //   peak = speak(c): |c| argmax with the reference's scan-order rules,
 //          3x3 paraboloid fit, wrap to (-n/2, n/2].
 //
 // Pipeline per batch of image pairs (all FP32, sizes 2..4096 whose prime
-// factors are 2, 3, 5 and 7):
+// factors are 2, 3, 5 and 7), H = nx/2+1:
 //   1. rows:    z = x + i*y, complex FFT of each row (one transform gives the
 //               row spectra of both real images), split into the half spectra
-//               Xh, Yh [ny][nx/2+1] (Hermitian symmetry).
-//   2. columns: column FFTs of Xh and Yh, C = conj(X)*Y, inverse column FFT,
-//               written back over Xh (each block owns its columns).
-//   3. rows:    Hermitian row -> inverse complex FFT -> c (real part), with
+//               S[ny][H] = (X, Y), interleaved.
+//   2. columns: column FFTs of X and Y in step, C = conj(X)*Y, inverse column
+//               FFT -> W[ny][H].
+//   3. rows:    two Hermitian rows a, b as one complex inverse FFT of
+//               A + i*B: c rows a (real part) and b (imaginary part), with
 //               per-row peak statistics fused.
 //   4. peak:    one block per pair reduces the row statistics exactly in the
 //               reference's x-major scan order and fits the paraboloid in FP64.
-// FFTs run in shared memory: Stockham passes, twiddles from a per-length table
-// computed in double on the host.  Powers of two: radix 16 and one radix-2/4/8
-// pass, one radix-16 butterfly per thread per pass held in registers; other
-// lengths: radix 16/8/4/2 and then 7/5/3 passes, each thread holding up to 16
-// elements' butterflies.
+// The Fourier shift runs the same row passes on pairs of rows of one image and
+// a column pass that multiplies the phase factor.
+//
+// The transforms (arec_fft.cuh) keep 16 points per thread in registers: a pass
+// reads its lines once and writes them once, so what is left is the traffic of
+// the three passes (36 bytes per pixel of a pair: 8 + 8 rows, 8 + 4 columns,
+// 4 + 4 rows; the Fourier shift 24).  Against Stockham passes that staged every
+// line in shared memory first and last, gathered 16 scattered twiddles per
+// butterfly and spilled (one block per SM), whole calls: 48 pairs of 2048^2
+// 9.36 -> 2.52 ms, 30 pairs of 750 x 1000 1.89 -> 0.89 ms, the shift of 180
+// images of 512^2 (then full complex spectra) 4.89 -> 0.53 ms.
 #include <math.h>
 
 #include <algorithm>
@@ -31,189 +39,17 @@
 #include <mutex>
 #include <vector>
 
+#include "arec_fft.cuh"
 #include "arec_internal.cuh"
 
 namespace arecgb {
 
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-
-// In-register radix-R DFT (forward sign) of v[off .. off+R), iterative DIT.
-template <int R>
-__device__ __forceinline__ void dft_reg(float2 *v) {
-    constexpr int LOG = R == 2 ? 1 : R == 4 ? 2 : R == 8 ? 3 : 4;
-    // cos/sin(2*pi*m/16), m = 0..7
-    const float C16[8] = {1.0f, 0.92387953251128676f, 0.70710678118654752f,
-                          0.38268343236508977f, 0.0f, -0.38268343236508977f,
-                          -0.70710678118654752f, -0.92387953251128676f};
-    const float S16[8] = {0.0f, 0.38268343236508977f, 0.70710678118654752f,
-                          0.92387953251128676f, 1.0f, 0.92387953251128676f,
-                          0.70710678118654752f, 0.38268343236508977f};
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-        int j = 0;
-#pragma unroll
-        for (int bbit = 0; bbit < LOG; bbit++) j |= ((i >> bbit) & 1) << (LOG - 1 - bbit);
-        if (i < j) {
-            float2 t = v[i];
-            v[i] = v[j];
-            v[j] = t;
-        }
-    }
-#pragma unroll
-    for (int len = 2; len <= R; len <<= 1) {
-        const int half = len >> 1;
-#pragma unroll
-        for (int s = 0; s < R; s += len) {
-#pragma unroll
-            for (int k = 0; k < half; k++) {
-                const int m = k * (16 / len);
-                const float c = C16[m], sn = S16[m];
-                const float2 a = v[s + k], b = v[s + k + half];
-                // b * exp(-2*pi*i*k/len)
-                const float2 bw = make_float2(b.x * c + b.y * sn, b.y * c - b.x * sn);
-                v[s + k] = make_float2(a.x + bw.x, a.y + bw.y);
-                v[s + k + half] = make_float2(a.x - bw.x, a.y - bw.y);
-            }
-        }
-    }
-}
-
-// Shared-memory lines are padded by one element per 16 (index i at
-// pz(i) = i + i/16, line length plen(N)): the Stockham passes write with
-// strides of 16 elements, which would otherwise fall in one bank.
-__device__ __host__ __forceinline__ int pz(int i) { return i + (i >> 4); }
-__device__ __host__ __forceinline__ int plen(int n) { return n + (n >> 4); }
-
-template <int R>
-__device__ __forceinline__ void stockham_pass(float2 *L, int N, int Ns, int b, bool active,
-                                              const float2 *__restrict__ tw) {
-    constexpr int NBT = 16 / R;
-    const int NR = N / R;
-    float2 v[16];
-    if (active) {
-#pragma unroll
-        for (int i = 0; i < NBT; i++) {
-            const int j = b * NBT + i;
-            const int k = j % Ns;
-            const int step = N / (Ns * R);
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                const float2 x = L[pz(j + r * NR)];
-                const float2 w = __ldg(&tw[(r * k * step) & (N - 1)]);
-                v[i * R + r] = cmul(x, w);
-            }
-        }
-    }
-    __syncthreads();
-    if (active) {
-#pragma unroll
-        for (int i = 0; i < NBT; i++) {
-            dft_reg<R>(v + i * R);
-            const int j = b * NBT + i;
-            const int k = j % Ns;
-            const int d = (j / Ns) * Ns * R + k;
-#pragma unroll
-            for (int r = 0; r < R; r++) L[pz(d + r * Ns)] = v[i * R + r];
-        }
-    }
-    __syncthreads();
-}
-
-// Direct DFT (forward sign) of R = 3, 5 or 7 values in registers: the
-// butterflies of the lengths with odd prime factors.  cos / sin(2 pi m / R)
-// for m <= R / 2 (the other half by symmetry).
-template <int R>
-__device__ __forceinline__ void dft_odd(float2 *v) {
-    static_assert(R == 3 || R == 5 || R == 7, "odd radices 3, 5, 7");
-    float C[R], S[R];
-    if constexpr (R == 3) {
-        C[1] = -0.5f;
-        S[1] = 0.86602540378443865f;
-    } else if constexpr (R == 5) {
-        C[1] = 0.30901699437494742f;
-        S[1] = 0.95105651629515357f;
-        C[2] = -0.80901699437494742f;
-        S[2] = 0.58778525229247313f;
-    } else {
-        C[1] = 0.62348980185873353f;
-        S[1] = 0.78183148246802981f;
-        C[2] = -0.22252093395631440f;
-        S[2] = 0.97492791218182361f;
-        C[3] = -0.90096886790241913f;
-        S[3] = 0.43388373911755812f;
-    }
-    C[0] = 1.0f;
-    S[0] = 0.0f;
-#pragma unroll
-    for (int m = 1; m <= R / 2; m++) {
-        C[R - m] = C[m];
-        S[R - m] = -S[m];
-    }
-    float2 out[R];
-#pragma unroll
-    for (int m = 0; m < R; m++) {
-        float re = v[0].x, im = v[0].y;
-#pragma unroll
-        for (int r = 1; r < R; r++) {
-            const int e = (r * m) % R;  // v_r * exp(-2 pi i r m / R)
-            re += v[r].x * C[e] + v[r].y * S[e];
-            im += v[r].y * C[e] - v[r].x * S[e];
-        }
-        out[m] = make_float2(re, im);
-    }
-#pragma unroll
-    for (int m = 0; m < R; m++) v[m] = out[m];
-}
-
-template <int R>
-__device__ __forceinline__ void dft_any(float2 *v) {
-    if constexpr (R == 3 || R == 5 || R == 7)
-        dft_odd<R>(v);
-    else
-        dft_reg<R>(v);
-}
-
-// Lines of length n per block: G * n <= 4096 elements (16 per thread).
-__device__ __host__ __forceinline__ int lines_per_block(int n) { return n >= 4096 ? 1 : 4096 / n; }
-
-// One Stockham pass of radix R over G lines of any length N (N % R == 0,
-// G * N <= 4096), every thread of the 256 holding up to ceil(16 / R)
-// butterflies: all loads (times twiddles) before a barrier, then the
-// butterflies and the stores.  Twiddle index r * k * N / (Ns * R) < N.
-template <int R>
-__device__ void mixed_pass(float2 *buf, int N, int lstride, int G, int Ns,
-                           const float2 *__restrict__ tw) {
-    constexpr int NBT = (16 + R - 1) / R;
-    const int NR = N / R, B = G * NR, step = N / (Ns * R);
-    float2 v[NBT * R];
-#pragma unroll
-    for (int i = 0; i < NBT; i++) {
-        const int t = threadIdx.x + i * 256;
-        if (t < B) {
-            const int line = t / NR, j = t % NR, k = j % Ns;
-            const float2 *L = buf + (size_t)line * lstride;
-#pragma unroll
-            for (int r = 0; r < R; r++)
-                v[i * R + r] = cmul(L[pz(j + r * NR)], __ldg(&tw[r * k * step]));
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < NBT; i++) {
-        const int t = threadIdx.x + i * 256;
-        if (t < B) {
-            dft_any<R>(v + i * R);
-            const int line = t / NR, j = t % NR, k = j % Ns;
-            float2 *L = buf + (size_t)line * lstride;
-            const int d = (j / Ns) * Ns * R + k;
-#pragma unroll
-            for (int r = 0; r < R; r++) L[pz(d + r * Ns)] = v[i * R + r];
-        }
-    }
-    __syncthreads();
-}
+using fft::FastDiv;
+using fft::fdiv;
+using fft::Passes;
+using fft::plen;
+using fft::Pow2;
+using fft::pz;
 
 // Lengths whose prime factors are 2, 3, 5 and 7 (the reference's FFTW takes any
 // length; these cover the detector and crop sizes the alignment sees).
@@ -225,175 +61,195 @@ static inline bool smooth_length(int n) {
     return n == 1;
 }
 
-// Forward FFT of G lines of a length that is not a power of two: radix 16, 8,
-// 4, 2, 7, 5, 3 passes in that order (the product of the radices done is Ns).
-__device__ void fft_lines_mixed(float2 *buf, int N, int lstride, int G, const float2 *tw) {
-    int rest = N, Ns = 1;
-    while (rest > 1) {
-        int R;
-        if (rest % 16 == 0) R = 16;
-        else if (rest % 8 == 0) R = 8;
-        else if (rest % 4 == 0) R = 4;
-        else if (rest % 2 == 0) R = 2;
-        else if (rest % 7 == 0) R = 7;
-        else if (rest % 5 == 0) R = 5;
-        else R = 3;
-        switch (R) {
-            case 16: mixed_pass<16>(buf, N, lstride, G, Ns, tw); break;
-            case 8: mixed_pass<8>(buf, N, lstride, G, Ns, tw); break;
-            case 4: mixed_pass<4>(buf, N, lstride, G, Ns, tw); break;
-            case 2: mixed_pass<2>(buf, N, lstride, G, Ns, tw); break;
-            case 7: mixed_pass<7>(buf, N, lstride, G, Ns, tw); break;
-            case 5: mixed_pass<5>(buf, N, lstride, G, Ns, tw); break;
-            default: mixed_pass<3>(buf, N, lstride, G, Ns, tw); break;
+// Lines of length n per block of the row passes (16 points per thread).
+__device__ __host__ __forceinline__ int lines_per_block(int n) {
+    return n >= fft::kElems ? 1 : fft::kElems / n;
+}
+static inline bool pow2_length(int n) { return n >= 16 && (n & (n - 1)) == 0; }
+// Columns per block of a column pass over points of `w` bytes: the largest
+// power of two with 4096 points per block; the run-time lengths hold two
+// buffers and take 4096 points of 8 bytes or 2048 of 16 (about 70 KB, three
+// blocks per SM).
+static inline int col_tile(int ny, int w) {
+    const int cap = pow2_length(ny) || w == 8 ? fft::kElems : fft::kElems / 2;
+    int ct = 1;
+    while (2 * ct * ny <= cap) ct *= 2;
+    return ct;
+}
+// Stride between a column tile's lines in shared memory, in points of `w`
+// bytes (u of them in 128 bytes): a warp reads ct lines x 32/ct consecutive
+// points, so the lines start u / ct points apart modulo u; tiles of u lines or
+// more take any odd stride.
+__device__ __host__ __forceinline__ constexpr int col_stride(int n, int ct, int w) {
+    const int u = 128 / w;
+    return ct < u ? (plen(n) + u - 1) / u * u + u / ct : (plen(n) | 1);
+}
+
+// What a row pass transforms: pairs of images (shift search) or pairs of rows
+// of one image (Fourier shift).
+enum RowMode { kPairs = 0, kRows = 1 };
+
+// ---------------------------------------------------------------------------
+// Row passes, forward.  kPairs: z = x + i y per row, S[row][k] = (X, Y) as one
+// float4.  kRows: z = row 2l + i row 2l+1, F[row][k] as float2.
+// N > 0: a power of two; N = 0: `P`'s run-time length.
+struct RowSpectra {
+    float4 *S;   // kPairs: [nz][ny][H]
+    float2 *F;   // kRows:  [nz][ny][H]
+};
+
+template <int MODE>
+__device__ __forceinline__ void store_split(const RowSpectra &o, size_t img_row, int row, int ny,
+                                            int H, int k, float2 Z, float2 Zm) {
+    const float2 X = make_float2(0.5f * (Z.x + Zm.x), 0.5f * (Z.y - Zm.y));
+    const float2 Y = make_float2(0.5f * (Z.y + Zm.y), -0.5f * (Z.x - Zm.x));
+    if constexpr (MODE == kPairs) {
+        o.S[img_row * H + k] = make_float4(X.x, X.y, Y.x, Y.y);
+    } else {
+        o.F[img_row * H + k] = X;
+        if (row + 1 < ny) o.F[(img_row + 1) * H + k] = Y;
+    }
+}
+
+template <int N, int MODE>
+__global__ void __launch_bounds__(fft::kThreads, 3)
+    k_rows_fwd(const float *__restrict__ x, const float *__restrict__ y, RowSpectra o, int nx,
+               int ny, Passes P, FastDiv dH, const float2 *__restrict__ tw) {
+    extern __shared__ float4 sm4[];
+    float2 *sm = reinterpret_cast<float2 *>(sm4);
+    const int n = N > 0 ? N : nx, H = n / 2 + 1;
+    const int G = N > 0 ? Pow2<N ? N : 16>::G : lines_per_block(n);
+    const int line0 = blockIdx.x * G, LS = plen(n);
+    const size_t img = (size_t)blockIdx.y * ny;  // first row of the image
+    const float *xi = x + img * n, *yi = MODE == kPairs ? y + img * n : x + img * n;
+    auto load = [&](int line, int i) -> float2 {
+        const int l = line0 + line;
+        if constexpr (MODE == kPairs)
+            return l < ny ? make_float2(xi[(size_t)l * n + i], yi[(size_t)l * n + i])
+                          : make_float2(0.f, 0.f);
+        else
+            return make_float2(2 * l < ny ? xi[(size_t)(2 * l) * n + i] : 0.f,
+                               2 * l + 1 < ny ? xi[(size_t)(2 * l + 1) * n + i] : 0.f);
+    };
+    if constexpr (N > 0) {
+        using L2 = Pow2<N>;
+        constexpr int TPL = L2::TPL, Ra = L2::template radix<false>(0);
+        constexpr int Rl = L2::template radix<false>(L2::P - 1);
+        constexpr bool WARP = TPL <= 32;
+        const int line = threadIdx.x / TPL, b = threadIdx.x % TPL;
+        float2 *L = sm + (size_t)line * LS;
+        float2 v[1][16];
+#pragma unroll
+        for (int i = 0; i < 16 / Ra; i++)
+#pragma unroll
+            for (int r = 0; r < Ra; r++) v[0][i * Ra + r] = load(line, b + i * TPL + r * (N / Ra));
+        fft::transform<N, false, WARP, 1>(v, L, b, tw);
+        fft::exchange_sync<WARP>();
+#pragma unroll
+        for (int i = 0; i < 16 / Rl; i++)
+#pragma unroll
+            for (int r = 0; r < Rl; r++) L[pz(b + i * TPL + r * (N / Rl))] = v[0][i * Rl + r];
+        fft::exchange_sync<WARP>();
+        const int row = MODE == kPairs ? line0 + line : 2 * (line0 + line);
+        if (row >= ny) return;
+#pragma unroll
+        for (int i = 0; i < 16 / Rl; i++)
+#pragma unroll
+            for (int r = 0; r <= Rl / 2; r++) {
+                const int j = b + i * TPL, k = j + r * (N / Rl);
+                if (r < Rl / 2 || j == 0)
+                    store_split<MODE>(o, img + row, row, ny, H, k, v[0][i * Rl + r],
+                                      L[pz((N - k) & (N - 1))]);
+            }
+    } else {
+        fft::mixed_fill<false>(n, P.dn, G, 0, sm, LS, load);
+        const float2 *z = fft::mixed_transform<1, false>(P, G, 0, sm, sm + G * LS, LS, tw);
+        for (int t = threadIdx.x; t < G * H; t += fft::kThreads) {
+            const int line = fdiv(t, dH), k = t - line * H;
+            const int row = MODE == kPairs ? line0 + line : 2 * (line0 + line);
+            if (row < ny)
+                store_split<MODE>(o, img + row, row, ny, H, k, z[line * LS + pz(k)],
+                                  z[line * LS + pz(k ? n - k : 0)]);
         }
-        Ns *= R;
-        rest /= R;
     }
-}
-
-// In-place forward FFT of G lines of length N (power of two, 16..4096; G * N
-// <= 4096) held in shared memory at buf + l*lstride (padded lines: element i
-// at pz(i)).  N/16 threads per line, one radix-16 butterfly per thread per
-// pass; all threads of the block must call it.
-__device__ void fft_lines(float2 *buf, int N, int lstride, int G, const float2 *tw) {
-    const int tpl = N / 16;
-    const int line = threadIdx.x / tpl, b = threadIdx.x % tpl;
-    const bool active = line < G;
-    float2 *L = buf + (size_t)(active ? line : 0) * lstride;
-    for (int Ns = 1; Ns < N;) {
-        const int R = min(16, N / Ns);
-        if (R == 16) stockham_pass<16>(L, N, Ns, b, active, tw);
-        else if (R == 8) stockham_pass<8>(L, N, Ns, b, active, tw);
-        else if (R == 4) stockham_pass<4>(L, N, Ns, b, active, tw);
-        else stockham_pass<2>(L, N, Ns, b, active, tw);
-        Ns *= R;
-    }
-}
-
-// The kernels below are instantiated twice: MIXED = false for power-of-two
-// lengths (fft_lines), true for the other lengths (fft_lines_mixed), so the
-// power-of-two kernels keep their own register allocation.
-template <bool MIXED>
-__device__ __forceinline__ void fft_any(float2 *buf, int N, int lstride, int G, const float2 *tw) {
-    if constexpr (MIXED)
-        fft_lines_mixed(buf, N, lstride, G, tw);
-    else
-        fft_lines(buf, N, lstride, G, tw);
 }
 
 // ---------------------------------------------------------------------------
+// Column pass of the shift search: ct columns of S per block; W = IDFT_col(
+// conj(X)*Y).  The inverse transform starts on the registers the forward ones
+// end with (its radices in reversed order).
+__device__ __forceinline__ float2 conj_product(float2 a, float2 b) {
+    // conj(conj(a) * b): the inverse transform is conj DFT conj
+    return make_float2(a.x * b.x + a.y * b.y, -(a.x * b.y - a.y * b.x));
+}
+
+template <int N>
+__global__ void __launch_bounds__(fft::kThreads, 2)
+    k_cc_cols(const float4 *__restrict__ S, float2 *__restrict__ W, int nx, int ny, int ct, int lg,
+              Passes P, const float2 *__restrict__ tw, const float2 *__restrict__ twr) {
+    extern __shared__ float4 sm4[];
+    float2 *sm2 = reinterpret_cast<float2 *>(sm4);
+    const int n = N > 0 ? N : ny, H = nx / 2 + 1;
+    const int c0 = blockIdx.x * ct;
+    const size_t img = (size_t)blockIdx.y * n;
+    const int LS4 = col_stride(n, ct, 16), LS2 = col_stride(n, ct, 8);
+    auto load = [&](int c, int row) -> float4 {
+        return c0 + c < H ? S[(img + row) * H + c0 + c] : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    if constexpr (N > 0) {
+        using L2 = Pow2<N>;
+        constexpr int TPL = L2::TPL, CT = L2::G;
+        constexpr int Ra = L2::template radix<false>(0), Rl = L2::template radix<false>(L2::P - 1);
+        const int c = threadIdx.x % CT, b = threadIdx.x / CT;
+        float2 v[2][16];
+#pragma unroll
+        for (int i = 0; i < 16 / Ra; i++)
+#pragma unroll
+            for (int r = 0; r < Ra; r++) {
+                const float4 q = load(c, b + i * TPL + r * (N / Ra));
+                v[0][i * Ra + r] = make_float2(q.x, q.y);
+                v[1][i * Ra + r] = make_float2(q.z, q.w);
+            }
+        fft::transform<N, false, false, 2>(v, sm4 + c * LS4, b, tw);
+        float2 w[1][16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) w[0][i] = conj_product(v[0][i], v[1][i]);
+        __syncthreads();  // the lines' layout changes
+        fft::transform<N, true, false, 1>(w, sm2 + c * LS2, b, twr);
+        if (c0 + c >= H) return;
+        (void)Rl;
+#pragma unroll
+        for (int i = 0; i < 16 / Ra; i++)
+#pragma unroll
+            for (int r = 0; r < Ra; r++) {
+                const float2 z = w[0][i * Ra + r];
+                W[(img + b + i * TPL + r * (N / Ra)) * H + c0 + c] = make_float2(z.x, -z.y);
+            }
+    } else {
+        fft::mixed_fill<true>(n, P.dn, ct, lg, sm4, LS4, load);
+        float4 *z4 = fft::mixed_transform<2, true>(P, ct, lg, sm4, sm4 + ct * LS4, LS4, tw);
+        // the products stay in the slots of X (the inverse transform strides
+        // over float4 slots)
+        for (int t = threadIdx.x; t < ct * n; t += fft::kThreads) {
+            float4 &q = z4[(t & (ct - 1)) * LS4 + pz(t >> lg)];
+            const float2 z = conj_product(make_float2(q.x, q.y), make_float2(q.z, q.w));
+            q.x = z.x;
+            q.y = z.y;
+        }
+        __syncthreads();
+        z4 = fft::mixed_transform<1, true>(P, ct, lg, z4, z4 == sm4 ? sm4 + ct * LS4 : sm4, LS4, tw);
+        fft::mixed_drain<true>(n, P.dn, ct, lg, z4, LS4, [&](int c, int i, float4 z) {
+            if (c0 + c < H) W[(img + i) * H + c0 + c] = make_float2(z.x, -z.y);
+        });
+    }
+}
+
 struct RowStat {
     float m;   // max |c| over the row
     int xpos;  // first x with c == +m (INT_MAX if none)
     int xneg;  // last x with c == -m (-1 if none)
     int pad;
 };
-
-// Global loads per thread issued together before their shared-memory stores
-// (a block stages 4096 elements: 16 per thread in one batch).  The three
-// passes are capped at 128 registers (two blocks per SM): the radix-16
-// butterflies spill a little, which costs less than running one block per SM.
-constexpr int kLoadBatch = 16;
-
-// Pass 1: rows of z = x + i*y -> half spectra of x and y.
-template <bool MIXED>
-__global__ void __launch_bounds__(256, 2) k_cc_rows_fwd(const float *__restrict__ x,
-                                                     const float *__restrict__ y,
-                                                     float2 *__restrict__ Xh,
-                                                     float2 *__restrict__ Yh, int nx, int ny,
-                                                     const float2 *__restrict__ tw) {
-    extern __shared__ float2 sm[];
-    const int G = lines_per_block(nx);
-    const int row0 = blockIdx.x * G, pair = blockIdx.y;
-    const int H = nx / 2 + 1;
-    const size_t img = (size_t)pair * nx * ny;
-    // all of a thread's loads issued before any store (G * nx = 4096: 16 each)
-    for (int i0 = 0; i0 < G * nx; i0 += kLoadBatch * 256) {
-        float2 z[kLoadBatch];
-#pragma unroll
-        for (int e = 0; e < kLoadBatch; e++) {
-            const int i = i0 + e * 256 + threadIdx.x, l = i / nx, c = i % nx, row = row0 + l;
-            z[e] = make_float2(0.f, 0.f);
-            if (i < G * nx && row < ny)
-                z[e] = make_float2(x[img + (size_t)row * nx + c], y[img + (size_t)row * nx + c]);
-        }
-#pragma unroll
-        for (int e = 0; e < kLoadBatch; e++) {
-            const int i = i0 + e * 256 + threadIdx.x, l = i / nx, c = i % nx;
-            if (i < G * nx) sm[l * plen(nx) + pz(c)] = z[e];
-        }
-    }
-    __syncthreads();
-    fft_any<MIXED>(sm, nx, plen(nx), G, tw);
-    const size_t half = (size_t)pair * ny * H;
-    for (int i = threadIdx.x; i < G * H; i += blockDim.x) {
-        const int l = i / H, k = i % H, row = row0 + l;
-        if (row >= ny) continue;
-        const float2 Z = sm[l * plen(nx) + pz(k)], Zm = sm[l * plen(nx) + pz(k ? nx - k : 0)];
-        Xh[half + (size_t)row * H + k] = make_float2(0.5f * (Z.x + Zm.x), 0.5f * (Z.y - Zm.y));
-        Yh[half + (size_t)row * H + k] = make_float2(0.5f * (Z.y + Zm.y), -0.5f * (Z.x - Zm.x));
-    }
-}
-
-// Pass 2: columns.  ct columns of Xh and Yh per block (ct = col_tile(ny): the
-// two arrays' ct columns stay within 64 KB of shared memory, so several blocks
-// share an SM); W = IDFT_col(conj(X)*Y) overwrites Xh.
-constexpr int kColTile = 4;
-static inline int col_tile(int ny) { return ny <= 1024 ? 4 : (ny <= 2048 ? 2 : 1); }
-template <bool MIXED>
-__global__ void __launch_bounds__(256, 2) k_cc_cols(float2 *__restrict__ Xh,
-                                                 const float2 *__restrict__ Yh, int nx, int ny,
-                                                 const float2 *__restrict__ tw, int ct) {
-    extern __shared__ float2 sm[];
-    const int H = nx / 2 + 1;
-    const int c0 = blockIdx.x * ct, pair = blockIdx.y;
-    const int nc = min(ct, H - c0);
-    const size_t half = (size_t)pair * ny * H;
-    const int PN = plen(ny);
-    float2 *sx = sm, *sy = sm + ct * PN;
-    for (int i0 = 0; i0 < ct * ny; i0 += kLoadBatch * 256) {
-        float2 a[kLoadBatch], b[kLoadBatch];
-#pragma unroll
-        for (int e = 0; e < kLoadBatch; e++) {
-            const int i = i0 + e * 256 + threadIdx.x, row = i / ct, c = i % ct;
-            a[e] = b[e] = make_float2(0.f, 0.f);
-            if (i < ct * ny && c < nc) {
-                a[e] = Xh[half + (size_t)row * H + c0 + c];
-                b[e] = Yh[half + (size_t)row * H + c0 + c];
-            }
-        }
-#pragma unroll
-        for (int e = 0; e < kLoadBatch; e++) {
-            const int i = i0 + e * 256 + threadIdx.x, row = i / ct, c = i % ct;
-            if (i < ct * ny) {
-                sx[c * PN + pz(row)] = a[e];
-                sy[c * PN + pz(row)] = b[e];
-            }
-        }
-    }
-    __syncthreads();
-    const int G = lines_per_block(ny);
-    for (int l0 = 0; l0 < 2 * ct; l0 += G)
-        fft_any<MIXED>(sm + (size_t)l0 * PN, ny, PN, min(G, 2 * ct - l0), tw);
-    // conj(X)*Y, conjugated again for the inverse transform (IDFT = conj DFT conj)
-    for (int i = threadIdx.x; i < ct * ny; i += blockDim.x) {
-        const int c = i / ny, row = i % ny, o = c * PN + pz(row);
-        const float2 a = sx[o], b = sy[o];
-        const float2 cc = make_float2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
-        sx[o] = make_float2(cc.x, -cc.y);
-    }
-    __syncthreads();
-    for (int l0 = 0; l0 < ct; l0 += G)
-        fft_any<MIXED>(sm + (size_t)l0 * PN, ny, PN, min(G, ct - l0), tw);
-    for (int i = threadIdx.x; i < ct * ny; i += blockDim.x) {
-        const int row = i / ct, c = i % ct;
-        if (c < nc) {
-            const float2 w = sx[c * PN + pz(row)];
-            Xh[half + (size_t)row * H + c0 + c] = make_float2(w.x, -w.y);
-        }
-    }
-}
 
 // Combine two row statistics in favour of the reference's scan order.
 __device__ __forceinline__ RowStat stat_merge(RowStat a, RowStat b) {
@@ -405,64 +261,156 @@ __device__ __forceinline__ RowStat stat_merge(RowStat a, RowStat b) {
     return r;
 }
 
-// Pass 3: inverse row transforms -> c rows, with per-row peak statistics.
-template <bool MIXED>
-__global__ void __launch_bounds__(256, 2) k_cc_rows_inv(const float2 *__restrict__ Wh,
-                                                     float *__restrict__ c, RowStat *stats,
-                                                     int nx, int ny,
-                                                     const float2 *__restrict__ tw) {
-    extern __shared__ float2 sm[];
-    const int G = lines_per_block(nx);
-    const int row0 = blockIdx.x * G, pair = blockIdx.y;
-    const int H = nx / 2 + 1;
-    const size_t half = (size_t)pair * ny * H;
-    for (int i0 = 0; i0 < G * nx; i0 += kLoadBatch * 256) {
-        float2 w[kLoadBatch];
+// The statistics of one value at x (NaN never wins).
+__device__ __forceinline__ RowStat stat_of(float v, int x) {
+    const float a = fabsf(v);
+    if (!(a == a)) return RowStat{-1.0f, INT_MAX, -1, 0};
+    return RowStat{a, v == a ? x : INT_MAX, v == -a && v != a ? x : -1, 0};
+}
+
+__device__ __forceinline__ RowStat stat_warp(RowStat s) {
+    for (int o = 16; o > 0; o >>= 1) {
+        RowStat t;
+        t.m = __shfl_down_sync(0xffffffffu, s.m, o);
+        t.xpos = __shfl_down_sync(0xffffffffu, s.xpos, o);
+        t.xneg = __shfl_down_sync(0xffffffffu, s.xneg, o);
+        t.pad = 0;
+        s = stat_merge(s, t);
+    }
+    return s;
+}
+
+// ---------------------------------------------------------------------------
+// Row passes, inverse: rows a = 2l and b = 2l+1 of the half spectra W as one
+// complex transform of A + i B (A, B real: their spectra Hermitian, so the
+// zero and Nyquist terms are real).  kPairs: c rows and their peak
+// statistics; kRows: out rows divided by nx*ny.
+template <int N, int MODE>
+__global__ void __launch_bounds__(fft::kThreads, 3)
+    k_rows_inv(const float2 *__restrict__ W, float *__restrict__ c, RowStat *__restrict__ stats,
+               int nx, int ny, Passes P, const float2 *__restrict__ tw) {
+    extern __shared__ float4 sm4[];
+    float2 *sm = reinterpret_cast<float2 *>(sm4);
+    __shared__ unsigned s_m[512];
+    __shared__ int s_pos[512], s_neg[512];
+    const int n = N > 0 ? N : nx, H = n / 2 + 1;
+    const int G = N > 0 ? Pow2<N ? N : 16>::G : lines_per_block(n);
+    const int line0 = blockIdx.x * G, LS = plen(n);
+    const size_t img = (size_t)blockIdx.y * ny;
+    const float scale = (float)(nx * ny);
+    auto load = [&](int line, int i) -> float2 {
+        const int row = 2 * (line0 + line);
+        const bool up = 2 * i > n;  // conj(Z[n - i]) of the Hermitian rows
+        const int k = up ? n - i : i;
+        const float2 *w = W + (img + row) * H + k;
+        float2 a = row < ny ? w[0] : make_float2(0.f, 0.f);
+        float2 b = row + 1 < ny ? w[H] : make_float2(0.f, 0.f);
+        if (i == 0 || 2 * i == n) a.y = b.y = 0.f;
+        // conj(A + i B): the inverse transform is conj DFT conj
+        return up ? make_float2(a.x + b.y, a.y - b.x) : make_float2(a.x - b.y, -(a.y + b.x));
+    };
+    if constexpr (N > 0) {
+        using L2 = Pow2<N>;
+        constexpr int TPL = L2::TPL, Ra = L2::template radix<false>(0);
+        constexpr int Rl = L2::template radix<false>(L2::P - 1);
+        const int line = threadIdx.x / TPL, b = threadIdx.x % TPL;
+        float2 v[1][16];
 #pragma unroll
-        for (int e = 0; e < kLoadBatch; e++) {
-            const int i = i0 + e * 256 + threadIdx.x, l = i / nx, k = i % nx, row = row0 + l;
-            w[e] = make_float2(0.f, 0.f);
-            if (i < G * nx && row < ny) {
-                if (k < H) {
-                    w[e] = Wh[half + (size_t)row * H + k];
-                    w[e].y = -w[e].y;  // conj for the inverse
-                } else {
-                    w[e] = Wh[half + (size_t)row * H + (nx - k)];  // conj(conj(W[nx-k]))
+        for (int i = 0; i < 16 / Ra; i++)
+#pragma unroll
+            for (int r = 0; r < Ra; r++) v[0][i * Ra + r] = load(line, b + i * TPL + r * (N / Ra));
+        fft::transform<N, false, (TPL <= 32), 1>(v, sm + (size_t)line * LS, b, tw);
+        const int row = 2 * (line0 + line);
+        const bool ra = row < ny, rb = row + 1 < ny;
+        float *ca = c + (img + row) * n;
+        if constexpr (MODE == kRows) {
+#pragma unroll
+            for (int i = 0; i < 16 / Rl; i++)
+#pragma unroll
+                for (int r = 0; r < Rl; r++) {
+                    const int x = b + i * TPL + r * (N / Rl);
+                    const float2 z = v[0][i * Rl + r];
+                    if (ra) ca[x] = z.x / scale;
+                    if (rb) ca[n + x] = -z.y / scale;
                 }
+        } else {
+            // per row: max |c| (as an ordered integer; NaN never wins), then
+            // the first x of +max and the last of -max
+            for (int t = threadIdx.x; t < 2 * G; t += fft::kThreads) {
+                s_m[t] = 0u;
+                s_pos[t] = INT_MAX;
+                s_neg[t] = -1;
+            }
+            unsigned ma = 0u, mb = 0u;
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const unsigned ua = __float_as_uint(fabsf(v[0][i].x));
+                const unsigned ub = __float_as_uint(fabsf(v[0][i].y));
+                ma = max(ma, ua > 0x7f800000u ? 0u : ua);
+                mb = max(mb, ub > 0x7f800000u ? 0u : ub);
+            }
+            if constexpr (TPL >= 32) {
+                ma = __reduce_max_sync(0xffffffffu, ma);
+                mb = __reduce_max_sync(0xffffffffu, mb);
+            }
+            __syncthreads();
+            if (TPL < 32 || (threadIdx.x & 31) == 0) {
+                atomicMax(&s_m[2 * line], ma);
+                atomicMax(&s_m[2 * line + 1], mb);
+            }
+            __syncthreads();
+            const unsigned Ma = s_m[2 * line], Mb = s_m[2 * line + 1];
+#pragma unroll
+            for (int i = 0; i < 16 / Rl; i++)
+#pragma unroll
+                for (int r = 0; r < Rl; r++) {
+                    const int x = b + i * TPL + r * (N / Rl);
+                    const float va = v[0][i * Rl + r].x, vb = -v[0][i * Rl + r].y;
+                    if (ra) ca[x] = va;
+                    if (rb) ca[n + x] = vb;
+                    if (__float_as_uint(fabsf(va)) == Ma) {
+                        if (va == fabsf(va)) atomicMin(&s_pos[2 * line], x);
+                        else atomicMax(&s_neg[2 * line], x);
+                    }
+                    if (__float_as_uint(fabsf(vb)) == Mb) {
+                        if (vb == fabsf(vb)) atomicMin(&s_pos[2 * line + 1], x);
+                        else atomicMax(&s_neg[2 * line + 1], x);
+                    }
+                }
+            __syncthreads();
+            for (int t = threadIdx.x; t < 2 * G; t += fft::kThreads)
+                if (2 * line0 + t < ny)
+                    stats[img + 2 * line0 + t] =
+                        RowStat{__uint_as_float(s_m[t]), s_pos[t], s_neg[t], 0};
+        }
+    } else {
+        fft::mixed_fill<false>(n, P.dn, G, 0, sm, LS, load);
+        const float2 *zs = fft::mixed_transform<1, false>(P, G, 0, sm, sm + G * LS, LS, tw);
+        if constexpr (MODE == kRows) {
+            fft::mixed_drain<false>(n, P.dn, G, 0, zs, LS, [&](int line, int i, float2 z) {
+                const int row = 2 * (line0 + line);
+                float *ca = c + (img + row) * n + i;
+                if (row < ny) ca[0] = z.x / scale;
+                if (row + 1 < ny) ca[n] = -z.y / scale;
+            });
+        } else {
+            // one warp per row: store it and take its statistics
+            const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            const float *sf = reinterpret_cast<const float *>(zs);
+            for (int t = warp; t < 2 * G; t += fft::kThreads / 32) {
+                const int row = 2 * line0 + t;
+                if (row >= ny) continue;
+                RowStat s{-1.0f, INT_MAX, -1, 0};
+                for (int i = lane; i < n; i += 32) {
+                    const float z = sf[2 * ((t >> 1) * LS + pz(i)) + (t & 1)];
+                    const float v = t & 1 ? -z : z;
+                    c[(img + row) * n + i] = v;
+                    s = stat_merge(s, stat_of(v, i));
+                }
+                s = stat_warp(s);
+                if (lane == 0) stats[img + row] = s;
             }
         }
-#pragma unroll
-        for (int e = 0; e < kLoadBatch; e++) {
-            const int i = i0 + e * 256 + threadIdx.x, l = i / nx, k = i % nx;
-            if (i < G * nx) sm[l * plen(nx) + pz(k)] = w[e];
-        }
-    }
-    __syncthreads();
-    fft_any<MIXED>(sm, nx, plen(nx), G, tw);
-    // one warp per row for the statistics
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t img = (size_t)pair * nx * ny;
-    for (int l = warp; l < G; l += blockDim.x / 32) {
-        const int row = row0 + l;
-        if (row >= ny) continue;
-        RowStat s{-1.0f, INT_MAX, -1, 0};
-        for (int i = lane; i < nx; i += 32) {
-            const float v = sm[l * plen(nx) + pz(i)].x;
-            if (c) c[img + (size_t)row * nx + i] = v;
-            const float a = fabsf(v);
-            RowStat t{a, v == a && a == a ? i : INT_MAX, v == -a && v != a ? i : -1, 0};
-            if (!(a == a)) t = RowStat{-1.0f, INT_MAX, -1, 0};  // NaN never wins
-            s = stat_merge(s, t);
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            RowStat t;
-            t.m = __shfl_down_sync(0xffffffffu, s.m, o);
-            t.xpos = __shfl_down_sync(0xffffffffu, s.xpos, o);
-            t.xneg = __shfl_down_sync(0xffffffffu, s.xneg, o);
-            t.pad = 0;
-            s = stat_merge(s, t);
-        }
-        if (lane == 0) stats[(size_t)pair * ny + row] = s;
     }
 }
 
@@ -474,21 +422,8 @@ __global__ void __launch_bounds__(256) k_row_stats(const float *__restrict__ c, 
     if (row >= ny) return;
     const float *cr = c + ((size_t)pair * ny + row) * nx;
     RowStat s{-1.0f, INT_MAX, -1, 0};
-    for (int i = lane; i < nx; i += 32) {
-        const float v = cr[i];
-        const float a = fabsf(v);
-        RowStat t{a, v == a ? i : INT_MAX, (v == -a && v != a) ? i : -1, 0};
-        if (!(a == a)) t = RowStat{-1.0f, INT_MAX, -1, 0};
-        s = stat_merge(s, t);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        RowStat t;
-        t.m = __shfl_down_sync(0xffffffffu, s.m, o);
-        t.xpos = __shfl_down_sync(0xffffffffu, s.xpos, o);
-        t.xneg = __shfl_down_sync(0xffffffffu, s.xneg, o);
-        t.pad = 0;
-        s = stat_merge(s, t);
-    }
+    for (int i = lane; i < nx; i += 32) s = stat_merge(s, stat_of(cr[i], i));
+    s = stat_warp(s);
     if (lane == 0) stats[(size_t)pair * ny + row] = s;
 }
 
@@ -604,140 +539,218 @@ __global__ void __launch_bounds__(256) k_peak(const float *__restrict__ c,
 }
 
 // ---------------------------------------------------------------------------
-// Fourier shift (fshift2d, align2dstack.cpp:566-630) of a stack of images:
+// Fourier shift (fshift2d) of a stack of images:
 //   out = Re(IDFT2(DFT2(in) * exp(i * phase))) / (nx * ny),
-//   phase = -2 pi (sx kx + sy ky) in the reference's precisions: the frequencies
-//   and sx*kx + sy*ky in float, the product with 2 pi in double rounded to a
-//   float, then the float cosine and sine (cos/sin of a float resolve to the
-//   float overloads) and a float complex product.  Full complex transforms, as
-//   the reference's: at the Nyquist frequencies the factor is not conjugate
-//   symmetric and only the real part is kept.
+//   phase = -2 pi (sx kx + sy ky), frequencies -1/2 at an even length's middle.
+// The images are real, so the half spectrum H = nx/2+1 carries everything;
+// keeping only the real part of the result is the factor's Hermitian part:
+// the factor itself except at the middle frequencies of even lengths, where
+// the reference's factor is not conjugate symmetric and its average with the
+// conjugate at the mirrored frequency stands in.  The factor is a product
+// ex[kx] ey[ky]: one table per image, each entry from an exactly reduced
+// argument (the reference rounds the whole phase to float).
 
-// Pass 1: real rows -> complex spectra of the rows.
-template <bool MIXED>
-__global__ void __launch_bounds__(256) k_fs_rows(const float *__restrict__ in,
-                                                 float2 *__restrict__ C, int nx, int ny,
-                                                 const float2 *__restrict__ tw) {
-    extern __shared__ float2 sm[];
-    const int G = lines_per_block(nx);
-    const int row0 = blockIdx.x * G;
-    const size_t img = (size_t)blockIdx.y * nx * ny;
-    for (int i = threadIdx.x; i < G * nx; i += blockDim.x) {
-        const int l = i / nx, c = i % nx, row = row0 + l;
-        sm[l * plen(nx) + pz(c)] = make_float2(row < ny ? in[img + (size_t)row * nx + c] : 0.f, 0.f);
-    }
-    __syncthreads();
-    fft_any<MIXED>(sm, nx, plen(nx), G, tw);
-    for (int i = threadIdx.x; i < G * nx; i += blockDim.x) {
-        const int l = i / nx, c = i % nx, row = row0 + l;
-        if (row < ny) C[img + (size_t)row * nx + c] = sm[l * plen(nx) + pz(c)];
-    }
+// ex[0..H), ey[0..ny) of every image: exp(-2 pi i s k / n).
+__global__ void k_fs_phase(const float *__restrict__ sxs, const float *__restrict__ sys, int nx,
+                           int ny, float2 *__restrict__ tab) {
+    const int H = nx / 2 + 1, i = blockIdx.x * blockDim.x + threadIdx.x, z = blockIdx.y;
+    if (i >= H + ny) return;
+    const int n = i < H ? nx : ny, j = i < H ? i : i - H;
+    const float s = i < H ? sxs[z] : sys[z];
+    const float k = (float)(j < (n + 1) / 2 ? j : j - n);
+    // s k / n modulo 1: s k as an exact float pair, whole turns taken off exactly
+    const float p = __fmul_rn(s, k), pe = __fmaf_rn(s, k, -p);
+    const float r = __fadd_rn(__fmaf_rn(-rintf(p / (float)n), (float)n, p), pe);
+    float sn, cs;
+    sincospif(-2.f * (r / (float)n), &sn, &cs);
+    tab[(size_t)z * (H + ny) + i] = make_float2(cs, sn);
 }
 
-__device__ __forceinline__ float fs_freq(int i, int n) {
-    const int h = (n + 1) / 2;  // ceil(n / 2)
-    return i < h ? (float)i / (float)n : (float)(i - n) / (float)n;
+__device__ __forceinline__ float2 fs_apply(float2 f, float2 ex, float2 ey, bool mx, bool my) {
+    float2 e = fft::cmul(ex, ey);
+    if (mx || my) {
+        if (mx && my) e.y = 0.f;
+        else if (mx) e = make_float2(ex.x * ey.x, ex.x * ey.y);
+        else e = make_float2(ex.x * ey.x, ex.y * ey.x);
+    }
+    const float2 g = fft::cmul(f, e);
+    return make_float2(g.x, -g.y);  // conjugated: IDFT = conj(DFT(conj))
 }
 
-// Pass 2: column transforms, the phase factor, inverse column transforms.
-template <bool MIXED>
-__global__ void __launch_bounds__(256) k_fs_cols(float2 *__restrict__ C, int nx, int ny,
-                                                 const float *__restrict__ sxs,
-                                                 const float *__restrict__ sys,
-                                                 const float2 *__restrict__ tw) {
-    extern __shared__ float2 sm[];
-    const int c0 = blockIdx.x * kColTile;
-    const size_t img = (size_t)blockIdx.y * nx * ny;
-    const float sx = sxs[blockIdx.y], sy = sys[blockIdx.y];
-    const double two_pi = 2.0 * 3.14159265358979323846;
-    const int PN = plen(ny);
-    for (int i = threadIdx.x; i < kColTile * ny; i += blockDim.x) {
-        const int row = i / kColTile, c = i % kColTile;
-        sm[c * PN + pz(row)] = c0 + c < nx ? C[img + (size_t)row * nx + c0 + c] : make_float2(0.f, 0.f);
-    }
-    __syncthreads();
-    const int G = lines_per_block(ny);
-    for (int l0 = 0; l0 < kColTile; l0 += G)
-        fft_any<MIXED>(sm + (size_t)l0 * PN, ny, PN, min(G, kColTile - l0), tw);
-    for (int i = threadIdx.x; i < kColTile * ny; i += blockDim.x) {
-        const int c = i / ny, row = i % ny, o = c * PN + pz(row);
-        const float t = __fadd_rn(__fmul_rn(sx, fs_freq(c0 + c, nx)), __fmul_rn(sy, fs_freq(row, ny)));
-        const float ph = (float)(-two_pi * (double)t);
-        float sn, cs;
-        sincosf(ph, &sn, &cs);
-        const float2 f = sm[o];
-        const float re = __fsub_rn(__fmul_rn(f.x, cs), __fmul_rn(f.y, sn));
-        const float im = __fadd_rn(__fmul_rn(f.x, sn), __fmul_rn(f.y, cs));
-        sm[o] = make_float2(re, -im);  // conjugated: IDFT = conj(DFT(conj))
-    }
-    __syncthreads();
-    for (int l0 = 0; l0 < kColTile; l0 += G)
-        fft_any<MIXED>(sm + (size_t)l0 * PN, ny, PN, min(G, kColTile - l0), tw);
-    for (int i = threadIdx.x; i < kColTile * ny; i += blockDim.x) {
-        const int row = i / kColTile, c = i % kColTile;
-        const float2 w = sm[c * PN + pz(row)];
-        if (c0 + c < nx) C[img + (size_t)row * nx + c0 + c] = make_float2(w.x, -w.y);
-    }
-}
-
-// Pass 3: inverse row transforms, real part, divided by nx*ny.
-template <bool MIXED>
-__global__ void __launch_bounds__(256) k_fs_rows_inv(const float2 *__restrict__ C,
-                                                     float *__restrict__ out, int nx, int ny,
-                                                     const float2 *__restrict__ tw) {
-    extern __shared__ float2 sm[];
-    const int G = lines_per_block(nx);
-    const int row0 = blockIdx.x * G;
-    const size_t img = (size_t)blockIdx.y * nx * ny;
-    for (int i = threadIdx.x; i < G * nx; i += blockDim.x) {
-        const int l = i / nx, c = i % nx, row = row0 + l;
-        float2 z = make_float2(0.f, 0.f);
-        if (row < ny) {
-            z = C[img + (size_t)row * nx + c];
-            z.y = -z.y;
+// Column pass of the Fourier shift, in place on F: transforms, the phase
+// factor, inverse transforms.
+template <int N>
+__global__ void __launch_bounds__(fft::kThreads, 3)
+    k_fs_cols(float2 *__restrict__ F, int nx, int ny, int ct, int lg, Passes P,
+              const float2 *__restrict__ tab, const float2 *__restrict__ tw,
+              const float2 *__restrict__ twr) {
+    extern __shared__ float4 sm4[];
+    float2 *sm = reinterpret_cast<float2 *>(sm4);
+    const int n = N > 0 ? N : ny, H = nx / 2 + 1;
+    const int c0 = blockIdx.x * ct, LS = col_stride(n, ct, 8);
+    const size_t img = (size_t)blockIdx.y * n;
+    const float2 *ex = tab + (size_t)blockIdx.y * (H + n) + c0, *ey = ex - c0 + H;
+    auto load = [&](int c, int row) -> float2 {
+        return c0 + c < H ? F[(img + row) * H + c0 + c] : make_float2(0.f, 0.f);
+    };
+    auto shift = [&](float2 f, int c, int row) -> float2 {
+        if (c0 + c >= H) return f;
+        return fs_apply(f, __ldg(ex + c), __ldg(ey + row), 2 * (c0 + c) == nx, 2 * row == n);
+    };
+    if constexpr (N > 0) {
+        using L2 = Pow2<N>;
+        constexpr int TPL = L2::TPL, CT = L2::G;
+        constexpr int Ra = L2::template radix<false>(0), Rl = L2::template radix<false>(L2::P - 1);
+        const int c = threadIdx.x % CT, b = threadIdx.x / CT;
+        float2 v[1][16];
+#pragma unroll
+        for (int i = 0; i < 16 / Ra; i++)
+#pragma unroll
+            for (int r = 0; r < Ra; r++) v[0][i * Ra + r] = load(c, b + i * TPL + r * (N / Ra));
+        fft::transform<N, false, false, 1>(v, sm + c * LS, b, tw);
+#pragma unroll
+        for (int i = 0; i < 16 / Rl; i++)
+#pragma unroll
+            for (int r = 0; r < Rl; r++)
+                v[0][i * Rl + r] = shift(v[0][i * Rl + r], c, b + i * TPL + r * (N / Rl));
+        fft::transform<N, true, false, 1>(v, sm + c * LS, b, twr);
+        if (c0 + c >= H) return;
+#pragma unroll
+        for (int i = 0; i < 16 / Ra; i++)
+#pragma unroll
+            for (int r = 0; r < Ra; r++) {
+                const float2 z = v[0][i * Ra + r];
+                F[(img + b + i * TPL + r * (N / Ra)) * H + c0 + c] = make_float2(z.x, -z.y);
+            }
+    } else {
+        fft::mixed_fill<true>(n, P.dn, ct, lg, sm, LS, load);
+        float2 *a = sm, *bo = sm + ct * LS;
+        for (int pass = 0; pass < 2; pass++) {
+            float2 *z = fft::mixed_transform<1, true>(P, ct, lg, a, bo, LS, tw);
+            bo = z == a ? bo : a;
+            a = z;
+            if (pass == 1) break;
+            for (int t = threadIdx.x; t < ct * n; t += fft::kThreads) {
+                float2 &f = a[(t & (ct - 1)) * LS + pz(t >> lg)];
+                f = shift(f, t & (ct - 1), t >> lg);
+            }
+            __syncthreads();
         }
-        sm[l * plen(nx) + pz(c)] = z;
-    }
-    __syncthreads();
-    fft_any<MIXED>(sm, nx, plen(nx), G, tw);
-    const float scale = (float)(nx * ny);
-    for (int i = threadIdx.x; i < G * nx; i += blockDim.x) {
-        const int l = i / nx, c = i % nx, row = row0 + l;
-        if (row < ny) out[img + (size_t)row * nx + c] = sm[l * plen(nx) + pz(c)].x / scale;
+        fft::mixed_drain<true>(n, P.dn, ct, lg, a, LS, [&](int c, int i, float2 z) {
+            if (c0 + c < H) F[(img + i) * H + c0 + c] = make_float2(z.x, -z.y);
+        });
     }
 }
 
 // ---------------------------------------------------------------------------
 // Host side.
 
+// Radices of a length's passes, in order: the kernels' own for powers of two
+// from 16, else the fewest out of {2..10, 16} (the smallest sum among those),
+// largest first.
+static void radices(int n, std::vector<int> &out) {
+    out.clear();
+    if (n >= 16 && (n & (n - 1)) == 0) {
+        const int r0 = n == 512 ? 8 : 16, r1 = n == 512 ? 8 : std::min(16, n / r0);
+        for (int r : {r0, r1, n / (r0 * r1)})
+            if (r > 1) out.push_back(r);
+        return;
+    }
+    std::vector<int> cur, best;
+    int best_sum = INT_MAX;
+    auto rec = [&](auto &&self, int m, int top, int sum) -> void {
+        if (m == 1) {
+            if (best.empty() || cur.size() < best.size() ||
+                (cur.size() == best.size() && sum < best_sum)) {
+                best = cur;
+                best_sum = sum;
+            }
+            return;
+        }
+        if (!best.empty() && cur.size() >= best.size()) return;
+        for (int r : {16, 10, 9, 8, 7, 6, 5, 4, 3, 2})
+            if (r <= top && m % r == 0) {
+                cur.push_back(r);
+                self(self, m / r, r, sum + r);
+                cur.pop_back();
+            }
+    };
+    rec(rec, n, 16, 0);
+    out = best;
+}
+
+static Passes make_passes(int n, const std::vector<int> &r) {
+    Passes p{};
+    p.n = n;
+    p.np = (int)r.size();
+    p.dn = fft::make_fastdiv(n);
+    int ns = 1;
+    for (int i = 0; i < p.np; i++) {
+        p.r[i] = r[i];
+        p.ns[i] = ns;
+        p.dnr[i] = fft::make_fastdiv(n / r[i]);
+        p.dns[i] = fft::make_fastdiv(ns);
+        ns *= r[i];
+    }
+    return p;
+}
+
+// Twiddles of both orders of a length's passes (forward at 0, reversed at n).
+static void fill_twiddles(int n, float2 *h) {
+    std::vector<int> r;
+    radices(n, r);
+    for (int o = 0; o < 2; o++) {
+        int ns = 1;
+        for (int R : r) {
+            for (int q = 1; q < R; q++)
+                for (int k = 0; k < ns; k++) {
+                    const double a = 2.0 * M_PI * (double)q * (double)k / ((double)ns * R);
+                    h[o * n + ns - 1 + (q - 1) * ns + k] =
+                        make_float2((float)std::cos(a), (float)-std::sin(a));
+                }
+            ns *= R;
+        }
+        std::reverse(r.begin(), r.end());
+    }
+}
+
+// A length's passes and its device table (twiddles of both orders).
+struct LinePlan {
+    Passes fwd;
+    const float2 *tw, *twr;
+};
+
 static std::mutex g_tw_mu;
 static std::map<std::pair<int, int>, float2 *> g_tw;  // (device, N) -> table
 
-static int twiddles(int N, const float2 **out) {
+static void line_passes(int n, LinePlan *lp) {
+    std::vector<int> r;
+    radices(n, r);
+    lp->fwd = make_passes(n, r);
+}
+
+static int line_plan(int N, LinePlan *lp) {
+    line_passes(N, lp);
     int dev = 0;
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lk(g_tw_mu);
     auto it = g_tw.find({dev, N});
-    if (it != g_tw.end()) {
-        *out = it->second;
-        return 0;
+    if (it == g_tw.end()) {
+        std::vector<float2> h(2 * N, make_float2(0.f, 0.f));
+        fill_twiddles(N, h.data());
+        float2 *d = nullptr;
+        ARECGB_CUDA(cudaMalloc(&d, sizeof(float2) * 2 * N));
+        cudaError_t e = cudaMemcpy(d, h.data(), sizeof(float2) * 2 * N, cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {
+            cudaFree(d);
+            ARECGB_CUDA(e);
+        }
+        it = g_tw.insert({{dev, N}, d}).first;
     }
-    std::vector<float2> h(N);
-    for (int k = 0; k < N; k++) {
-        const double a = 2.0 * M_PI * (double)k / (double)N;
-        h[k] = make_float2((float)std::cos(a), (float)-std::sin(a));
-    }
-    float2 *d = nullptr;
-    ARECGB_CUDA(cudaMalloc(&d, sizeof(float2) * N));
-    ARECGB_CUDA(cudaMemcpy(d, h.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
-    g_tw[{dev, N}] = d;
-    *out = d;
+    lp->tw = it->second;
+    lp->twr = it->second + N;
     return 0;
 }
-
-static bool pow2_ok(int n) { return n >= 16 && n <= 4096 && (n & (n - 1)) == 0; }
-
-static int rows_per_block(int nx) { return lines_per_block(nx); }
 
 static std::mutex g_smem_mu;
 static std::map<std::pair<int, const void *>, size_t> g_smem;  // (device, kernel) -> limit set
@@ -756,54 +769,136 @@ static int set_smem(const void *fn, size_t bytes) {
     return 0;
 }
 
-// Correlate `np` pairs; optionally keep the correlation images in `c`
-// (np*ny*nx floats) and/or reduce them to peaks.
-static int correlate_batch(const float *d1, const float *d2, int np, int ny, int nx, float *c,
-                           RowStat *stats, float2 *Xh, float2 *Yh, cudaStream_t st) {
-    const float2 *twx, *twy;
-    int rc = twiddles(nx, &twx);
-    if (!rc) rc = twiddles(ny, &twy);
-    if (rc) return rc;
-    const int G = rows_per_block(nx);
-    const int ct = col_tile(ny);
-    const size_t row_smem = sizeof(float2) * (size_t)G * plen(nx);
-    const size_t col_smem = sizeof(float2) * 2 * ct * (size_t)plen(ny);
-    // kernel instantiations for the two lengths (MIXED: not a power of two)
-    auto rows_fwd = pow2_ok(nx) ? k_cc_rows_fwd<false> : k_cc_rows_fwd<true>;
-    auto rows_inv = pow2_ok(nx) ? k_cc_rows_inv<false> : k_cc_rows_inv<true>;
-    auto cols = pow2_ok(ny) ? k_cc_cols<false> : k_cc_cols<true>;
-    if ((rc = set_smem((const void *)rows_fwd, row_smem))) return rc;
-    if ((rc = set_smem((const void *)rows_inv, row_smem))) return rc;
-    if ((rc = set_smem((const void *)cols, col_smem))) return rc;
-    const int H = nx / 2 + 1;
-    rows_fwd<<<dim3((ny + G - 1) / G, np), 256, row_smem, st>>>(d1, d2, Xh, Yh, nx, ny, twx);
-    cols<<<dim3((H + ct - 1) / ct, np), 256, col_smem, st>>>(Xh, Yh, nx, ny, twy, ct);
-    rows_inv<<<dim3((ny + G - 1) / G, np), 256, row_smem, st>>>(Xh, c, stats, nx, ny, twx);
-    ARECGB_CUDA(cudaGetLastError());
-    return 0;
+// Calls f with the length as a compile-time constant (0: not a power of two
+// from 16).
+template <typename F>
+static int with_length(int n, F &&f) {
+    switch (n) {
+#define ARECGB_LEN(n) \
+    case n: return f(std::integral_constant<int, n>{});
+        ARECGB_LEN(16) ARECGB_LEN(32) ARECGB_LEN(64) ARECGB_LEN(128) ARECGB_LEN(256)
+        ARECGB_LEN(512) ARECGB_LEN(1024) ARECGB_LEN(2048) ARECGB_LEN(4096)
+#undef ARECGB_LEN
+        default: return f(std::integral_constant<int, 0>{});
+    }
 }
 
+// Forward row pass of nz images (kPairs: image pairs x, y).
+template <int MODE>
+static int rows_fwd(const LinePlan &lp, const float *x, const float *y, RowSpectra o, int nz,
+                    int ny, int nx, cudaStream_t st) {
+    return with_length(nx, [&](auto n) -> int {
+        auto fn = k_rows_fwd<decltype(n)::value, MODE>;
+        const int G = lines_per_block(nx), lines = MODE == kPairs ? ny : (ny + 1) / 2;
+        const size_t smem = sizeof(float2) * (size_t)G * plen(nx) * (pow2_length(nx) ? 1 : 2);
+        if (int rc = set_smem((const void *)fn, smem)) return rc;
+        fn<<<dim3((lines + G - 1) / G, nz), fft::kThreads, smem, st>>>(
+            x, y, o, nx, ny, lp.fwd, fft::make_fastdiv(nx / 2 + 1), lp.tw);
+        return 0;
+    });
+}
+
+template <int MODE>
+static int rows_inv(const LinePlan &lp, const float2 *W, float *c, RowStat *stats, int nz, int ny,
+                    int nx, cudaStream_t st) {
+    return with_length(nx, [&](auto n) -> int {
+        auto fn = k_rows_inv<decltype(n)::value, MODE>;
+        const int G = lines_per_block(nx), lines = (ny + 1) / 2;
+        const size_t smem = sizeof(float2) * (size_t)G * plen(nx) * (pow2_length(nx) ? 1 : 2);
+        if (int rc = set_smem((const void *)fn, smem)) return rc;
+        fn<<<dim3((lines + G - 1) / G, nz), fft::kThreads, smem, st>>>(W, c, stats, nx, ny, lp.fwd,
+                                                                      lp.tw);
+        return 0;
+    });
+}
+
+static int log2_of(int n) {
+    int l = 0;
+    while ((1 << l) < n) l++;
+    return l;
+}
+
+static int cc_cols(const LinePlan &lp, const float4 *S, float2 *W, int nz, int ny, int nx,
+                   cudaStream_t st) {
+    return with_length(ny, [&](auto n) -> int {
+        auto fn = k_cc_cols<decltype(n)::value>;
+        const int ct = col_tile(ny, 16), H = nx / 2 + 1;
+        const size_t smem =
+            sizeof(float4) * (size_t)ct * col_stride(ny, ct, 16) * (pow2_length(ny) ? 1 : 2);
+        if (int rc = set_smem((const void *)fn, smem)) return rc;
+        fn<<<dim3((H + ct - 1) / ct, nz), fft::kThreads, smem, st>>>(
+            S, W, nx, ny, ct, log2_of(ct), lp.fwd, lp.tw, lp.twr);
+        return 0;
+    });
+}
+
+static int fs_cols(const LinePlan &lp, float2 *F, const float2 *tab, int nz, int ny, int nx,
+                   cudaStream_t st) {
+    return with_length(ny, [&](auto n) -> int {
+        auto fn = k_fs_cols<decltype(n)::value>;
+        const int ct = col_tile(ny, 8), H = nx / 2 + 1;
+        const size_t smem =
+            sizeof(float2) * (size_t)ct * col_stride(ny, ct, 8) * (pow2_length(ny) ? 1 : 2);
+        if (int rc = set_smem((const void *)fn, smem)) return rc;
+        fn<<<dim3((H + ct - 1) / ct, nz), fft::kThreads, smem, st>>>(
+            F, nx, ny, ct, log2_of(ct), lp.fwd, tab, lp.tw, lp.twr);
+        return 0;
+    });
+}
+
+// Scratch of a batch of np pairs, one piece: S [np][ny][H] float4, W
+// [np][ny][H] float2.  S is dead once the column pass is done; the
+// correlation images and row statistics take its place.
 struct CcScratch {
-    float2 *Xh = nullptr, *Yh = nullptr;
-    float *c = nullptr;
-    RowStat *stats = nullptr;
+    float4 *S;
+    float2 *W;
+    float *c;
+    RowStat *stats;
 };
 
-static void cc_free(CcScratch &s) {
-    cudaFree(s.Xh);
-    cudaFree(s.Yh);
-    cudaFree(s.c);
-    cudaFree(s.stats);
+static size_t round256(size_t b) { return (b + 255) / 256 * 256; }
+
+static size_t cc_s_bytes(int np, int ny, int nx) {
+    const size_t spec = (size_t)np * ny * (nx / 2 + 1);
+    return round256(sizeof(float4) * spec + 512);  // >= the images and the statistics
 }
 
-static int cc_alloc(CcScratch &s, int np, int ny, int nx, bool need_c) {
-    const size_t H = nx / 2 + 1;
-    ARECGB_CUDA(cudaMalloc(&s.Xh, sizeof(float2) * H * ny * np));
-    ARECGB_CUDA(cudaMalloc(&s.Yh, sizeof(float2) * H * ny * np));
-    if (need_c) ARECGB_CUDA(cudaMalloc(&s.c, sizeof(float) * (size_t)nx * ny * np));
-    ARECGB_CUDA(cudaMalloc(&s.stats, sizeof(RowStat) * (size_t)ny * np));
-    return 0;
+static size_t cc_bytes(int np, int ny, int nx) {
+    return cc_s_bytes(np, ny, nx) + sizeof(float2) * (size_t)np * ny * (nx / 2 + 1);
 }
+
+static CcScratch cc_carve(void *p, int np, int ny, int nx) {
+    CcScratch s;
+    s.S = (float4 *)p;
+    s.W = (float2 *)((char *)p + cc_s_bytes(np, ny, nx));
+    s.c = (float *)p;
+    s.stats = (RowStat *)((char *)p + round256(sizeof(float) * (size_t)np * ny * nx));
+    return s;
+}
+
+// Correlation images and row statistics of np pairs into s.c and s.stats.
+static int correlate_batch(const LinePlan &px, const LinePlan &py, const float *d1,
+                           const float *d2, int np, int ny, int nx, const CcScratch &s,
+                           cudaStream_t st) {
+    int rc = rows_fwd<kPairs>(px, d1, d2, RowSpectra{s.S, nullptr}, np, ny, nx, st);
+    if (!rc) rc = cc_cols(py, s.S, s.W, np, ny, nx, st);
+    if (!rc) rc = rows_inv<kPairs>(px, s.W, s.c, s.stats, np, ny, nx, st);
+    if (!rc) ARECGB_CUDA(cudaGetLastError());
+    return rc;
+}
+
+// Images per batch: the scratch near `target` bytes.
+static int batch_for(int nz, size_t per, size_t target) {
+    return (int)std::max<size_t>(
+        1, std::min<size_t>(std::min<size_t>((size_t)nz, 65535), target / std::max<size_t>(per, 1)));
+}
+
+// Scratch per batch.  Measured on 48 pairs of 2048^2 (50 MB each): 64 MB 3.26
+// ms, 128 MB 2.71, 256 MB 2.49, 1 GiB 2.82 — large enough to fill the SMs
+// several times over per launch, small enough that part of a batch's spectra
+// is still in the 129 MB L2 when the next pass reads it (and to allocate
+// quickly).  512^2 images: no difference from 64 MB up.
+constexpr size_t kBatchBytes = (size_t)256 << 20;
 
 int cc_shifts(const float *d1, const float *d2, int nz, int ny, int nx, float *sx, float *sy,
               int *ix, int *iy, cudaStream_t st) {
@@ -813,15 +908,18 @@ int cc_shifts(const float *d1, const float *d2, int nz, int ny, int nx, float *s
         return ARECGB_ERR_ARG;
     }
     if (nz == 0) return 0;
-    // pairs per batch: keep the scratch near 1 GiB
-    const size_t per_pair = (size_t)ny * ((size_t)(nx / 2 + 1) * 16 + (size_t)nx * 4 + 16);
-    const int batch = (int)std::max<size_t>(1, std::min<size_t>(nz, (1ull << 30) / per_pair));
-    CcScratch s;
-    int rc = cc_alloc(s, batch, ny, nx, true);
+    LinePlan px, py;
+    int rc = line_plan(nx, &px);
+    if (!rc) rc = line_plan(ny, &py);
+    if (rc) return rc;
+    const int batch = batch_for(nz, cc_bytes(1, ny, nx), kBatchBytes);
+    void *buf = nullptr;
+    ARECGB_CUDA(cudaMalloc(&buf, cc_bytes(batch, ny, nx)));
     for (int p0 = 0; !rc && p0 < nz; p0 += batch) {
         const int np = std::min(batch, nz - p0);
         const size_t off = (size_t)p0 * nx * ny;
-        rc = correlate_batch(d1 + off, d2 + off, np, ny, nx, s.c, s.stats, s.Xh, s.Yh, st);
+        const CcScratch s = cc_carve(buf, np, ny, nx);
+        rc = correlate_batch(px, py, d1 + off, d2 + off, np, ny, nx, s, st);
         if (rc) break;
         k_peak<<<np, 256, 0, st>>>(s.c, s.stats, nx, ny, sx + p0, sy + p0, ix ? ix + p0 : nullptr,
                                    iy ? iy + p0 : nullptr);
@@ -832,7 +930,7 @@ int cc_shifts(const float *d1, const float *d2, int nz, int ny, int nx, float *s
         }
     }
     cudaStreamSynchronize(st);
-    cc_free(s);
+    cudaFree(buf);
     return rc;
 }
 
@@ -842,11 +940,17 @@ int ccorr_image(const float *dx, const float *dy, float *dc, int ny, int nx, cud
                   std::to_string(nx) + " x " + std::to_string(ny) + ")");
         return ARECGB_ERR_ARG;
     }
-    CcScratch s;
-    int rc = cc_alloc(s, 1, ny, nx, false);
-    if (!rc) rc = correlate_batch(dx, dy, 1, ny, nx, dc, s.stats, s.Xh, s.Yh, st);
+    LinePlan px, py;
+    int rc = line_plan(nx, &px);
+    if (!rc) rc = line_plan(ny, &py);
+    if (rc) return rc;
+    void *buf = nullptr;
+    ARECGB_CUDA(cudaMalloc(&buf, cc_bytes(1, ny, nx)));
+    CcScratch s = cc_carve(buf, 1, ny, nx);
+    s.c = dc;
+    rc = correlate_batch(px, py, dx, dy, 1, ny, nx, s, st);
     cudaStreamSynchronize(st);
-    cc_free(s);
+    cudaFree(buf);
     return rc;
 }
 
@@ -859,41 +963,32 @@ int fshift_stack(const float *d_in, float *d_out, int nz, int ny, int nx, const 
         return ARECGB_ERR_ARG;
     }
     if (nz == 0) return 0;
-    const float2 *twx, *twy;
-    int rc = twiddles(nx, &twx);
-    if (!rc) rc = twiddles(ny, &twy);
+    LinePlan px, py;
+    int rc = line_plan(nx, &px);
+    if (!rc) rc = line_plan(ny, &py);
     if (rc) return rc;
-    const int G = rows_per_block(nx);
-    const size_t row_smem = sizeof(float2) * (size_t)G * plen(nx);
-    const size_t col_smem = sizeof(float2) * kColTile * (size_t)plen(ny);
-    auto fs_rows = pow2_ok(nx) ? k_fs_rows<false> : k_fs_rows<true>;
-    auto fs_rows_inv = pow2_ok(nx) ? k_fs_rows_inv<false> : k_fs_rows_inv<true>;
-    auto fs_cols = pow2_ok(ny) ? k_fs_cols<false> : k_fs_cols<true>;
-    if ((rc = set_smem((const void *)fs_rows, row_smem))) return rc;
-    if ((rc = set_smem((const void *)fs_rows_inv, row_smem))) return rc;
-    if ((rc = set_smem((const void *)fs_cols, col_smem))) return rc;
-    // images per batch: complex scratch near 1 GiB
-    const size_t per = sizeof(float2) * (size_t)nx * ny;
-    const int batch = (int)std::max<size_t>(1, std::min<size_t>(nz, (1ull << 30) / per));
-    float2 *C = nullptr;
-    ARECGB_CUDA(cudaMalloc(&C, per * batch));
+    const int H = nx / 2 + 1;
+    const size_t spec = sizeof(float2) * (size_t)ny * H, tabs = sizeof(float2) * (size_t)(H + ny);
+    const int batch = batch_for(nz, spec + tabs, kBatchBytes);
+    void *buf = nullptr;
+    ARECGB_CUDA(cudaMalloc(&buf, (spec + tabs) * batch));
+    float2 *F = (float2 *)buf, *tab = F + (size_t)ny * H * batch;
     for (int z0 = 0; z0 < nz && !rc; z0 += batch) {
         const int nb = std::min(batch, nz - z0);
         const size_t off = (size_t)z0 * nx * ny;
-        fs_rows<<<dim3((ny + G - 1) / G, nb), 256, row_smem, st>>>(d_in + off, C, nx, ny, twx);
-        fs_cols<<<dim3((nx + kColTile - 1) / kColTile, nb), 256, col_smem, st>>>(
-            C, nx, ny, d_sx + z0, d_sy + z0, twy);
-        fs_rows_inv<<<dim3((ny + G - 1) / G, nb), 256, row_smem, st>>>(C, d_out + off, nx, ny,
-                                                                     twx);
-        count_launches(3);
+        k_fs_phase<<<dim3((H + ny + 127) / 128, nb), 128, 0, st>>>(d_sx + z0, d_sy + z0, nx, ny, tab);
+        rc = rows_fwd<kRows>(px, d_in + off, nullptr, RowSpectra{nullptr, F}, nb, ny, nx, st);
+        if (!rc) rc = fs_cols(py, F, tab, nb, ny, nx, st);
+        if (!rc) rc = rows_inv<kRows>(px, F, d_out + off, nullptr, nb, ny, nx, st);
+        count_launches(4);
         cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) {
+        if (!rc && e != cudaSuccess) {
             set_error(std::string("fshift2d: ") + cudaGetErrorString(e));
             rc = cuda_status(e);
         }
     }
     cudaStreamSynchronize(st);
-    cudaFree(C);
+    cudaFree(buf);
     return rc;
 }
 
@@ -916,8 +1011,6 @@ int peak_search(const float *dc, int nz, int ny, int nx, float *sx, float *sy, i
     }
     return 0;
 }
-
-
 // ---------------------------------------------------------------------------
 // Shift search without allocation (arecgb_cc_shifts_static).
 //
@@ -928,10 +1021,11 @@ int peak_search(const float *dc, int nz, int ny, int nx, float *sx, float *sy, i
 // allocator (a caching allocator that already holds the free HBM).
 //
 // Scratch: one file-scope device array of kStaticBytes (3.5 MiB), carved into
-//   Xh, Yh  float2 [kStaticSpec]   half spectra of both images
-//   c       float  [kStaticPixels] correlation images
-//   stats   RowStat[kStaticRows]   per-row peak statistics
-//   tw      float2 [1008]          twiddles for N = 16..512, table N at offset N - 16
+//   S       float4 [kStaticSpec]   half spectra of both images; then the
+//                                  correlation images and row statistics
+//   W       float2 [kStaticSpec]   the product's spectrum after the column pass
+//   tw      float2 [2016]          twiddles for N = 16..512, both pass orders,
+//                                  table N at offset 2 (N - 16)
 // Limit: nx, ny powers of two in [16, 512] and nz * ny * nx <= kStaticPixels
 // (one 512 x 512 pair, or e.g. 64 pairs of 64 x 64).  Larger requests are
 // rejected with ARECGB_ERR_ARG; arecgb_cc_shifts has no such limit.
@@ -943,15 +1037,11 @@ int peak_search(const float *dc, int nz, int ny, int nx, float *sx, float *sy, i
 constexpr size_t kStaticPixels = 512 * 512;
 constexpr size_t kStaticRows = kStaticPixels / 16;                  // ny * nz <= pixels / nx
 constexpr size_t kStaticSpec = kStaticPixels / 2 + kStaticRows;     // (nx/2 + 1) * ny * nz
-constexpr size_t kStaticTw = 1024;                                  // 16 + 32 + ... + 512 = 1008
-constexpr size_t kOffYh = sizeof(float2) * kStaticSpec;
-constexpr size_t kOffC = 2 * kOffYh;
-constexpr size_t kOffStats = kOffC + sizeof(float) * kStaticPixels;
-constexpr size_t kOffTw = kOffStats + sizeof(RowStat) * kStaticRows;
+constexpr size_t kStaticTw = 2048;                                  // 2 (16 + ... + 512) = 2016
+constexpr size_t kOffW = (sizeof(float4) * kStaticSpec + 512 + 255) / 256 * 256;
+constexpr size_t kOffTw = kOffW + sizeof(float2) * kStaticSpec;
 constexpr size_t kStaticBytes = kOffTw + sizeof(float2) * kStaticTw;
-static_assert(kOffYh % 256 == 0 && kOffC % 256 == 0 && kOffStats % 256 == 0 &&
-                  kOffTw % 256 == 0,
-              "scratch pieces must stay 256-byte aligned");
+static_assert(kOffW % 256 == 0 && kOffTw % 256 == 0, "scratch pieces must stay 256-byte aligned");
 
 static __device__ __align__(256) unsigned char g_cc_static[kStaticBytes];
 
@@ -986,11 +1076,7 @@ static int static_setup(unsigned char **base) {
         return cuda_status(e != cudaSuccess ? e : cudaErrorInvalidSymbol);
     }
     std::vector<float2> h(kStaticTw, make_float2(0.f, 0.f));
-    for (int N = 16; N <= 512; N *= 2)
-        for (int k = 0; k < N; k++) {
-            const double a = 2.0 * M_PI * (double)k / (double)N;
-            h[N - 16 + k] = make_float2((float)std::cos(a), (float)-std::sin(a));
-        }
+    for (int N = 16; N <= 512; N *= 2) fill_twiddles(N, h.data() + 2 * (N - 16));
     e = cudaMemcpy((unsigned char *)ptr + kOffTw, h.data(), sizeof(float2) * kStaticTw,
                    cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
@@ -1021,28 +1107,19 @@ int cc_shifts_static(const float *d1, const float *d2, int nz, int ny, int nx, f
     int rc = static_setup(&base);
     if (rc) return rc;
     if (nz == 0) return 0;
-    float2 *Xh = reinterpret_cast<float2 *>(base);
-    float2 *Yh = reinterpret_cast<float2 *>(base + kOffYh);
-    float *c = reinterpret_cast<float *>(base + kOffC);
-    RowStat *stats = reinterpret_cast<RowStat *>(base + kOffStats);
     const float2 *tw = reinterpret_cast<const float2 *>(base + kOffTw);
-    const float2 *twx = tw + (nx - 16), *twy = tw + (ny - 16);
-    // shared memory: 8 * G * nx = 32 KB per row block, 64 * ny <= 32 KB per
-    // column block (set_smem only ever raises the kernels' limits).
-    const int G = rows_per_block(nx);
-    const size_t row_smem = sizeof(float2) * (size_t)G * plen(nx);
-    const size_t col_smem = sizeof(float2) * 2 * kColTile * (size_t)plen(ny);
-    if ((rc = set_smem((const void *)k_cc_rows_fwd<false>, row_smem))) return rc;
-    if ((rc = set_smem((const void *)k_cc_rows_inv<false>, row_smem))) return rc;
-    if ((rc = set_smem((const void *)k_cc_cols<false>, col_smem))) return rc;
-    const int H = nx / 2 + 1;
-    k_cc_rows_fwd<false><<<dim3((ny + G - 1) / G, nz), 256, row_smem, st>>>(d1, d2, Xh, Yh, nx, ny,
-                                                                           twx);
-    k_cc_cols<false><<<dim3((H + kColTile - 1) / kColTile, nz), 256, col_smem, st>>>(Xh, Yh, nx, ny, twy,
-                                                                            kColTile);
-    k_cc_rows_inv<false><<<dim3((ny + G - 1) / G, nz), 256, row_smem, st>>>(Xh, c, stats, nx, ny,
-                                                                           twx);
-    k_peak<<<nz, 256, 0, st>>>(c, stats, nx, ny, sx, sy, ix, iy);
+    LinePlan px, py;
+    line_passes(nx, &px);
+    line_passes(ny, &py);
+    px.tw = tw + 2 * (nx - 16);
+    px.twr = px.tw + nx;
+    py.tw = tw + 2 * (ny - 16);
+    py.twr = py.tw + ny;
+    // nz ny (nx/2 + 1) <= kStaticSpec for every accepted shape, so S and W end
+    // before the twiddles
+    const CcScratch s = cc_carve(base, nz, ny, nx);
+    if ((rc = correlate_batch(px, py, d1, d2, nz, ny, nx, s, st))) return rc;
+    k_peak<<<nz, 256, 0, st>>>(s.c, s.stats, nx, ny, sx, sy, ix, iy);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error(std::string("cc_shifts_static: ") + cudaGetErrorString(e));
