@@ -18,8 +18,9 @@
 // the concatenation buffers cat1, cat2, cat3, where the pooling and the
 // decoder read them (no copy).
 // The 3x3 convolutions of 32+ input channels, forward and data-gradient, run on
-// the tensor cores (tcgen05, arec_unet_conv.cu); weight gradients, pooling,
-// upsampling, the first and last layers run on CUDA cores (arec_unet_ops.cu).
+// the tensor cores (tcgen05, arec_unet_conv.cu), and so do their weight
+// gradients (arec_unet_wgrad.cu); pooling, upsampling, the first and last
+// layers run on CUDA cores (arec_unet_ops.cu).
 //
 // Parameters: one flat FP32 vector, per layer W then b, W in [Cout][9][Cin]
 // (c1a: [32][9]; output: [32]); a bf16 mirror with the same offsets feeds the
@@ -245,8 +246,9 @@ static int conv_bwd(Net *n, int l, const __nv_bfloat16 *x, const __nv_bfloat16 *
                     cudaStream_t st) {
     const size_t P = (size_t)N * h * w;
     const int ci = kCin[l], co = kCout[l];
-    relu_bwd_s(y, ys, 0, dy, dys, 0, n->gpre, P, co, st);
-    conv_wgrad(x, n->gpre, n->grads + n->woff[l], n->grads + n->boff[l], N, h, w, ci, co, st);
+    relu_bwd_bias(y, ys, dy, dys, n->gpre, n->grads + n->boff[l], P, co, st);
+    if (int rc = conv_wgrad(x, n->gpre, n->grads + n->woff[l], N, h, w, ci, co, n->err, st))
+        return rc;
     if (dx)
         return conv3x3_bf16(n->gpre, n->wflip + n->woff[l], nullptr, dx, N, h, w, co, ci, 0, 0,
                             n->err, st, ci);

@@ -39,11 +39,12 @@ void chan_add(const __nv_bfloat16 *src, float *dst, size_t P, int C, int Cs, int
 void f32_to_bf16(const float *a, __nv_bfloat16 *b, size_t n, cudaStream_t st);
 void relu_bwd(const __nv_bfloat16 *y, const __nv_bfloat16 *dy, __nv_bfloat16 *dpre, size_t n,
               cudaStream_t st);
-// dpre[p][c] = dy[p*dys + dyo + c] * (y[p*yys + yo + c] > 0), c < C
-void relu_bwd_s(const __nv_bfloat16 *y, int yys, int yo, const __nv_bfloat16 *dy, int dys, int dyo,
-                __nv_bfloat16 *dpre, size_t P, int C, cudaStream_t st);
-void conv_wgrad(const __nv_bfloat16 *x, const __nv_bfloat16 *dpre, float *gw, float *gb, int N,
-                int H, int W, int Cin, int Cout, cudaStream_t st);
+// dpre[p][c] = dy[p*dys + c] * (y[p*yys + c] > 0), c < C; gb[c] += sum_p dpre[p][c]
+void relu_bwd_bias(const __nv_bfloat16 *y, int yys, const __nv_bfloat16 *dy, int dys,
+                   __nv_bfloat16 *dpre, float *gb, size_t P, int C, cudaStream_t st);
+// gw[co][tap][ci] += sum_p dpre[p][co] x[p + tap][ci] (arec_unet_wgrad.cu)
+int conv_wgrad(const __nv_bfloat16 *x, const __nv_bfloat16 *dpre, float *gw, int N, int H, int W,
+               int Cin, int Cout, int *err, cudaStream_t st);
 void flip_weights(const float *w, __nv_bfloat16 *wt, int Cin, int Cout, cudaStream_t st);
 void mse(const float *out, const float *target, float *dout, double *partial, size_t n, float scale,
          int nblocks, cudaStream_t st);

@@ -470,21 +470,30 @@ bool encode_sino_map(CUtensorMap *m, const float *base, int ys, int nx, int na, 
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// NHWC bf16 tensor [N][H][W][C]: box = 32 channels x box_w x box_h pixels of
+// one image, 64-byte swizzle; false if the CUDA driver refuses it.
+bool encode_nhwc_map(CUtensorMap *m, const void *base, int N, int H, int W, int C, int box_w,
+                     int box_h) {
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc) return false;
+    const cuuint64_t d[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
+    const cuuint64_t s[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
+    const cuuint32_t b[4] = {32, (cuuint32_t)box_w, (cuuint32_t)box_h, 1};
+    const cuuint32_t one[4] = {1, 1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)base, d, s, b, one,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Tensor maps of one convolution; false if the CUDA driver refuses them (the
 // caller then uses the gather kernel).
 static bool conv_tensor_maps(const __nv_bfloat16 *x, const __nv_bfloat16 *w, int N, int H, int Wd,
                              int Cin, int Cout, CUtensorMap *tx, CUtensorMap *tw, int box_rows = 1) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return false;
-    const cuuint64_t xd[4] = {(cuuint64_t)Cin, (cuuint64_t)Wd, (cuuint64_t)H, (cuuint64_t)N};
-    const cuuint64_t xs[3] = {(cuuint64_t)Cin * 2, (cuuint64_t)Wd * Cin * 2,
-                              (cuuint64_t)H * Wd * Cin * 2};
-    const cuuint32_t xb[4] = {(cuuint32_t)kConvKC, 128, (cuuint32_t)box_rows, 1};
-    const cuuint32_t one[4] = {1, 1, 1, 1};
-    if (enc(tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)x, xd, xs, xb, one,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return false;
+    static_assert(kConvKC == 32, "encode_nhwc_map's box");
+    if (!encode_nhwc_map(tx, x, N, H, Wd, Cin, 128, box_rows)) return false;
+    const cuuint32_t one[3] = {1, 1, 1};
     const cuuint64_t wd[3] = {(cuuint64_t)Cin, 9, (cuuint64_t)Cout};
     const cuuint64_t ws[2] = {(cuuint64_t)Cin * 2, (cuuint64_t)9 * Cin * 2};
     const cuuint32_t wb[3] = {(cuuint32_t)kConvKC, 1, (cuuint32_t)Cout};

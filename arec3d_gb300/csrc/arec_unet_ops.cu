@@ -292,71 +292,41 @@ __global__ void k_relu_bwd(const __nv_bfloat16 *__restrict__ y, const __nv_bfloa
     GRID_STRIDE(i, n) { dpre[i] = bf(y[i]) > 0.f ? dy[i] : tobf(0.f); }
 }
 
-__global__ void k_relu_bwd_s(const __nv_bfloat16 *__restrict__ y, int yys, int yo,
-                             const __nv_bfloat16 *__restrict__ dy, int dys, int dyo,
-                             __nv_bfloat16 *__restrict__ dpre, size_t P, int C) {
-    GRID_STRIDE(i, P * C) {
-        const size_t p = i / C;
-        const int c = (int)(i % C);
-        dpre[i] = bf(y[p * yys + yo + c]) > 0.f ? dy[p * dys + dyo + c] : tobf(0.f);
-    }
-}
-
-// Weight gradient of a 3x3 conv on CUDA cores:
-//   gw[co][t][ci] += sum_p dpre[p][co] * x[p+t][ci],  gb[co] += sum_p dpre[p][co]
-// Block: 32 co x 32 ci for one tap, a slice of the pixels (grid.z); 256 threads,
-// each 2 co x 2 ci; pixels staged through shared memory 64 at a time.
+// The same with row strides, and the bias gradient gb[c] += sum_p dpre[p][c].
+// One thread per pixel and 8 channels (16-byte vectors); a thread keeps its
+// channels over its pixels, so the sums stay in registers until the block adds
+// them (FP32, one atomic per channel and block).  C a power of two in [32, 256].
 __global__ void __launch_bounds__(256)
-    k_conv_wgrad(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ dpre,
-                 float *__restrict__ gw, float *__restrict__ gb, int N, int H, int W, int Cin,
-                 int Cout) {
-    const int t = blockIdx.y % 9, cob = (blockIdx.y / 9) * 32, cib = blockIdx.x * 32;
-    __shared__ float sd[64][33], sx[64][33];
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;  // co pair ty, ci pair tx
-    float a00 = 0, a01 = 0, a10 = 0, a11 = 0, bsum0 = 0, bsum1 = 0;
-    const size_t P = (size_t)N * H * W;
-    const size_t per = (P + gridDim.z - 1) / gridDim.z;
-    const size_t p_begin = per * blockIdx.z, p_end = min(P, p_begin + per);
-    const int dy = t / 3 - 1, dx = t % 3 - 1;
-    for (size_t pc = p_begin; pc < p_end; pc += 64) {
-        for (int e = threadIdx.x; e < 64 * 32; e += 256) {
-            const int pp = e / 32, c = e % 32;
-            const size_t p = pc + pp;
-            float dv = 0.f, xv = 0.f;
-            if (p < p_end) {
-                dv = bf(dpre[p * Cout + cob + c]);
-                const int n = (int)(p / ((size_t)H * W)), h = (int)((p / W) % H), w = (int)(p % W);
-                const int hh = h + dy, ww = w + dx;
-                if (hh >= 0 && hh < H && ww >= 0 && ww < W)
-                    xv = bf(x[(((size_t)n * H + hh) * W + ww) * Cin + cib + c]);
-            }
-            sd[pp][c] = dv;
-            sx[pp][c] = xv;
+    k_relu_bwd_bias(const __nv_bfloat16 *__restrict__ y, int yys,
+                    const __nv_bfloat16 *__restrict__ dy, int dys,
+                    __nv_bfloat16 *__restrict__ dpre, float *__restrict__ gb, size_t P, int C) {
+    __shared__ float red[256][9];
+    const int C8 = C / 8, g = threadIdx.x & (C8 - 1), per = 256 / C8;
+    float acc[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) acc[j] = 0.f;
+    for (size_t p = (size_t)blockIdx.x * per + threadIdx.x / C8; p < P;
+         p += (size_t)gridDim.x * per) {
+        const uint4 yv = *reinterpret_cast<const uint4 *>(y + p * yys + g * 8);
+        const uint4 dv = *reinterpret_cast<const uint4 *>(dy + p * dys + g * 8);
+        const __nv_bfloat16 *yb = reinterpret_cast<const __nv_bfloat16 *>(&yv);
+        const __nv_bfloat16 *db = reinterpret_cast<const __nv_bfloat16 *>(&dv);
+        __align__(16) __nv_bfloat16 o[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            o[j] = bf(yb[j]) > 0.f ? db[j] : tobf(0.f);
+            acc[j] += bf(o[j]);
         }
-        __syncthreads();
-#pragma unroll 8
-        for (int pp = 0; pp < 64; pp++) {
-            const float d0 = sd[pp][2 * ty], d1 = sd[pp][2 * ty + 1];
-            const float x0 = sx[pp][2 * tx], x1 = sx[pp][2 * tx + 1];
-            a00 = fmaf(d0, x0, a00);
-            a01 = fmaf(d0, x1, a01);
-            a10 = fmaf(d1, x0, a10);
-            a11 = fmaf(d1, x1, a11);
-            if (t == 4 && blockIdx.x == 0 && tx == 0) {
-                bsum0 += d0;
-                bsum1 += d1;
-            }
-        }
-        __syncthreads();
+        *reinterpret_cast<uint4 *>(dpre + p * C + g * 8) = *reinterpret_cast<const uint4 *>(o);
     }
-    const int co0 = cob + 2 * ty, ci0 = cib + 2 * tx;
-    atomicAdd(&gw[((size_t)co0 * 9 + t) * Cin + ci0], a00);
-    atomicAdd(&gw[((size_t)co0 * 9 + t) * Cin + ci0 + 1], a01);
-    atomicAdd(&gw[((size_t)(co0 + 1) * 9 + t) * Cin + ci0], a10);
-    atomicAdd(&gw[((size_t)(co0 + 1) * 9 + t) * Cin + ci0 + 1], a11);
-    if (t == 4 && blockIdx.x == 0 && tx == 0) {
-        atomicAdd(&gb[co0], bsum0);
-        atomicAdd(&gb[co0 + 1], bsum1);
+#pragma unroll
+    for (int j = 0; j < 8; j++) red[threadIdx.x][j] = acc[j];
+    __syncthreads();
+    if ((int)threadIdx.x < C) {
+        const int gg = threadIdx.x / 8, j = threadIdx.x % 8;
+        float s = 0.f;
+        for (int t = gg; t < 256; t += C8) s += red[t][j];
+        atomicAdd(&gb[threadIdx.x], s);
     }
 }
 
@@ -563,16 +533,12 @@ void relu_bwd(const __nv_bfloat16 *y, const __nv_bfloat16 *dy, __nv_bfloat16 *dp
               cudaStream_t st) {
     k_relu_bwd<<<blocks_for(n), 256, 0, st>>>(y, dy, dpre, n);
 }
-void relu_bwd_s(const __nv_bfloat16 *y, int yys, int yo, const __nv_bfloat16 *dy, int dys, int dyo,
-                __nv_bfloat16 *dpre, size_t P, int C, cudaStream_t st) {
-    k_relu_bwd_s<<<blocks_for(P * C), 256, 0, st>>>(y, yys, yo, dy, dys, dyo, dpre, P, C);
-}
-void conv_wgrad(const __nv_bfloat16 *x, const __nv_bfloat16 *dpre, float *gw, float *gb, int N,
-                int H, int W, int Cin, int Cout, cudaStream_t st) {
-    const size_t P = (size_t)N * H * W;
-    const int tiles = (Cin / 32) * (Cout / 32) * 9;
-    int gz = (int)std::max<size_t>(1, std::min<size_t>((P + 4095) / 4096, (size_t)(152 * 8 / tiles + 1)));
-    k_conv_wgrad<<<dim3(Cin / 32, 9 * (Cout / 32), gz), 256, 0, st>>>(x, dpre, gw, gb, N, H, W, Cin, Cout);
+void relu_bwd_bias(const __nv_bfloat16 *y, int yys, const __nv_bfloat16 *dy, int dys,
+                   __nv_bfloat16 *dpre, float *gb, size_t P, int C, cudaStream_t st) {
+    // about 16 pixels per thread at least, 8 blocks per SM at most
+    const size_t per = 256 / (C / 8);
+    const int blocks = (int)std::max<size_t>(1, std::min<size_t>(152 * 8, P / (16 * per)));
+    k_relu_bwd_bias<<<blocks, 256, 0, st>>>(y, yys, dy, dys, dpre, gb, P, C);
 }
 void flip_weights(const float *w, __nv_bfloat16 *wt, int Cin, int Cout, cudaStream_t st) {
     k_flip_weights<<<blocks_for((size_t)Cout * 9 * Cin), 256, 0, st>>>(w, wt, Cin, Cout);
