@@ -10,6 +10,7 @@
 #include <cmath>
 
 #include "arec_internal.cuh"
+#include "arec_project_mma.cuh"
 
 namespace arecgb {
 
@@ -259,6 +260,10 @@ int plan_create(Plan **out, int weighting, double radius, int ny, int nangles,
         plan_destroy(p);
         return cuda_status(e);
     }
+    if (int rc = mma_plan_create(p, groups, ang, rows, cols, tables)) {
+        plan_destroy(p);
+        return rc;
+    }
     if (int rc = tables ? plan_build_tables(p) : 0) {
         plan_destroy(p);
         return rc;
@@ -290,6 +295,7 @@ void plan_destroy(Plan *p) {
     cudaFree(p->d_xT);
     cudaFree(p->d_bpw);
     cudaFree(p->d_bpf);
+    mma_plan_destroy(p);
     cudaFree(p->d_err);
     cudaFree(p->d_partials);
     for (auto &v : p->d_vol) cudaFree(v);

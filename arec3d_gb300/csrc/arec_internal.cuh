@@ -80,6 +80,23 @@ struct Plan {
     float4 *d_bpw = nullptr;      // [ntiles][na][32]
     int2 *d_bpf = nullptr;        // [ntiles][na]
     size_t table_bytes = 0;
+    // tensor-core projectors (arec_project_mma.cu): groups, strips and segments
+    // of the forward projection, tiles of the back projection, FP16 operands
+    int mma = 0;
+    int4 *d_mgroups = nullptr;
+    int2 *d_mstrips = nullptr, *d_msegs = nullptr;
+    int *d_mshear = nullptr, *d_mslots = nullptr, *d_mpix = nullptr;
+    int m_groups = 0, m_segs = 0, m_strips = 0;
+    uint4 *d_ptaps = nullptr;     // taps as FP16 pairs [ngroups][nrays][4] (with tables)
+    int2 *d_mtiles = nullptr;     // back projection: 16 x 16-pixel tiles
+    int m_tiles = 0;
+    // FP16 pairs of the volume and of the sinogram, [0] forward and [1] back
+    // projection; per slice the largest magnitude, then the wide-range flag; the
+    // end of the last call that used them
+    void *d_half[2] = {nullptr, nullptr};
+    unsigned *d_smax[2] = {nullptr, nullptr};
+    cudaEvent_t half_ev[2] = {nullptr, nullptr};
+    mutable std::mutex half_lock[2];
     int tuned = 0;                // launch shapes chosen by plan_autotune
     int2 *d_tiles = nullptr;      // back-projection ray tiles: (ix0, iz0) of 8x4-pixel tiles
     int ntiles = 0;

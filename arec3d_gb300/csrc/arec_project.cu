@@ -4,6 +4,7 @@
 #include <cstring>
 
 #include "arec_project_impl.cuh"
+#include "arec_project_mma.cuh"
 
 namespace arecgb {
 
@@ -22,33 +23,6 @@ int launch_fpb_kb(const OpArgs &, int, dim3, const float *, float *, int, int, i
 int launch_fpb_sq(const OpArgs &, int, dim3, const float *, float *, int, int, int, int,
                   const CUtensorMap &, const CUtensorMap &, cudaStream_t);
 int sumsq_partials(const float *d_v, size_t n, double *d_partials, int nblocks, cudaStream_t st);
-
-static OpArgs make_args(const Plan *p, const int *skip) {
-    OpArgs A;
-    A.ray = p->d_ray;
-    A.ang = p->d_ang;
-    A.rows = p->d_rows;
-    A.cols = p->d_cols;
-    A.groups = p->d_groups;
-    A.tiles = p->d_tiles;
-    A.nx = p->nx;
-    A.nrays = p->nrays;
-    A.ys = p->ys;
-    A.na = p->na;
-    A.ngroups = p->ngroups;
-    A.r_hi = p->r_hi;
-    A.r_lo = p->r_lo;
-    A.partials = p->d_partials;
-    A.skip = skip;
-    A.err = p->d_err;
-    A.taps = p->d_taps;
-    A.bpw = p->d_bpw;
-    A.bpf = p->d_bpf;
-    A.kinv = p->d_kinv;
-    A.lin_off = p->d_lin_off;
-    A.lin_list = p->d_lin_list;
-    return A;
-}
 
 // Back projection: floats per lane (the plan's, or the autotuner's choice).
 static int bp_vec(const Plan *p) { return p->bp_vec ? p->bp_vec : p->vec; }
@@ -75,8 +49,8 @@ static int fp_slice_blocks(const Plan *p) {
     return (p->ys + 32 * v - 1) / (32 * v);
 }
 
-// The forward projector's FP64 norm is a separate pass over q (1024 partials).
-int fp_grid_blocks(const Plan *) { return kNormBlocks; }
+// The forward projector's FP64 norm is a separate pass over q.
+int fp_grid_blocks(const Plan *) { return 2 * kNormBlocks; }  // two sums at a time (CGLS)
 
 int bp_grid_blocks(const Plan *p) { return p->ntiles * slice_blocks(p); }
 
@@ -153,6 +127,10 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
         // zero q, then each (orientation, line band) launch adds its part
         k_zero_unless<<<(unsigned)std::min<size_t>(152 * 8, (nq / 4 + 255) / 256), 256, 0, st>>>(
             reinterpret_cast<float4 *>(d_q), nq / 4, d_skip);
+        if (p->mma) {
+            rc = forward_project_mma(p, d_x, d_q, d_skip, st);
+            if (rc) return rc;
+        }
         const int ntile = (p->nx + kFpBins - 1) / kFpBins;
         rc = 0;
         // With the tables: tensor maps over x and over its column-major copy
@@ -161,7 +139,7 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
         CUtensorMap tmx, tmxT;
         memset(&tmx, 0, sizeof(tmx));
         memset(&tmxT, 0, sizeof(tmxT));
-        if (A.taps) {
+        if (A.taps && !p->mma) {
             const int span = 32 * fp_vec(p);
             if (p->ngroups_o[1]) {
                 const int ys4 = p->ys / 4;
@@ -177,7 +155,7 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
                 return ARECGB_ERR_ARG;
             }
         }
-        for (int o = 0; o < 2 && !rc; o++) {
+        for (int o = 0; o < 2 && !rc && !p->mma; o++) {
             const int ngo = p->ngroups_o[o];
             if (!ngo) continue;
             const int g0 = o ? p->ngroups_o[0] : 0;
@@ -206,6 +184,16 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
 
 int back_project(const Plan *p, const float *d_s, float *d_g, double *d_norm2,
                  const int *d_skip, cudaStream_t st) {
+    if (p->mma) {
+        int rc = timing_mark(p, false, false, st);
+        if (!rc) rc = back_project_mma(p, d_s, d_g, d_skip, st);
+        if (!rc && d_norm2) {
+            rc = sumsq_partials(d_g, vol_floats(p), p->d_partials, kNormBlocks, st);
+            if (!rc) rc = reduce_partials(p->d_partials, kNormBlocks, d_norm2, st);
+            count_launches(2);
+        }
+        return rc ? rc : timing_mark(p, false, true, st);
+    }
     const OpArgs A = make_args(p, d_skip);
     const int nsc = slice_chunks(p);
     dim3 grid(p->ntiles, slice_blocks(p));
@@ -277,32 +265,45 @@ int plan_build_tables(Plan *p) {
     if (p->weighting == ARECGB_LIN) return plan_build_lin_index(p);
     const char *env = getenv("ARECGB_PLAN_TABLES");
     if (env && env[0] == '0') return 0;
-    const size_t b_taps = sizeof(float4) * (size_t)p->ngroups * p->nrays * 4 +
-                          sizeof(float) * (size_t)p->nrays * p->ys;  // + x's column-major copy
-    const size_t b_bpw = sizeof(float4) * (size_t)p->ntiles * p->na * 32;
-    const size_t b_bpf = sizeof(int2) * (size_t)p->ntiles * p->na;
+    const size_t b_recs = sizeof(float4) * (size_t)p->ngroups * p->nrays * 4;
+    // the tensor-core projectors read packed taps; the others taps and x's
+    // column-major copy
+    const size_t b_taps = b_recs + (p->mma ? 0 : sizeof(float) * (size_t)p->nrays * p->ys);
+    const size_t b_bpw = p->mma ? 0 : sizeof(float4) * (size_t)p->ntiles * p->na * 32;
+    const size_t b_bpf = p->mma ? 0 : sizeof(int2) * (size_t)p->ntiles * p->na;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
-    if ((double)(b_taps + b_bpw + b_bpf) > 0.4 * (double)free_b) return 0;
-    if (cudaMalloc(&p->d_taps, sizeof(float4) * (size_t)p->ngroups * p->nrays * 4) != cudaSuccess ||
-        cudaMalloc(&p->d_xT, sizeof(float) * (size_t)p->nrays * p->ys) != cudaSuccess ||
-        cudaMalloc(&p->d_bpw, b_bpw) != cudaSuccess || cudaMalloc(&p->d_bpf, b_bpf) != cudaSuccess) {
+    const size_t work = p->mma ? mma_work_bytes(p->nx, p->na, p->ys) : 0;  // in use already
+    if ((double)(work + b_taps + b_bpw + b_bpf) > 0.4 * (double)(work + free_b)) return 0;
+    cudaError_t e = p->mma ? cudaMalloc(&p->d_ptaps, b_recs) : cudaMalloc(&p->d_taps, b_recs);
+    if (e == cudaSuccess && !p->mma) e = cudaMalloc(&p->d_xT, sizeof(float) * (size_t)p->nrays * p->ys);
+    if (e == cudaSuccess && !p->mma) e = cudaMalloc(&p->d_bpw, b_bpw);
+    if (e == cudaSuccess && !p->mma) e = cudaMalloc(&p->d_bpf, b_bpf);
+    if (e != cudaSuccess) {
         cudaGetLastError();  // an allocation failure is not sticky; run without tables
         cudaFree(p->d_taps);
+        cudaFree(p->d_ptaps);
         cudaFree(p->d_xT);
         cudaFree(p->d_bpw);
         cudaFree(p->d_bpf);
         p->d_taps = nullptr;
+        p->d_ptaps = nullptr;
         p->d_xT = nullptr;
         p->d_bpw = nullptr;
         p->d_bpf = nullptr;
         return 0;
     }
     OpArgs A = make_args(p, nullptr);
-    const int rc = p->weighting == ARECGB_KB
-                       ? launch_tables_kb(A, p->ntiles, p->d_taps, p->d_bpw, p->d_bpf, p->stream)
-                       : launch_tables_sq(A, p->ntiles, p->d_taps, p->d_bpw, p->d_bpf, p->stream);
-    count_launches(2);
+    int rc = 0;
+    if (p->mma) {
+        rc = mma_build_taps(p, A);
+        count_launches(1);
+    } else {
+        rc = p->weighting == ARECGB_KB
+                 ? launch_tables_kb(A, p->ntiles, p->d_taps, p->d_bpw, p->d_bpf, p->stream)
+                 : launch_tables_sq(A, p->ntiles, p->d_taps, p->d_bpw, p->d_bpf, p->stream);
+        count_launches(2);
+    }
     ARECGB_CUDA(cudaGetLastError());
     ARECGB_CUDA(cudaStreamSynchronize(p->stream));
     int err = 0;
@@ -318,9 +319,16 @@ int plan_build_tables(Plan *p) {
 // Autotuner: times the forward projector for band heights of 32, 64 and 128
 // lines and the back projector with one or two slice chunks per block on the
 // caller's buffers (x: a volume, q: a sinogram of this plan; both overwritten),
-// best of two runs each after a warm-up run, and keeps the fastest shapes.
+// best of two runs each after a warm-up run, and keeps the fastest shapes.  The
+// tensor-core projectors have one shape: they keep the plan's defaults.
 int plan_autotune(Plan *p, float *d_x, float *d_q, cudaStream_t st) {
     if (p->weighting == ARECGB_LIN) return 0;  // the linear pair has no shapes to choose
+    if (p->mma) {
+        p->fp_vec = p->bp_vec = p->vec;
+        p->bp_nsc = 1;
+        p->tuned = 1;
+        return 0;
+    }
     cudaEvent_t e0, e1;
     ARECGB_CUDA(cudaEventCreate(&e0));
     ARECGB_CUDA(cudaEventCreate(&e1));

@@ -33,35 +33,11 @@
 
 #include <climits>
 
+#include "arec_project_args.cuh"
 #include "arec_umma.cuh"
 #include "arec_weights.cuh"
 
 namespace arecgb {
-
-struct OpArgs {
-    const float4 *ray;
-    const AngleParams *ang;
-    const RowInfo *rows;
-    const ColInfo *cols;
-    const int4 *groups;
-    const int2 *tiles;
-    int nx, nrays, ys, na, ngroups;
-    float r_hi, r_lo;
-    double *partials;
-    const int *skip;
-    int *err;
-    // linear weighting: per angle, the rays grouped by first bin (lin_off
-    // [na][nx+2]: bucket j holds the rays whose first bin is j - 1; lin_list
-    // [na][nrays]: ray indices, ascending within a bucket)
-    const int *lin_off;
-    const int *lin_list;
-    // optional per-plan tables (null when the plan has none)
-    const float4 *taps;  // [ngroups][nrays][4]: ray_taps of each forward-projection angle
-                         // group's (up to 4) angles per ray: (iqx, w0, w1, w2)
-    const float4 *bpw;   // [ntiles][na][32]: the back projector's plan entries
-    const int2 *bpf;     // [ntiles][na]: footprint (first bin, bins) per tile and angle
-    const int *kinv;     // column-major ray index -> ray index
-};
 
 // A 2-D tensor map over rows of ys floats (x or its column-major copy): box =
 // box_cols slices x box_rows rays; false if the CUDA driver refuses it.

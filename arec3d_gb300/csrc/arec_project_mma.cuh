@@ -1,0 +1,90 @@
+// Projectors on the tensor cores (square-pixel and Kaiser-Bessel weightings):
+// shared definitions of arec_project_mma.cu and the projector dispatch.
+//
+// A projection is a product with a sparse matrix: a ray adds to three bins.
+// Taken 8 x 8 pixels at a time the matrix is dense enough for the tensor cores:
+// at any angle the 64 rays of a block reach at most 13 neighbouring bins, so
+// with windows of 16 bins a block's product with one angle is a 64 x 16 matrix
+// per slice, 16/3 of the multiply-adds of the sparse one, at 28 times the FP32
+// rate.  Both factors are split into two FP16 numbers each: three products
+// hi*hi, hi*lo, lo*hi carry 22 bits.  The tensor core's FP32 accumulation rounds
+// toward zero, so a sum stays in TMEM for one block only; FP32 registers take
+// it from there with ordinary rounding.
+#pragma once
+
+#include <cuda.h>
+#include <cuda_fp16.h>
+
+#include "arec_internal.cuh"
+
+namespace arecgb {
+
+// FP16 pairs: hi = fp16(v), lo = fp16((v - hi) 2^11), v = the weight times 2^12 or
+// the slice's value times 2^half_shift(the slice's largest magnitude).  The low
+// halves' own scale (taken back by the MMA that adds hi*hi, D = A B + D 2^-11)
+// keeps them normal: 22 bits down to 2^-29 of the slice's largest magnitude, an
+// error of 2^-51 of it below.
+constexpr float kWeightScale = 4096.f;
+constexpr int kLowBits = 11;
+constexpr float kLowScale = 2048.f;
+// Slices with values from 2^40 on (fill values, infinities, NaN) have neighbours
+// that these pairs cannot hold: such an operand takes the kernels that work ray
+// by ray in FP32.
+constexpr unsigned kWideBits = (127u + 40u) << 23;
+
+__device__ __forceinline__ int half_shift(unsigned max_bits) {
+    if (max_bits == 0u) return 0;
+    const int e = (int)(max_bits >> 23) - 127;
+    return max(-126, min(126, 14 - e));  // |v| 2^shift < 2^15
+}
+__device__ __forceinline__ float pow2f(int e) { return __uint_as_float((unsigned)(e + 127) << 23); }
+
+// Forward projection groups, strips and segments (see arec_project_mma.cu).
+struct MmaPlan {
+    const int4 *groups;   // (first angle, angles, orientation, segments)
+    const int2 *strips;   // (first strip, strips)
+    const int2 *segs;     // [groups][max_segs]: line blocks [first, last)
+    const int *shear;     // [groups][lblocks]: the strips' offset in pixels per line block
+    const int *slots;     // per angle its place in the taps table: 4 * (4-angle group) + column,
+                          // the sign bit set for column sweeps
+    const uint4 *taps;    // packed taps (null: computed by the kernel)
+    const int2 *tiles;    // back projection: 16 x 16-pixel tiles (first ix, iz)
+    int ngroups, max_segs, max_strips, lblocks;
+};
+
+// Plans whose projections run on the tensor cores.
+bool mma_takes(int weighting, int nx, int ys, int na);
+// spare: leave the plan to the FP32 kernels (p->mma = 0) when the operands would
+// take more than 40 % of the free memory.  It is left to them in any case when
+// they cannot be allocated.
+int mma_plan_create(Plan *p, const std::vector<int4> &groups4,
+                    const std::vector<AngleParams> &ang, const std::vector<RowInfo> &rows,
+                    const std::vector<ColInfo> &cols, bool spare);
+struct OpArgs;
+int mma_build_taps(Plan *p, const OpArgs &A);
+void mma_plan_destroy(Plan *p);
+int forward_project_mma(const Plan *p, const float *d_x, float *d_q, const int *d_skip,
+                        cudaStream_t st);
+int back_project_mma(const Plan *p, const float *d_s, float *d_g, const int *d_skip, cudaStream_t st);
+
+// A plan's FP16 operands serve one forward and one back projection at a time:
+// eager calls on other streams or threads wait for the last one's (on the device).
+// Held around launches of graphs whose projections use them.
+class MmaHold {
+  public:
+    MmaHold(Plan *const *plans, int n, cudaStream_t st);
+    ~MmaHold();
+    MmaHold(const MmaHold &) = delete;
+    MmaHold &operator=(const MmaHold &) = delete;
+
+  private:
+    std::vector<Plan *> held;
+    cudaStream_t st;
+};
+
+// Bytes of the FP16 operands and maxima of a plan.
+inline size_t mma_work_bytes(size_t nx, size_t na, size_t ys) {
+    return sizeof(float) * (nx * nx * ys + na * nx * ys + 2 * (ys + 4));
+}
+
+}  // namespace arecgb

@@ -6,7 +6,7 @@
 // Here many cylinders of uneven radius, detector width, slice and angle
 // counts are solved on one GPU.  Their inputs and results stay resident; the
 // solver workspace (three volume vectors and two sinograms per problem, plus
-// the plan's geometry tables) does not fit for all of them at once, so the
+// the plan's operands and geometry tables) does not fit for all of them at once, so the
 // problems are packed into waves whose workspace fits a byte budget (first
 // fit, largest first).  Per wave: one plan per problem (without the optional
 // projector tables: they would cost 32 B per ray and angle), the optional
@@ -28,6 +28,7 @@
 
 #include "arec_gb300.h"
 #include "arec_internal.cuh"
+#include "arec_project_mma.cuh"
 
 namespace arecgb {
 int cgls_batch(Plan *const *plans, const float *const *d_b, float *const *d_x, const int *warm,
@@ -100,7 +101,8 @@ int arecgb_solve_uneven(const arecgb_problem *probs, int n, size_t budget_bytes,
     }
     std::vector<int> net_of(n, -1);
     // workspace bytes per problem: CGLS's 3 volume + 2 sinogram vectors, the
-    // ray table and a margin for the plan's other tables and partials
+    // projectors' FP16 operands, the ray table and a margin for the plan's
+    // other tables and partials
     std::vector<size_t> bytes(n);
     for (int i = 0; i < n; i++) {
         const arecgb_problem &q = probs[i];
@@ -121,6 +123,8 @@ int arecgb_solve_uneven(const arecgb_problem *probs, int n, size_t budget_bytes,
         const size_t ys = (size_t)round8(q.ny);
         bytes[i] = sizeof(float) * (3 * (size_t)nr * ys + 2 * (size_t)q.nangles * nx * ys) +
                    sizeof(float4) * (size_t)nr + (64u << 20);
+        if (mma_takes(q.weighting, nx, (int)ys, q.nangles))
+            bytes[i] += mma_work_bytes(nx, q.nangles, ys);
     }
     // waves: first fit, largest first
     std::vector<int> order(n);

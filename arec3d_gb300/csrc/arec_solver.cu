@@ -2,6 +2,7 @@
 // All of these are HBM-bound: grid-stride loops over float4 where the layout
 // allows, sized to a multiple of the SM count.
 #include "arec_internal.cuh"
+#include "arec_project_mma.cuh"
 #include "arec_vector.cuh"
 
 #include <math.h>
@@ -196,6 +197,64 @@ __global__ void __launch_bounds__(256) k_cgls_p(SolveState *S, const float *__re
 __global__ void k_cgls_alpha(SolveState *S) {
     if (S->done) return;
     S->alpha = S->gamma / S->qnorm2;
+}
+
+// The two sums of a step on the tensor-core projectors: ||q||^2 (weighted: w) and
+// <s, q>, float4 by float4, in fixed order.
+__global__ void __launch_bounds__(256) k_cgls_dots(const SolveState *S, const float4 *__restrict__ q,
+                                                   const float4 *__restrict__ s,
+                                                   const float4 *__restrict__ w, size_t n4,
+                                                   double *__restrict__ partials) {
+    if (S->done) return;
+    __shared__ double red[2][8];
+    double qq = 0.0, sq = 0.0;
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256) {
+        const float4 a = q[i], b = s[i], c = w ? w[i] : make_float4(1.f, 1.f, 1.f, 1.f);
+        qq += ((double)__fmul_rn(__fmul_rn(a.x, a.x), c.x) + (double)__fmul_rn(__fmul_rn(a.y, a.y), c.y)) +
+              ((double)__fmul_rn(__fmul_rn(a.z, a.z), c.z) + (double)__fmul_rn(__fmul_rn(a.w, a.w), c.w));
+        sq += ((double)__fmul_rn(a.x, b.x) + (double)__fmul_rn(a.y, b.y)) +
+              ((double)__fmul_rn(a.z, b.z) + (double)__fmul_rn(a.w, b.w));
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        qq += __shfl_down_sync(0xffffffffu, qq, o);
+        sq += __shfl_down_sync(0xffffffffu, sq, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        red[0][threadIdx.x >> 5] = qq;
+        red[1][threadIdx.x >> 5] = sq;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double t = 0.0;
+        for (int k = 0; k < 8; k++) t += red[threadIdx.x][k];
+        partials[threadIdx.x * gridDim.x + blockIdx.x] = t;
+    }
+}
+
+// alpha = <s, q> / ||q||^2: gamma / ||q||^2 where g is exactly A^T s.  The tensor
+// cores round toward zero, so that A and A^T may differ by a few 1e-8 in scale;
+// gamma would carry that into every later direction (CGLS x 5 at 65 bins,
+// Kaiser-Bessel: 8e-6 from FP64 with gamma, 1.1e-6 with the sum; FP32 kernels 2.9e-6).
+__global__ void __launch_bounds__(256) k_cgls_alpha_dots(SolveState *S, const double *__restrict__ p,
+                                                         int n) {
+    if (S->done) return;
+    __shared__ double red[2][256];
+    double a = 0.0, b = 0.0;
+    for (int i = threadIdx.x; i < n; i += 256) a += p[i], b += p[n + i];
+    red[0][threadIdx.x] = a;
+    red[1][threadIdx.x] = b;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o) {
+            red[0][threadIdx.x] += red[0][threadIdx.x + o];
+            red[1][threadIdx.x] += red[1][threadIdx.x + o];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        S->qnorm2 = red[0][0];
+        S->alpha = red[1][0] / red[0][0];
+    }
 }
 
 // x += alpha*p over the volume and s -= alpha*q over the sinogram, in double,
@@ -421,15 +480,21 @@ static int cgls_iteration(Plan *p, SolveState *S, double *hist, float *x, float 
     k_cgls_save<<<gv, 256, 0, st>>>(S, x, xs, nv / 4);
     k_cgls_save_done<<<1, 1, 0, st>>>(S);
     k_cgls_p<<<gv, 256, 0, st>>>(S, g, pd, nv / 4);
-    int rc = forward_project(p, pd, q, w ? nullptr : &S->qnorm2, &S->done, st);
+    int rc = forward_project(p, pd, q, w || p->mma ? nullptr : &S->qnorm2, &S->done, st);
     if (rc) return rc;
-    if (w) {  // ||A p||^2 weighted
+    if (p->mma) {
+        const int nb = std::min(kRedBlocks, gs);
+        k_cgls_dots<<<nb, 256, 0, st>>>(S, (const float4 *)q, (const float4 *)s, (const float4 *)w,
+                                        ns / 4, p->d_partials);
+        k_cgls_alpha_dots<<<1, 256, 0, st>>>(S, p->d_partials, nb);
+        count_launches(1);
+    } else if (w) {  // ||A p||^2 weighted
         k_wsumsq<<<kRedBlocks, 256, 0, st>>>(q, w, ns, p->d_partials);
         rc = reduce_partials(p->d_partials, kRedBlocks, &S->qnorm2, st);
         if (rc) return rc;
         count_launches(2);
     }
-    k_cgls_alpha<<<1, 1, 0, st>>>(S);
+    if (!p->mma) k_cgls_alpha<<<1, 1, 0, st>>>(S);
     k_cgls_xs<<<gs, 256, 0, st>>>(S, x, pd, nv / 4, s, q, ns / 4, w);
     rc = back_project(p, s, g, &S->gnorm2, &S->done, st);
     if (rc) return rc;
@@ -607,6 +672,7 @@ int cgls_batch(Plan *const *plans, const float *const *d_b, float *const *d_x, c
         for (int i = 0; i < n; i++) all = all && H[i].done;
         if (all || launched >= maxit) break;
         const int nb = std::min(batch, maxit - launched);
+        const MmaHold hold(plans, n, cs);
         for (int k = 0; k < nb && !rc; k++) {
             e = cudaGraphLaunch(exec, cs);
             if (e != cudaSuccess) fail(e, "graph launch");

@@ -107,6 +107,70 @@ __device__ __forceinline__ void mma_commit(uint64_t *mbar) {
         : "memory");
 }
 
+// A value that is the same in all lanes, in a form the compiler knows to be so
+// (uniform registers and branches).
+template <typename T>
+__device__ __forceinline__ T uniform(T v) {
+    return __shfl_sync(0xffffffffu, v, 0);
+}
+
+// The same two issued by one elected lane of a converged warp.  With the whole
+// warp in the issuing loop the descriptors stay in the uniform registers the
+// instruction reads; a loop entered by one lane only moves each of them there
+// from ordinary registers, about 75 cycles per MMA, more than a small MMA takes.
+__device__ __forceinline__ void mma_f16_warp(uint32_t dtmem, uint64_t adesc, uint64_t bdesc,
+                                             uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "elect.sync _|q, 0xffffffff;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(dtmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// The same with D = A B + D 2^-S (0 <= S <= 15).
+template <int S>
+__device__ __forceinline__ void mma_f16_warp_scaled(uint32_t dtmem, uint64_t adesc, uint64_t bdesc,
+                                                    uint32_t idesc) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q;\n"
+        "setp.eq.b32 p, 0, 0;\n"
+        "elect.sync _|q, 0xffffffff;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %4;\n"
+        "}\n" ::"r"(dtmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "n"(S)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit_warp(uint64_t *mbar) {
+    asm volatile(
+        "{\n"
+        ".reg .pred q;\n"
+        "elect.sync _|q, 0xffffffff;\n"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+        "}\n" ::"r"(smem_addr(mbar))
+        : "memory");
+}
+
+// Store 16 32-bit columns of this thread's TMEM lane (tmem_wait_st before others read them).
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+        "%12, %13, %14, %15, %16};\n" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]),
+        "r"(r[3]), "r"(r[4]), "r"(r[5]),
+        "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]),
+        "r"(r[12]), "r"(r[13]), "r"(r[14]),
+        "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() {
+    asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+}
+
 // --- mbarrier -------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t *mbar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(mbar)), "r"(count)
@@ -133,6 +197,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *mbar, uint32_t parity) {
 __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity, uint32_t limit) {
     for (uint32_t i = 0; i < limit; i++)
         if (mbar_try_wait(mbar, parity)) return true;
+    return false;
+}
+
+// The same by a converged warp, in step (the result is uniform).
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *mbar, uint32_t parity, uint32_t limit) {
+    for (uint32_t i = 0; i < limit; i++)
+        if (__all_sync(0xffffffffu, mbar_try_wait(mbar, parity))) return true;
     return false;
 }
 
@@ -209,8 +280,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 }
 
 // The same for 16 columns.
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
         "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
@@ -220,6 +290,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
         : "r"(taddr)
         : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
+    tmem_ld16(taddr, r);
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }

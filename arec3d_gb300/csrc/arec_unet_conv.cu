@@ -457,6 +457,35 @@ bool encode_rows_map(CUtensorMap *m, const float *base, int ys, int nrows, int b
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// FP16 pairs [2][n2][n1][ys] (arec_project_mma.cuh): box = 64 slices x box1 x
+// box2 of one part, 128-byte swizzle.
+bool encode_half_map(CUtensorMap *m, const void *base, int ys, int n1, int n2, int box1, int box2) {
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc) return false;
+    const cuuint64_t d[4] = {(cuuint64_t)ys, (cuuint64_t)n1, (cuuint64_t)n2, 2};
+    const cuuint64_t st[3] = {(cuuint64_t)ys * 2, (cuuint64_t)ys * 2 * n1, (cuuint64_t)ys * 2 * n1 * n2};
+    const cuuint32_t b[4] = {64, (cuuint32_t)box1, (cuuint32_t)box2, 1};
+    const cuuint32_t one[4] = {1, 1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, (void *)base, d, st, b, one,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// FP16 pairs [2][na][groups][nx][8]: box = box_bins bins of 8 slices x 16 slice
+// groups of one angle and part.
+bool encode_foot_map(CUtensorMap *m, const void *base, int nx, int groups, int na, int box_bins) {
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc) return false;
+    const cuuint64_t row = (cuuint64_t)nx * 16;
+    const cuuint64_t d[4] = {(cuuint64_t)nx * 8, (cuuint64_t)groups, (cuuint64_t)na, 2};
+    const cuuint64_t st[3] = {row, row * groups, row * groups * na};
+    const cuuint32_t b[4] = {(cuuint32_t)box_bins * 8, 16, 1, 1};
+    const cuuint32_t one[4] = {1, 1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, (void *)base, d, st, b, one,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool encode_sino_map(CUtensorMap *m, const float *base, int ys, int nx, int na, int box_cols,
                      int box_bins) {
     EncodeTiledFn enc = encode_tiled();
