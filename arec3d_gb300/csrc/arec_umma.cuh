@@ -257,6 +257,22 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const void *tmap, int c0,
         : "memory");
 }
 
+// Tile from shared memory to global memory (elements outside the tensor are dropped);
+// its reads of shared memory are done after tma_store_wait_read<n> (all but the
+// thread's last n stores).
+__device__ __forceinline__ void tma_store_4d(const void *tmap, const void *src, int c0, int c1, int c2,
+                                             int c3) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];\n"
+        "cp.async.bulk.commit_group;\n" ::"l"(tmap),
+        "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_addr(src))
+        : "memory");
+}
+template <int N>
+__device__ __forceinline__ void tma_store_wait_read() {
+    asm volatile("cp.async.bulk.wait_group.read %0;\n" ::"n"(N) : "memory");
+}
+
 // --- TMEM -> registers ------------------------------------------------------------------------
 // Warp w of a warpgroup reads TMEM lanes 32w..32w+31; each thread gets 32
 // consecutive 32-bit columns starting at `taddr`'s column.

@@ -176,253 +176,247 @@ static int launch_conv(const __nv_bfloat16 *X, const __nv_bfloat16 *Wt, const fl
 }
 
 // ---------------------------------------------------------------------------
-// TMA path (image widths that are multiples of 128): a tile is 128 consecutive
-// pixels of one image row.  Per K chunk (one tap, 32 input channels) one TMA
-// load brings the tile's shifted neighbours from an NHWC tensor map (box 32
-// channels x 128 pixels; rows and columns outside the image arrive as zeros,
-// which is the convolution's padding) and one the chunk's weights from a
-// [Cout][9][Cin] tensor map, both with the 64-byte swizzle the tensor core
-// reads directly.  Four stages: thread 0 of warp 0 issues the loads, thread 0
-// of warp 1 the MMAs; each stage's commit frees it for the loads four chunks
-// later.  All four warps run the epilogue from TMEM.
+// TMA path.  One block per SM runs over the layer's tiles; one warp loads (TMA),
+// one issues the MMAs, four take the sums from TMEM to global memory, so that a
+// tile's loads, products and stores overlap its neighbours'.
 //
-// A block lives a few microseconds (9 or 18 chunks, each waiting on an L2
-// load), so throughput comes from blocks resident per SM: the narrow layers
-// take two stages (21-25 KB of shared memory: 8-10 blocks per SM within the
-// 512 TMEM columns), the wide ones four.
-template <int COUT>
-struct TmaCfg {
-    static constexpr int STAGES = COUT <= 64 ? 2 : 4;
-    static constexpr int A_BYTES = 128 * 64;  // 128 pixels x 32 channels
-    static constexpr int B_BYTES = COUT * 64;
-    static constexpr int STAGE = A_BYTES + B_BYTES;  // a multiple of 1024
-    static constexpr int SMEM = STAGES * STAGE + 1024;
-    static constexpr uint32_t NCOLS = COUT < 32 ? 32 : COUT;
+// A chunk of K is 32 or 64 input channels of one tap (or one column of taps): its
+// pixels come from an NHWC tensor map (rows and columns outside the image arrive
+// as zeros, which is the convolution's padding), its weights from a
+// [Cout][9][Cin] one, both with the 64 or 128-byte swizzle the tensor core reads
+// directly.  Two kinds of tiles, which add the same products in different orders:
+//
+// - BAND (32 or 64 output channels, widths that are multiples of 128): R rows of
+//   128 pixels, chunks over (dx, channels).  One box brings the R + 2 input rows,
+//   shifted by dx, and three the weights of the taps (dy, dx).  Input row j
+//   adds to the output rows j - 2 .. j with the taps dy = 2 .. 0: their sums are
+//   neighbouring columns of TMEM and the three weight slabs, in that order, one
+//   operand, so one MMA (N = 3 Cout) takes all three: a narrow MMA is bound by
+//   the reading of its A operand (44 clocks at N = 32, 56 at 96).  Per output
+//   row the order is (dx, channels, dy).
+// - otherwise R tiles of 128 pixels (2^lw x 128 / 2^lw, one above the other),
+//   chunks over (tap, channels); the tiles share a chunk's weights.
+//
+// What bounds it: the loads into shared memory (a band's rows arrive three times, a
+// tile's pixels nine times), at most 70 bytes per clock and SM from L2, and half
+// of that for rows of 64 bytes: where the input channels allow it a chunk is 64 of
+// them (the order of the products stays).  Forward pass at 16 x 1024^2, all layers
+// of a kind, from blocks of one tile each with one-lane issue (4.5, 3.0, 2.4 and
+// 0.46 ms for 32, 64, 128 and 256 output channels): 2.6, 1.6, 1.9 and 0.45 ms with
+// 32-channel chunks, 2.4, 1.6, 1.3 and 0.32 ms with 64.
+template <int COUT, int R, bool BAND, int KC, int ST>
+struct PipeCfg {
+    static constexpr int STAGES = ST;
+    static constexpr int A_TILE = 128 * KC * 2;  // 128 pixels
+    static constexpr int A_BYTES = (BAND ? R + 2 : R) * A_TILE;
+    static constexpr int B_TAP = COUT * KC * 2;  // one tap's weights
+    static constexpr int STAGE = A_BYTES + (BAND ? 3 : 1) * B_TAP;  // a multiple of 1024
+    static constexpr int OUT = 32 * 64;      // a warp's 32 pixels x 32 channels
+    static constexpr int NOUT = STAGES * STAGE > 212 * 1024 ? 1 : 2;  // such buffers per warp
+    static constexpr int SMEM = STAGES * STAGE + 4 * NOUT * OUT + 1024;
+    static_assert(SMEM <= 227 * 1024 - 1024, "shared memory");
+    static constexpr int COLS = R * COUT;
+    static constexpr uint32_t NCOLS = 2 * COLS <= 256 ? 2 * COLS : 512;  // two sets of sums
 };
-
-template <int COUT>
-__global__ void __launch_bounds__(128)
-    conv3x3_tma_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
-                       const float *__restrict__ bias, __nv_bfloat16 *__restrict__ Y, int H,
-                       int Wd, int Cin, int relu, int ystride, int *err) {
-    using Cfg = TmaCfg<COUT>;
-    extern __shared__ unsigned char sm_raw[];
-    __shared__ __align__(8) uint64_t full[Cfg::STAGES], empty[Cfg::STAGES], done;
-    __shared__ uint32_t tmem_base;
-    const uint32_t raw = umma::smem_addr(sm_raw);
-    unsigned char *sm = sm_raw + ((1024u - (raw & 1023u)) & 1023u);  // 1024-byte aligned stages
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int p0 = blockIdx.x * 128;
-    const int hw = H * Wd;
-    const int n = p0 / hw, h = (p0 / Wd) % H, w0 = p0 % Wd;
-
-    if (warp == 0) {
-        umma::tmem_alloc(&tmem_base, Cfg::NCOLS);
-        umma::tmem_relinquish();
-    }
-    if (tid == 0) {
-        for (int st = 0; st < Cfg::STAGES; st++) {
-            umma::mbar_init(&full[st], 1);
-            umma::mbar_init(&empty[st], 1);
-        }
-        umma::mbar_init(&done, 1);
-        umma::mbar_fence_init();
-    }
-    umma::fence_before_sync();
-    __syncthreads();
-    umma::fence_after_sync();
-    const uint32_t tmem = tmem_base;
-    const int cchunks = Cin / kConvKC, nchunks = 9 * cchunks;
-
-    if (warp == 0 && lane == 0) {
-        bool ok = true;
-        for (int c = 0; c < nchunks && ok; c++) {
-            const int st = c % Cfg::STAGES;
-            if (c >= Cfg::STAGES &&
-                !umma::mbar_wait(&empty[st], (uint32_t)(c / Cfg::STAGES - 1) & 1u, kWaitLimit)) {
-                ok = false;
-                atomicOr(err, 4);
-                break;
-            }
-            const int tap = c / cchunks, c0 = (c % cchunks) * kConvKC;
-            unsigned char *A = sm + st * Cfg::STAGE;
-            umma::mbar_arrive_expect_tx(&full[st], (uint32_t)Cfg::STAGE);
-            umma::tma_load_4d(A, &tmX, c0, w0 + tap % 3 - 1, h + tap / 3 - 1, n, &full[st]);
-            umma::tma_load_3d(A + Cfg::A_BYTES, &tmW, c0, tap, 0, &full[st]);
-        }
-    } else if (warp == 1 && lane == 0) {
-        constexpr uint32_t idesc = umma::idesc_bf16(128, COUT);
-        for (int c = 0; c < nchunks; c++) {
-            const int st = c % Cfg::STAGES;
-            if (!umma::mbar_wait(&full[st], (uint32_t)(c / Cfg::STAGES) & 1u, kWaitLimit)) {
-                atomicOr(err, 4);
-                break;
-            }
-            umma::fence_after_sync();
-            const uint32_t a = umma::smem_addr(sm + st * Cfg::STAGE), b = a + Cfg::A_BYTES;
-#pragma unroll
-            for (int k = 0; k < 2; k++)
-                umma::mma_bf16(tmem, umma::smem_desc_sw64(a + 32 * k),
-                               umma::smem_desc_sw64(b + 32 * k), idesc, (c > 0 || k > 0) ? 1u : 0u);
-            umma::mma_commit(&empty[st]);
-        }
-        umma::mma_commit(&done);  // arrives when every MMA above has completed
-    }
-    __syncwarp();
-    const bool dok = __all_sync(0xffffffffu, umma::mbar_wait(&done, 0, kWaitLimit));
-    umma::fence_after_sync();
-    if (!dok && lane == 0) atomicOr(err, 4);
-    if (dok) {
-        const int p = p0 + tid;  // TMEM lane = pixel
-#pragma unroll 1
-        for (int cc = 0; cc < COUT / 32; cc++) {
-            float v[32];
-            umma::tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(cc * 32), v);
-            __align__(16) __nv_bfloat16 out[32];
-#pragma unroll
-            for (int i = 0; i < 32; i++) {
-                float t = v[i] + (bias ? bias[cc * 32 + i] : 0.f);
-                if (relu) t = fmaxf(t, 0.f);
-                out[i] = __float2bfloat16(t);
-            }
-            uint4 *dst = reinterpret_cast<uint4 *>(Y + (size_t)p * ystride + cc * 32);
-#pragma unroll
-            for (int q = 0; q < 4; q++) dst[q] = reinterpret_cast<const uint4 *>(out)[q];
-        }
-    }
-    umma::fence_before_sync();
-    __syncthreads();
-    if (warp == 0) umma::tmem_dealloc(tmem, Cfg::NCOLS);
+// K-major operand whose rows are KC channels: 64-byte or 128-byte swizzle.
+template <int KC>
+__device__ __forceinline__ uint64_t desc_k(uint32_t saddr) {
+    if (KC == 32) return umma::smem_desc_sw64(saddr);
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+    d |= (uint64_t)1 << 16;            // leading byte offset (unused for this layout)
+    d |= (uint64_t)(1024 >> 4) << 32;  // stride byte offset
+    d |= (uint64_t)1 << 46;            // version
+    d |= (uint64_t)2 << 61;            // 128-byte swizzle
+    return d;
 }
 
-// Several output rows per block (TMA path, narrow layers): R consecutive rows
-// of one image x 128 pixels x COUT channels, one accumulator per row in TMEM
-// (R x COUT columns).  K runs over (column shift dx, 32-channel chunk): one
-// TMA box brings the R + 2 input rows the R output rows need, shifted by dx
-// (rows outside the image arrive as zeros), and three more the weights of
-// the taps (dy, dx), dy = 0, 1, 2; output row r then takes input row r + dy
-// with tap (dy, dx).  Each input row is loaded 3 (R + 2) / R times per output
-// row instead of 9 times, and a block's fixed costs are shared by R rows.
-template <int COUT, int R>
-struct RowsCfg {
-    static constexpr int STAGES = 2;
-    static constexpr int A_ROW = 128 * 64;              // one input row tile: 128 px x 32 ch
-    static constexpr int A_BYTES = (R + 2) * A_ROW;
-    static constexpr int B_TAP = COUT * 64;             // one tap's weights for 32 channels
-    static constexpr int STAGE = A_BYTES + 3 * B_TAP;   // a multiple of 1024
-    static constexpr int SMEM = STAGES * STAGE + 1024;
-    static constexpr uint32_t NCOLS = R * COUT;          // a power of two in [32, 512]
-};
+constexpr int kPipeLoad = 4, kPipeMma = 5, kPipeThreads = 32 * 6;
 
-template <int COUT, int R>
-__global__ void __launch_bounds__(128)
-    conv3x3_rows_kernel(const __grid_constant__ CUtensorMap tmX,
-                        const __grid_constant__ CUtensorMap tmW, const float *__restrict__ bias,
-                        __nv_bfloat16 *__restrict__ Y, int H, int Wd, int Cin, int relu,
-                        int ystride, int *err) {
-    using Cfg = RowsCfg<COUT, R>;
-    static_assert(Cfg::NCOLS >= 32 && Cfg::NCOLS <= 512 && (Cfg::NCOLS & (Cfg::NCOLS - 1)) == 0,
+template <int COUT, int R, bool BAND, int KC, int ST>
+__global__ void __launch_bounds__(kPipeThreads, 1)
+    conv3x3_pipe_kernel(const __grid_constant__ CUtensorMap tmX,
+                        const __grid_constant__ CUtensorMap tmW,
+                        const __grid_constant__ CUtensorMap tmY, const float *__restrict__ bias, int H,
+                        int Wd, int Cin, int lw, int relu, int wt, int ht, int ntiles, int *err) {
+    using Cfg = PipeCfg<COUT, R, BAND, KC, ST>;
+    static_assert(Cfg::NCOLS >= 32 && 2 * Cfg::COLS <= 512 && (Cfg::NCOLS & (Cfg::NCOLS - 1)) == 0,
                   "TMEM columns: a power of two in [32, 512]");
     static_assert(Cfg::STAGE % 1024 == 0, "stages stay 1024-byte aligned");
     extern __shared__ unsigned char sm_raw[];
-    __shared__ __align__(8) uint64_t full[Cfg::STAGES], empty[Cfg::STAGES], done;
+    __shared__ __align__(8) uint64_t full[ST], empty[ST], accfull[2], accfree[2];
+    __shared__ __align__(16) float s_bias[COUT];
     __shared__ uint32_t tmem_base;
     const uint32_t raw = umma::smem_addr(sm_raw);
     unsigned char *sm = sm_raw + ((1024u - (raw & 1023u)) & 1023u);  // 1024-byte aligned stages
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int wtiles = Wd / 128, hgroups = H / R;
-    const int b = blockIdx.x;
-    const int wt = b % wtiles, hg = (b / wtiles) % hgroups, n = b / (wtiles * hgroups);
-    const int h0 = hg * R, w0 = wt * 128;
+    const int tid = threadIdx.x, warp = umma::uniform(tid >> 5), lane = tid & 31;
+    const int cchunks = Cin / KC, nchunks = (BAND ? 3 : 9) * cchunks;
+    const int hb = BAND ? R : (128 >> lw) * R;  // image rows per tile
 
-    if (warp == 0) {
+    if (warp == kPipeLoad) {
         umma::tmem_alloc(&tmem_base, Cfg::NCOLS);
         umma::tmem_relinquish();
     }
     if (tid == 0) {
-        for (int st = 0; st < Cfg::STAGES; st++) {
-            umma::mbar_init(&full[st], 1);
-            umma::mbar_init(&empty[st], 1);
+        for (int s = 0; s < ST; s++) {
+            umma::mbar_init(&full[s], 1);
+            umma::mbar_init(&empty[s], 1);
         }
-        umma::mbar_init(&done, 1);
+        for (int b = 0; b < 2; b++) {
+            umma::mbar_init(&accfull[b], 1);
+            umma::mbar_init(&accfree[b], 4);
+        }
         umma::mbar_fence_init();
     }
+    for (int i = tid; i < COUT; i += kPipeThreads) s_bias[i] = bias ? bias[i] : 0.f;
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
-    const uint32_t tmem = tmem_base;
-    const int cchunks = Cin / kConvKC, nchunks = 3 * cchunks;  // (dx, channel chunk)
+    const uint32_t tmem = umma::uniform(tmem_base);
 
-    if (warp == 0 && lane == 0) {
-        for (int c = 0; c < nchunks; c++) {
-            const int st = c % Cfg::STAGES;
-            if (c >= Cfg::STAGES &&
-                !umma::mbar_wait(&empty[st], (uint32_t)(c / Cfg::STAGES - 1) & 1u, kWaitLimit)) {
-                atomicOr(err, 4);
-                break;
-            }
-            const int dx = c / cchunks, c0 = (c % cchunks) * kConvKC;
-            unsigned char *A = sm + st * Cfg::STAGE;
-            umma::mbar_arrive_expect_tx(&full[st], (uint32_t)Cfg::STAGE);
-            umma::tma_load_4d(A, &tmX, c0, w0 + dx - 1, h0 - 1, n, &full[st]);
+    if (warp == kPipeLoad) {
+        if (lane == 0) {
+            bool ok = true;
+            int it = 0;
+            for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+                const int w0 = t % wt << lw, h0 = t / wt % ht * hb, n = t / wt / ht;
+                for (int c = 0; c < nchunks; c++, it++) {
+                    const int s = it % ST;
+                    if (it >= ST &&
+                        !umma::mbar_wait(&empty[s], (uint32_t)(it / ST - 1) & 1u, kWaitLimit)) {
+                        ok = false;
+                        break;
+                    }
+                    const int tap = c / cchunks, c0 = (c % cchunks) * KC;
+                    unsigned char *A = sm + s * Cfg::STAGE, *B = A + Cfg::A_BYTES;
+                    umma::mbar_arrive_expect_tx(&full[s], (uint32_t)Cfg::STAGE);
+                    if (BAND) {
+                        umma::tma_load_4d(A, &tmX, c0, w0 + tap - 1, h0 - 1, n, &full[s]);
 #pragma unroll
-            for (int dy = 0; dy < 3; dy++)
-                umma::tma_load_3d(A + Cfg::A_BYTES + dy * Cfg::B_TAP, &tmW, c0, 3 * dy + dx, 0,
-                                  &full[st]);
-        }
-    } else if (warp == 1 && lane == 0) {
-        constexpr uint32_t idesc = umma::idesc_bf16(128, COUT);
-        for (int c = 0; c < nchunks; c++) {
-            const int st = c % Cfg::STAGES;
-            if (!umma::mbar_wait(&full[st], (uint32_t)(c / Cfg::STAGES) & 1u, kWaitLimit)) {
-                atomicOr(err, 4);
-                break;
-            }
-            umma::fence_after_sync();
-            const uint32_t a = umma::smem_addr(sm + st * Cfg::STAGE), bw = a + Cfg::A_BYTES;
-#pragma unroll
-            for (int r = 0; r < R; r++)
-#pragma unroll
-                for (int dy = 0; dy < 3; dy++)
-#pragma unroll
-                    for (int k = 0; k < 2; k++)
-                        umma::mma_bf16(tmem + (uint32_t)(r * COUT),
-                                       umma::smem_desc_sw64(a + (r + dy) * Cfg::A_ROW + 32 * k),
-                                       umma::smem_desc_sw64(bw + dy * Cfg::B_TAP + 32 * k), idesc,
-                                       (c > 0 || dy > 0 || k > 0) ? 1u : 0u);
-            umma::mma_commit(&empty[st]);
-        }
-        umma::mma_commit(&done);  // arrives when every MMA above has completed
-    }
-    __syncwarp();
-    const bool dok = __all_sync(0xffffffffu, umma::mbar_wait(&done, 0, kWaitLimit));
-    umma::fence_after_sync();
-    if (!dok && lane == 0) atomicOr(err, 4);
-    if (dok) {
-#pragma unroll 1
-        for (int r = 0; r < R; r++) {
-            const size_t p = ((size_t)n * H + h0 + r) * Wd + w0 + tid;  // TMEM lane = pixel
-#pragma unroll 1
-            for (int cc = 0; cc < COUT / 32; cc++) {
-                float v[32];
-                umma::tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(r * COUT + cc * 32),
-                                v);
-                __align__(16) __nv_bfloat16 out[32];
-#pragma unroll
-                for (int i = 0; i < 32; i++) {
-                    float t = v[i] + (bias ? bias[cc * 32 + i] : 0.f);
-                    if (relu) t = fmaxf(t, 0.f);
-                    out[i] = __float2bfloat16(t);
+                        for (int dy = 0; dy < 3; dy++)
+                            umma::tma_load_3d(B + (2 - dy) * Cfg::B_TAP, &tmW, c0, 3 * dy + tap, 0,
+                                              &full[s]);
+                    } else {
+                        umma::tma_load_4d(A, &tmX, c0, w0 + tap % 3 - 1, h0 + tap / 3 - 1, n, &full[s]);
+                        umma::tma_load_3d(B, &tmW, c0, tap, 0, &full[s]);
+                    }
                 }
-                uint4 *dst = reinterpret_cast<uint4 *>(Y + p * ystride + cc * 32);
+            }
+            if (!ok) atomicOr(err, 4);
+        }
+        __syncwarp();
+    } else if (warp == kPipeMma) {
+        const uint32_t sm0 = umma::uniform(umma::smem_addr(sm));
+        bool ok = true;
+        int it = 0, i = 0;
+        for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, i++) {
+            const uint32_t tm = tmem + (uint32_t)((i & 1) * Cfg::COLS);
+            if (i >= 2) ok = umma::mbar_wait_warp(&accfree[i & 1], (uint32_t)(i / 2 - 1) & 1u, kWaitLimit);
+            for (int c = 0; c < nchunks && ok; c++, it++) {
+                const int s = it % ST;
+                ok = umma::mbar_wait_warp(&full[s], (uint32_t)(it / ST) & 1u, kWaitLimit);
+                if (!ok) break;
+                umma::fence_after_sync();
+                const uint32_t a = sm0 + (uint32_t)(s * Cfg::STAGE), bw = a + Cfg::A_BYTES;
+                if (BAND) {
 #pragma unroll
-                for (int q = 0; q < 4; q++) dst[q] = reinterpret_cast<const uint4 *>(out)[q];
+                    for (int half = 0; half < KC / 32; half++)
+#pragma unroll
+                        for (int j = 0; j < R + 2; j++) {
+                            // output rows r0 .. r1, their taps from slab s0 on
+                            const int r0 = j < 2 ? 0 : j - 2, r1 = j < R ? j : R - 1;
+                            const int s0 = j < 2 ? 2 - j : 0;
+                            const uint32_t d = tm + (uint32_t)(r0 * COUT);
+#pragma unroll
+                            for (int k = 2 * half; k < 2 * half + 2; k++) {
+                                const uint64_t ad = desc_k<KC>(a + j * Cfg::A_TILE + 32 * k);
+                                const uint64_t bd = desc_k<KC>(bw + s0 * Cfg::B_TAP + 32 * k);
+                                if (c == 0 && k == 0 && j < R) {
+                                    // output row j starts here (dy = 0, the last slab)
+                                    if (r1 > r0)
+                                        umma::mma_f16_warp(d, ad, bd,
+                                                           umma::idesc_bf16(128, (r1 - r0) * COUT), 1u);
+                                    umma::mma_f16_warp(tm + (uint32_t)(j * COUT), ad,
+                                                       desc_k<KC>(bw + 2 * Cfg::B_TAP),
+                                                       umma::idesc_bf16(128, COUT), 0u);
+                                } else {
+                                    umma::mma_f16_warp(d, ad, bd,
+                                                       umma::idesc_bf16(128, (r1 - r0 + 1) * COUT), 1u);
+                                }
+                            }
+                        }
+                } else {
+#pragma unroll
+                    for (int m = 0; m < R; m++)
+#pragma unroll
+                        for (int k = 0; k < KC / 16; k++)
+                            umma::mma_f16_warp(tm + (uint32_t)(m * COUT),
+                                               desc_k<KC>(a + m * Cfg::A_TILE + 32 * k),
+                                               desc_k<KC>(bw + 32 * k), umma::idesc_bf16(128, COUT),
+                                               (c > 0 || k > 0) ? 1u : 0u);
+                }
+                umma::mma_commit_warp(&empty[s]);
+            }
+            if (ok) umma::mma_commit_warp(&accfull[i & 1]);
+        }
+        if (!ok && lane == 0) atomicOr(err, 4);
+        __syncwarp();
+    } else {
+        // TMEM lane = pixel of a tile, this warp's from 32 warp on
+        unsigned char *out = sm + ST * Cfg::STAGE + warp * Cfg::NOUT * Cfg::OUT;
+        const int pw = (32 * warp) & ((1 << lw) - 1), ph = (32 * warp) >> lw;
+        bool ok = true;
+        int i = 0, q = 0;
+        for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, i++) {
+            const int w0 = (t % wt << lw) + pw, h0 = t / wt % ht * hb + ph, n = t / wt / ht;
+            ok = __all_sync(0xffffffffu,
+                            umma::mbar_wait(&accfull[i & 1], (uint32_t)(i / 2) & 1u, kWaitLimit));
+            if (!ok) break;
+            umma::fence_after_sync();
+            const uint32_t tm = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)((i & 1) * Cfg::COLS);
+#pragma unroll 1
+            for (int cc = 0; cc < Cfg::COLS / 32; cc++) {
+                const int m = cc / (COUT / 32), c0 = cc % (COUT / 32) * 32;
+                const int h = h0 + (BAND ? m : m * (128 >> lw));
+                float v[32];
+                umma::tmem_ld32(tm + (uint32_t)(cc * 32), v);
+                if (cc == Cfg::COLS / 32 - 1) {
+                    umma::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) umma::mbar_arrive(&accfree[i & 1]);
+                }
+                if (w0 >= Wd || h >= H) continue;  // uniform over the warp
+                if (lane == 0) umma::tma_store_wait_read<Cfg::NOUT - 1>();
+                __syncwarp();
+                const float4 *bs = reinterpret_cast<const float4 *>(s_bias + c0);
+#pragma unroll
+                for (int g = 0; g < 4; g++) {  // 8 channels, 16 bytes, swizzled as the map has it
+                    const float4 b0 = bs[2 * g], b1 = bs[2 * g + 1];
+                    const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+                    __align__(16) __nv_bfloat16 o[8];
+#pragma unroll
+                    for (int e = 0; e < 8; e++) {
+                        float f = v[8 * g + e] + bb[e];
+                        if (relu) f = fmaxf(f, 0.f);
+                        o[e] = __float2bfloat16(f);
+                    }
+                    *reinterpret_cast<uint4 *>(out + q * Cfg::OUT + lane * 64 +
+                                               ((g ^ ((lane >> 1) & 3)) << 4)) =
+                        *reinterpret_cast<const uint4 *>(o);
+                }
+                umma::fence_async_smem();
+                __syncwarp();
+                if (lane == 0) umma::tma_store_4d(&tmY, out + q * Cfg::OUT, c0, w0, h, n);
+                q = (q + 1) % Cfg::NOUT;
             }
         }
+        if (!ok && lane == 0) atomicOr(err, 4);
+        if (lane == 0) umma::tma_store_wait_read<0>();
+        __syncwarp();
     }
     umma::fence_before_sync();
     __syncthreads();
-    if (warp == 0) umma::tmem_dealloc(tmem, Cfg::NCOLS);
+    if (warp == kPipeLoad) umma::tmem_dealloc(tmem, Cfg::NCOLS);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
@@ -499,80 +493,105 @@ bool encode_sino_map(CUtensorMap *m, const float *base, int ys, int nx, int na, 
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// NHWC bf16 tensor [N][H][W][C]: box = 32 channels x box_w x box_h pixels of
-// one image, 64-byte swizzle; false if the CUDA driver refuses it.
+// Swizzle of boxes whose rows are kc (32 or 64) bf16 channels.
+static CUtensorMapSwizzle swizzle_for(int kc) {
+    return kc == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+}
+
+// NHWC bf16 tensor [N][H][W][C]: box = kc (32 or 64) channels x box_w x box_h
+// pixels of one image, 64 or 128-byte swizzle; false if the CUDA driver refuses it.
 bool encode_nhwc_map(CUtensorMap *m, const void *base, int N, int H, int W, int C, int box_w,
-                     int box_h) {
+                     int box_h, int kc) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return false;
     const cuuint64_t d[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
     const cuuint64_t s[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
-    const cuuint32_t b[4] = {32, (cuuint32_t)box_w, (cuuint32_t)box_h, 1};
+    const cuuint32_t b[4] = {(cuuint32_t)kc, (cuuint32_t)box_w, (cuuint32_t)box_h, 1};
     const cuuint32_t one[4] = {1, 1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)base, d, s, b, one,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(kc),
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // Tensor maps of one convolution; false if the CUDA driver refuses them (the
 // caller then uses the gather kernel).
-static bool conv_tensor_maps(const __nv_bfloat16 *x, const __nv_bfloat16 *w, int N, int H, int Wd,
-                             int Cin, int Cout, CUtensorMap *tx, CUtensorMap *tw, int box_rows = 1) {
+struct ConvMaps {
+    CUtensorMap x, w, y;
+};
+static bool conv_tensor_maps(const __nv_bfloat16 *x, const __nv_bfloat16 *w, __nv_bfloat16 *y, int N,
+                             int H, int Wd, int Cin, int Cout, int ystride, int box_w, int box_h, int kc,
+                             ConvMaps *m) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return false;
-    static_assert(kConvKC == 32, "encode_nhwc_map's box");
-    if (!encode_nhwc_map(tx, x, N, H, Wd, Cin, 128, box_rows)) return false;
-    const cuuint32_t one[3] = {1, 1, 1};
+    if (!encode_nhwc_map(&m->x, x, N, H, Wd, Cin, box_w, box_h, kc)) return false;
+    const cuuint32_t one[4] = {1, 1, 1, 1};
     const cuuint64_t wd[3] = {(cuuint64_t)Cin, 9, (cuuint64_t)Cout};
     const cuuint64_t ws[2] = {(cuuint64_t)Cin * 2, (cuuint64_t)9 * Cin * 2};
-    const cuuint32_t wb[3] = {(cuuint32_t)kConvKC, 1, (cuuint32_t)Cout};
-    return enc(tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void *)w, wd, ws, wb, one,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    const cuuint32_t wb[3] = {(cuuint32_t)kc, 1, (cuuint32_t)Cout};
+    if (enc(&m->w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void *)w, wd, ws, wb, one,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(kc), CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
+    // stores: a warp's 32 pixels x 32 channels
+    const cuuint64_t yd[4] = {(cuuint64_t)Cout, (cuuint64_t)Wd, (cuuint64_t)H, (cuuint64_t)N};
+    const cuuint64_t row = (cuuint64_t)ystride * 2;
+    const cuuint64_t ys[3] = {row, row * Wd, row * Wd * H};
+    const cuuint32_t bw = box_w < 32 ? (cuuint32_t)box_w : 32;
+    const cuuint32_t yb[4] = {32, bw, 32 / bw, 1};
+    return enc(&m->y, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)y, yd, ys, yb, one,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int COUT>
-static int launch_conv_tma(const CUtensorMap &tx, const CUtensorMap &tw, const float *bias,
-                           __nv_bfloat16 *Y, int H, int Wd, int Cin, int P, int relu, int ystride,
-                           int *err, cudaStream_t st) {
-    using Cfg = TmaCfg<COUT>;
-    static bool configured = false;
-    if (!configured) {
-        ARECGB_CUDA(cudaFuncSetAttribute(conv3x3_tma_kernel<COUT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
-        configured = true;
+// Width 2^lw of a 128-pixel tile: the widest of those that cover the image with
+// the fewest tiles.
+static int conv_tile(int H, int Wd) {
+    int best = 7;
+    long long least = -1;
+    for (int lw = 7; lw >= 3; lw--) {
+        const int hb = 128 >> lw;
+        const long long t = (long long)((Wd + (1 << lw) - 1) >> lw) * ((H + hb - 1) / hb);
+        if (least < 0 || t < least) best = lw, least = t;
     }
-    conv3x3_tma_kernel<COUT><<<P / 128, 128, Cfg::SMEM, st>>>(tx, tw, bias, Y, H, Wd, Cin, relu,
-                                                              ystride, err);
+    return best;
+}
+
+static int sm_count() {
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+// -1: no tensor maps.
+template <int COUT, int R, bool BAND, int KC, int ST>
+static int launch_conv_pipe(const __nv_bfloat16 *x, const __nv_bfloat16 *w, const float *bias,
+                            __nv_bfloat16 *y, int N, int H, int Wd, int Cin, int lw, int relu,
+                            int ystride, int *err, cudaStream_t st) {
+    using Cfg = PipeCfg<COUT, R, BAND, KC, ST>;
+    const int hb = BAND ? R : (128 >> lw) * R;
+    ConvMaps m;
+    if (!conv_tensor_maps(x, w, y, N, H, Wd, Cin, COUT, ystride, 1 << lw, BAND ? R + 2 : hb, KC,
+                          &m))
+        return -1;
+    static std::once_flag once;
+    static cudaError_t attr = cudaSuccess;
+    std::call_once(once, [] {
+        attr = cudaFuncSetAttribute(conv3x3_pipe_kernel<COUT, R, BAND, KC, ST>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
+    });
+    ARECGB_CUDA(attr);
+    const int wt = (Wd + (1 << lw) - 1) >> lw, ht = (H + hb - 1) / hb, ntiles = N * wt * ht;
+    const int sms = sm_count();
+    conv3x3_pipe_kernel<COUT, R, BAND, KC, ST><<<ntiles < sms ? ntiles : sms, kPipeThreads, Cfg::SMEM, st>>>(
+        m.x, m.w, m.y, bias, H, Wd, Cin, lw, relu, wt, ht, ntiles, err);
     ARECGB_CUDA(cudaGetLastError());
     return 0;
 }
 
-template <int COUT, int R>
-static int launch_conv_rows(const CUtensorMap &tx, const CUtensorMap &tw, const float *bias,
-                            __nv_bfloat16 *Y, int N, int H, int Wd, int Cin, int relu, int ystride,
-                            int *err, cudaStream_t st) {
-    using Cfg = RowsCfg<COUT, R>;
-    static bool configured = false;
-    if (!configured) {
-        ARECGB_CUDA(cudaFuncSetAttribute(conv3x3_rows_kernel<COUT, R>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
-        configured = true;
-    }
-    conv3x3_rows_kernel<COUT, R><<<N * (H / R) * (Wd / 128), 128, Cfg::SMEM, st>>>(
-        tx, tw, bias, Y, H, Wd, Cin, relu, ystride, err);
-    ARECGB_CUDA(cudaGetLastError());
-    return 0;
-}
-
-// Output rows per block of the multi-row TMA kernel: 4 for 32 output channels,
-// 2 for 64 (two blocks per SM fit in shared memory), else 1 (the one-row kernel).
-static int conv_rows_for(int Cout) { return Cout == 32 ? 4 : (Cout == 64 ? 2 : 1); }
-
-// layout: 0 = TMA path when the width is a multiple of 128, else the gather
-//         kernel with (LBO 128, SBO 256) [K-halves 128 B apart, row groups 256 B
-//         apart]; 1 = the gather kernel with the two offsets exchanged (for
-//         validating the descriptor fields); 2 = the gather kernel always.
+// layout: 0 = TMA path; 1 = the gather kernel with (LBO 256, SBO 128) (for
+//         validating the descriptor fields); 2 = the gather kernel with
+//         (LBO 128, SBO 256) [K-halves 128 B apart, row groups 256 B apart].
 int conv3x3_bf16(const void *X, const void *Wt, const float *bias, void *Y, int N, int H, int Wd,
                  int Cin, int Cout, int relu, int layout, int *err, cudaStream_t st, int ystride) {
     if (ystride <= 0) ystride = Cout;
@@ -585,21 +604,38 @@ int conv3x3_bf16(const void *X, const void *Wt, const float *bias, void *Y, int 
     const auto *w = reinterpret_cast<const __nv_bfloat16 *>(Wt);
     auto *y = reinterpret_cast<__nv_bfloat16 *>(Y);
     const int P = N * H * Wd;
-    if (layout == 0 && Wd % 128 == 0) {
-        CUtensorMap tx, tw;
-        const int R = conv_rows_for(Cout);
-        if (R > 1 && H % R == 0 && conv_tensor_maps(x, w, N, H, Wd, Cin, Cout, &tx, &tw, R + 2)) {
-            if (Cout == 32)
-                return launch_conv_rows<32, 4>(tx, tw, bias, y, N, H, Wd, Cin, relu, ystride, err, st);
-            if (Cout == 64)
-                return launch_conv_rows<64, 2>(tx, tw, bias, y, N, H, Wd, Cin, relu, ystride, err, st);
+    if (layout == 0) {
+        int rc = -1;
+#define ARECGB_CONV_PIPE(C, R, BAND, KC, ST, LW) \
+    rc = launch_conv_pipe<C, R, BAND, KC, ST>(x, w, bias, y, N, H, Wd, Cin, LW, relu, ystride, err, st)
+        const int lw = conv_tile(H, Wd);
+        const bool wide = Cin % 64 == 0;
+        // Two tiles share a chunk's weights (48 KB loaded for them instead of 64 at
+        // 128 channels) where that leaves every SM a pair.  Bands: as many rows as
+        // two stages of their chunks leave room for.
+        const bool pairs = (P + 255) / 256 >= sm_count();
+        if (Cout == 32 && Wd % 128 == 0 && H % 4 == 0) {
+            if (wide) ARECGB_CONV_PIPE(32, 4, true, 64, 2, 7);
+            else ARECGB_CONV_PIPE(32, 4, true, 32, 3, 7);
+        } else if (Cout == 64 && Wd % 128 == 0 && H % 2 == 0) {
+            if (wide) ARECGB_CONV_PIPE(64, 3, true, 64, 2, 7);
+            else ARECGB_CONV_PIPE(64, 4, true, 32, 3, 7);
+        } else if (Cout == 32) {
+            if (wide) ARECGB_CONV_PIPE(32, 2, false, 64, 5, lw);
+            else ARECGB_CONV_PIPE(32, 2, false, 32, 8, lw);
+        } else if (Cout == 64) {
+            if (wide) ARECGB_CONV_PIPE(64, 2, false, 64, 4, lw);
+            else ARECGB_CONV_PIPE(64, 2, false, 32, 8, lw);
+        } else if (Cout == 128) {
+            if (wide && pairs) ARECGB_CONV_PIPE(128, 2, false, 64, 4, lw);
+            else if (wide) ARECGB_CONV_PIPE(128, 1, false, 64, 6, lw);
+            else ARECGB_CONV_PIPE(128, 2, false, 32, 8, lw);
+        } else if (Cout == 256) {
+            if (wide) ARECGB_CONV_PIPE(256, 1, false, 64, 4, lw);
+            else ARECGB_CONV_PIPE(256, 1, false, 32, 8, lw);
         }
-        if (conv_tensor_maps(x, w, N, H, Wd, Cin, Cout, &tx, &tw)) {
-#define ARECGB_CONV_TMA(C) \
-    if (Cout == C) return launch_conv_tma<C>(tx, tw, bias, y, H, Wd, Cin, P, relu, ystride, err, st);
-            ARECGB_CONV_TMA(32) ARECGB_CONV_TMA(64) ARECGB_CONV_TMA(128) ARECGB_CONV_TMA(256)
-#undef ARECGB_CONV_TMA
-        }
+#undef ARECGB_CONV_PIPE
+        if (rc >= 0) return rc;
     }
     if (layout == 2) layout = 0;
 #define ARECGB_CONV(C)                                                                     \

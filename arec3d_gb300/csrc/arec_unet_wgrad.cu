@@ -12,7 +12,7 @@
 // dpre's blocks (zero outside: ragged chunks add nothing), 64-byte swizzle.
 // Eight pixels of a 32-channel block are one 512-byte swizzle atom, so dy is an
 // offset of 512 bytes and a K step of 16 pixels one of 1024; the 32-channel
-// blocks of a tile lie one region apart.  One thread issues the loads, one the
+// blocks of a tile lie one region apart.  One thread issues the loads, one warp the
 // MMAs (four K steps per chunk and tile, starting from zero); twelve warps add
 // each chunk's accumulators from TMEM to FP32 registers (up to 12 blocks of 32
 // columns, 4 per warp) and at the end to gw (FP32 atomics).
@@ -23,8 +23,10 @@
 // sign (the CUDA-core kernel it replaces 2.0e-7, and 6.0e-7 on data of both
 // signs); four steps per chunk and rounded adds give 1.9e-7 and 2.9e-7.
 // Time of that layer 3.08 -> 0.21 ms, 256 -> 256 at 16 x 32^2 2.49 -> 0.08 ms,
-// one training batch's gradient (16 x 256^2) 63.5 -> 6.5 ms.  Splits: dy, ci and co are divided over blocks when their tiles
-// exceed 384 TMEM columns; the pixel chunks over as many blocks as fill the SMs.
+// one training batch's gradient (16 x 256^2) 63.5 -> 6.5 ms; with the MMAs issued by
+// a whole warp all layers of it take 1.50 ms instead of 1.90.  Splits: dy, ci and co
+// are divided over blocks when their tiles exceed 384 TMEM columns; the pixel chunks
+// over as many blocks as fill the SMs.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -38,7 +40,7 @@
 namespace arecgb {
 
 bool encode_nhwc_map(CUtensorMap *m, const void *base, int N, int H, int W, int C, int box_w,
-                     int box_h);
+                     int box_h, int kc);
 
 namespace unet {
 
@@ -86,7 +88,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
     __shared__ uint32_t tmem_base;
     const uint32_t raw = umma::smem_addr(sm_raw);
     unsigned char *sm = sm_raw + ((1024u - (raw & 1023u)) & 1023u);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = umma::uniform(tid >> 5), lane = tid & 31;
     int job = blockIdx.y;
     const int dy0 = J.ndy == 3 ? 0 : job % 3;
     if (J.ndy != 3) job /= 3;
@@ -138,30 +140,30 @@ __global__ void __launch_bounds__(kWgThreads, 1)
             }
         __syncwarp();
     } else if (warp == kEpiWarps + 1) {
-        if (lane == 0) {
-            // BF16 operands, both MN-major (bits 15, 16)
-            const uint32_t idesc = umma::idesc_bf16(128, N) | (1u << 15) | (1u << 16);
-            for (int it = 0; it < nc; it++) {
-                const int s = it % J.stages, b = it % J.bufs, use = it / J.bufs;
-                if (!umma::mbar_wait(&full[s], (uint32_t)(it / J.stages) & 1u, kWgWait) ||
-                    (use > 0 && !umma::mbar_wait(&accfree[b], (uint32_t)(use - 1) & 1u, kWgWait))) {
-                    atomicOr(err, 4);
-                    break;
-                }
-                umma::fence_after_sync();
-                const uint32_t x = umma::smem_addr(sm + (size_t)s * J.stage), d = x + nreg * J.region;
-                for (int k = 0; k < kPix * kPix / 16; k++) {
-                    const uint64_t bd = desc_mn_sw64(d + k * 1024, kDBlock);
-                    for (int dy = 0; dy < J.ndy; dy++)
-                        for (int q = 0; q < J.tiles; q++)
-                            umma::mma_bf16(
-                                tmem + (uint32_t)(b * nblk * 32 + (dy * J.tiles + q) * N),
-                                desc_mn_sw64(x + 4 * q * J.region + dy * kAtom + k * 1024, J.region),
-                                bd, idesc, k > 0 ? 1u : 0u);
-                }
-                umma::mma_commit(&empty[s]);
-                umma::mma_commit(&accfull[b]);
+        // BF16 operands, both MN-major (bits 15, 16)
+        const uint32_t idesc = umma::idesc_bf16(128, N) | (1u << 15) | (1u << 16);
+        const uint32_t tm = umma::uniform(tmem), base = umma::uniform(umma::smem_addr(sm));
+        for (int it = 0; it < nc; it++) {
+            const int s = it % J.stages, b = it % J.bufs, use = it / J.bufs;
+            if (!umma::mbar_wait_warp(&full[s], (uint32_t)(it / J.stages) & 1u, kWgWait) ||
+                (use > 0 && !umma::mbar_wait_warp(&accfree[b], (uint32_t)(use - 1) & 1u, kWgWait))) {
+                if (lane == 0) atomicOr(err, 4);
+                break;
             }
+            umma::fence_after_sync();
+            const uint32_t x = base + (uint32_t)(s * J.stage), d = x + nreg * J.region;
+#pragma unroll
+            for (int k = 0; k < kPix * kPix / 16; k++) {
+                const uint64_t bd = desc_mn_sw64(d + k * 1024, kDBlock);
+                for (int dy = 0; dy < J.ndy; dy++)
+                    for (int q = 0; q < J.tiles; q++)
+                        umma::mma_f16_warp(
+                            tm + (uint32_t)(b * nblk * 32 + (dy * J.tiles + q) * N),
+                            desc_mn_sw64(x + 4 * q * J.region + dy * kAtom + k * 1024, J.region), bd,
+                            idesc, k > 0 ? 1u : 0u);
+            }
+            umma::mma_commit_warp(&empty[s]);
+            umma::mma_commit_warp(&accfull[b]);
         }
         __syncwarp();
     } else {
@@ -241,8 +243,8 @@ int conv_wgrad(const __nv_bfloat16 *x, const __nv_bfloat16 *dpre, float *gw, int
     J.cols = 32;
     while (J.cols < (uint32_t)(J.bufs * set)) J.cols *= 2;
     CUtensorMap tx, td;
-    if (!encode_nhwc_map(&tx, x, N, H, W, Cin, kPix, kPix + J.ndy - 1) ||
-        !encode_nhwc_map(&td, dpre, N, H, W, Cout, kPix, kPix)) {
+    if (!encode_nhwc_map(&tx, x, N, H, W, Cin, kPix, kPix + J.ndy - 1, 32) ||
+        !encode_nhwc_map(&td, dpre, N, H, W, Cout, kPix, kPix, 32)) {
         set_error("conv_wgrad: tensor map encoding failed");
         return ARECGB_ERR_ARG;
     }
