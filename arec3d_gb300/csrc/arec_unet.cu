@@ -67,7 +67,8 @@ struct Net {
     int lastN = 0;
     // training scratch
     __nv_bfloat16 *gX = nullptr, *gY = nullptr, *gpre = nullptr;
-    float *de1 = nullptr, *de2 = nullptr, *de3 = nullptr, *out = nullptr, *dout = nullptr;
+    __nv_bfloat16 *de1 = nullptr, *de2 = nullptr, *de3 = nullptr;  // gradients of the skip tensors
+    float *out = nullptr, *dout = nullptr;
     double *partials = nullptr, *h_partials = nullptr;
     int *err = nullptr;
     std::vector<void *> blocks;  // everything cudaMalloc'd
@@ -200,7 +201,7 @@ static int conv(Net *n, int l, const __nv_bfloat16 *x, __nv_bfloat16 *y, int N, 
 static int forward(Net *n, const float *x, float *y, int N, cudaStream_t st) {
     const int H = n->H, W = n->W;
     const int H1 = H / 2, W1 = W / 2, H2 = H / 4, W2 = W / 4, H3 = H / 8, W3 = W / 8;
-    const size_t P0 = (size_t)N * H * W, P1 = P0 / 4, P2 = P0 / 16;
+    const size_t P0 = (size_t)N * H * W;
     int rc = 0;
     if (!n->mirrors_fresh && (rc = refresh_mirrors(n, st))) return rc;
     conv_in(x, n->params + n->woff[C1A], n->params + n->boff[C1A], n->a1, N, H, W, 32, st);
@@ -268,44 +269,36 @@ static int backward(Net *n, const float *dout, cudaStream_t st) {
     // decoder level 0
     if ((rc = conv_bwd(n, D1B, n->f1, n->g1, 32, gY, 32, gX, N, H, W, st))) return rc;
     if ((rc = conv_bwd(n, D1A, n->cat1, n->f1, 32, gX, 32, gY, N, H, W, st))) return rc;
-    ARECGB_CUDA(cudaMemsetAsync(n->de1, 0, sizeof(float) * P0 * 32, st));
-    chan_add(gY, n->de1, P0, 32, 64, 32, st);
+    chan_take(gY, n->de1, P0, 32, 64, 32, st);
     if ((rc = conv_bwd(n, U1, n->up1, n->cat1, 64, gY, 64, gX, N, H, W, st))) return rc;
     upsample_bwd(gX, gY, N, H1, W1, 64, 64, st);
     // decoder level 1
     if ((rc = conv_bwd(n, D2B, n->f2, n->g2, 64, gY, 64, gX, N, H1, W1, st))) return rc;
     if ((rc = conv_bwd(n, D2A, n->cat2, n->f2, 64, gX, 64, gY, N, H1, W1, st))) return rc;
-    ARECGB_CUDA(cudaMemsetAsync(n->de2, 0, sizeof(float) * P1 * 64, st));
-    chan_add(gY, n->de2, P1, 64, 128, 64, st);
+    chan_take(gY, n->de2, P1, 64, 128, 64, st);
     if ((rc = conv_bwd(n, U2, n->up2, n->cat2, 128, gY, 128, gX, N, H1, W1, st))) return rc;
     upsample_bwd(gX, gY, N, H2, W2, 128, 128, st);
     // decoder level 2
     if ((rc = conv_bwd(n, D3B, n->f3, n->g3, 128, gY, 128, gX, N, H2, W2, st))) return rc;
     if ((rc = conv_bwd(n, D3A, n->cat3, n->f3, 128, gX, 128, gY, N, H2, W2, st))) return rc;
-    ARECGB_CUDA(cudaMemsetAsync(n->de3, 0, sizeof(float) * P2 * 128, st));
-    chan_add(gY, n->de3, P2, 128, 256, 128, st);
+    chan_take(gY, n->de3, P2, 128, 256, 128, st);
     if ((rc = conv_bwd(n, U3, n->up3, n->cat3, 256, gY, 256, gX, N, H2, W2, st))) return rc;
     upsample_bwd(gX, gY, N, H3, W3, 256, 256, st);
     // encoder level 3
     if ((rc = conv_bwd(n, C4B, n->a4, n->e4, 256, gY, 256, gX, N, H3, W3, st))) return rc;
     if ((rc = conv_bwd(n, C4A, n->q3, n->a4, 256, gX, 256, gY, N, H3, W3, st))) return rc;
-    maxpool_bwd(gY, n->arg3, n->de3, N, H2, W2, 128, st);
-    f32_to_bf16(n->de3, gX, P2 * 128, st);
+    skip_grad(n->de3, gY, n->arg3, gX, N, H2, W2, 128, st);
     // encoder level 2
     if ((rc = conv_bwd(n, C3B, n->a3, n->cat3 + 128, 256, gX, 128, gY, N, H2, W2, st))) return rc;
     if ((rc = conv_bwd(n, C3A, n->q2, n->a3, 128, gY, 128, gX, N, H2, W2, st))) return rc;
-    maxpool_bwd(gX, n->arg2, n->de2, N, H1, W1, 64, st);
-    f32_to_bf16(n->de2, gY, P1 * 64, st);
+    skip_grad(n->de2, gX, n->arg2, gY, N, H1, W1, 64, st);
     // encoder level 1
     if ((rc = conv_bwd(n, C2B, n->a2, n->cat2 + 64, 128, gY, 64, gX, N, H1, W1, st))) return rc;
     if ((rc = conv_bwd(n, C2A, n->q1, n->a2, 64, gX, 64, gY, N, H1, W1, st))) return rc;
-    maxpool_bwd(gY, n->arg1, n->de1, N, H, W, 32, st);
-    f32_to_bf16(n->de1, gX, P0 * 32, st);
+    skip_grad(n->de1, gY, n->arg1, gX, N, H, W, 32, st);
     // encoder level 0
     if ((rc = conv_bwd(n, C1B, n->a1, n->cat1 + 32, 64, gX, 32, gY, N, H, W, st))) return rc;
-    relu_bwd(n->a1, gY, n->gpre, P0 * 32, st);
-    conv_in_wgrad(n->in, n->gpre, n->grads + n->woff[C1A], n->grads + n->boff[C1A], N, H, W, 32,
-                  st);
+    conv_in_bwd(n->in, n->a1, gY, n->grads + n->woff[C1A], n->grads + n->boff[C1A], N, H, W, 32, st);
     ARECGB_CUDA(cudaGetLastError());
     return 0;
 }

@@ -18,27 +18,23 @@ namespace unet {
 
 void conv_in(const float *x, const float *w, const float *b, __nv_bfloat16 *y, int N, int H, int W,
              int C, cudaStream_t st);
-void conv_in_wgrad(const float *x, const __nv_bfloat16 *dpre, float *gw, float *gb, int N, int H,
-                   int W, int C, cudaStream_t st);
+void conv_in_bwd(const float *x, const __nv_bfloat16 *y, const __nv_bfloat16 *dy, float *gw, float *gb,
+                 int N, int H, int W, int C, cudaStream_t st);
 void conv_out(const __nv_bfloat16 *h, const float *w, const float *b, const float *x0, float *y,
               size_t P, int C, cudaStream_t st);
 void conv_out_bwd(const __nv_bfloat16 *h, const float *w, const float *dy, __nv_bfloat16 *dh,
                   float *gw, float *gb, size_t P, int C, cudaStream_t st);
 void maxpool(const __nv_bfloat16 *x, __nv_bfloat16 *y, uint8_t *arg, int N, int H, int W, int C,
              cudaStream_t st, int xs = 0);
-void maxpool_bwd(const __nv_bfloat16 *dy, const uint8_t *arg, float *dx_acc, int N, int H, int W,
-                 int C, cudaStream_t st);
+void skip_grad(const __nv_bfloat16 *skip, const __nv_bfloat16 *dy, const uint8_t *arg, __nv_bfloat16 *dx,
+               int N, int H, int W, int C, cudaStream_t st);
 void upsample(const __nv_bfloat16 *x, __nv_bfloat16 *y, int N, int H, int W, int C, int Cy,
               cudaStream_t st);
 void upsample_bwd(const __nv_bfloat16 *dy, __nv_bfloat16 *dx, int N, int H, int W, int C, int Cy,
                   cudaStream_t st);
-void chan_copy(const __nv_bfloat16 *x, __nv_bfloat16 *y, size_t P, int C, int Cy, int off,
+void chan_take(const __nv_bfloat16 *x, __nv_bfloat16 *y, size_t P, int C, int Cx, int off,
                cudaStream_t st);
-void chan_add(const __nv_bfloat16 *src, float *dst, size_t P, int C, int Cs, int off,
-              cudaStream_t st);
 void f32_to_bf16(const float *a, __nv_bfloat16 *b, size_t n, cudaStream_t st);
-void relu_bwd(const __nv_bfloat16 *y, const __nv_bfloat16 *dy, __nv_bfloat16 *dpre, size_t n,
-              cudaStream_t st);
 // dpre[p][c] = dy[p*dys + c] * (y[p*yys + c] > 0), c < C; gb[c] += sum_p dpre[p][c]
 void relu_bwd_bias(const __nv_bfloat16 *y, int yys, const __nv_bfloat16 *dy, int dys,
                    __nv_bfloat16 *dpre, float *gb, size_t P, int C, cudaStream_t st);

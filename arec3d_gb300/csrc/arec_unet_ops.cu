@@ -24,85 +24,177 @@ static int blocks_for(size_t n) {
 #define GRID_STRIDE(i, n) \
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += (size_t)gridDim.x * blockDim.x)
 
-// ---- first layer: 1 -> C channels, 3x3, bias, ReLU (CUDA cores: 9 MACs per output) ---------
-// One thread per pixel and all C channels: the 9 inputs are read once, the
-// outputs leave as 16-byte vectors; per output the FMAs run in tap order from
-// the bias (taps outside the image skipped).
-template <int C>
-__global__ void __launch_bounds__(256)
-    k_conv_in(const float *__restrict__ x, const float *__restrict__ w,
-              const float *__restrict__ b, __nv_bfloat16 *__restrict__ y, int N, int H, int W) {
-    __shared__ float sw[C * 9], sb[C];
-    for (int i = threadIdx.x; i < C * 9; i += blockDim.x) sw[i] = w[i];
-    for (int i = threadIdx.x; i < C; i += blockDim.x) sb[i] = b[i];
-    __syncthreads();
-    const size_t P = (size_t)N * H * W;
-    GRID_STRIDE(p, P) {
-        const int wx = (int)(p % W);
-        const size_t nh = p / W;
-        const int h = (int)(nh % H);
-        const size_t row0 = nh - h;  // first row of this image
-        float v[9];
-        bool in[9];
+// ---- first layer: 1 -> 32 channels, 3x3, bias, ReLU (CUDA cores: 9 MACs per output) --------
+// A warp takes 8 columns (lane / 4) x 32 channels (lane % 4: eight of them, their
+// weights in registers) and runs down kInRows rows with a window of 3 x 3 inputs.
+constexpr int kInC = 32, kInRows = 16;
+
+struct InWindow {
+    const float *col;  // the image's column wx, row 0
+    int H, W, wx;
+    float v[4][3];  // rows h - 1 .. h + 2 (the last one is on its way) from v[(h - h0) % 4] on
+
+    // Row h of the window's columns (0 outside the image).
+    __device__ __forceinline__ void row(float (&r)[3], int h) const {
+        const float *p = col + (ptrdiff_t)h * W;
 #pragma unroll
-        for (int t = 0; t < 9; t++) {
-            const int hh = h + t / 3 - 1, ww = wx + t % 3 - 1;
-            in[t] = hh >= 0 && hh < H && ww >= 0 && ww < W;
-            v[t] = in[t] ? x[(row0 + hh) * W + ww] : 0.f;
-        }
-        uint4 *yp = reinterpret_cast<uint4 *>(y + p * C);
+        for (int d = 0; d < 3; d++)
+            r[d] = h >= 0 && h < H && wx + d > 0 && wx + d <= W ? __ldg(p + d - 1) : 0.f;
+    }
+    __device__ __forceinline__ bool inside(int h, int t) const {
+        const int hh = h + t / 3 - 1, ww = wx + t % 3 - 1;
+        return hh >= 0 && hh < H && ww >= 0 && ww < W;
+    }
+    __device__ __forceinline__ void start(int h0) {
 #pragma unroll
-        for (int q = 0; q < C / 8; q++) {
-            __align__(16) __nv_bfloat16 o[8];
+        for (int i = 0; i < 3; i++) row(v[i], h0 - 1 + i);
+    }
+    // Tap t at the u-th row of four.
+    __device__ __forceinline__ float tap(int u, int t) const { return v[(u + t / 3) & 3][t % 3]; }
+};
+
+// Strip `t` of an N x H x W stack: image, first column and row.
+__device__ __forceinline__ void in_strip(size_t t, int H, int W, size_t &n, int &w0, int &h0) {
+    const int wt = (W + 7) / 8, ht = (H + kInRows - 1) / kInRows;
+    w0 = (int)(t % wt) * 8;
+    h0 = (int)(t / wt % ht) * kInRows;
+    n = t / wt / ht;
+}
+static size_t in_strips(int N, int H, int W) {
+    return (size_t)N * ((W + 7) / 8) * ((H + kInRows - 1) / kInRows);
+}
+
+// Per output the FMAs run in tap order from the bias (taps outside the image
+// skipped).  Bound by the issue of its instructions (288 multiply-adds per pixel, in
+// pairs; the 64 bytes written per pixel would take 160 us at 16 x 1024^2): 438 us
+// there; 752 with one thread per pixel and all channels, whose 288 weights came from
+// shared memory for every pixel.  Rows take turns in the window's registers (a copy
+// from one to the next would wait for the load in flight).
+__global__ void __launch_bounds__(128, 4)
+    k_conv_in(const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ b,
+              __nv_bfloat16 *__restrict__ y, int N, int H, int W, size_t strips) {
+    const int lane = threadIdx.x & 31, q = lane & 3;
+    float2 sw[4][9], sb[4];
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const int c = q * 8 + j;
-                float s = sb[c];
+    for (int j = 0; j < 4; j++) {
+        const int c = q * 8 + 2 * j;
+        sb[j] = make_float2(b[c], b[c + 1]);
+#pragma unroll
+        for (int t = 0; t < 9; t++) sw[j][t] = make_float2(w[c * 9 + t], w[(c + 1) * 9 + t]);
+    }
+    for (size_t s = (size_t)blockIdx.x * 4 + (threadIdx.x >> 5); s < strips; s += (size_t)gridDim.x * 4) {
+        size_t n;
+        int w0, h0;
+        in_strip(s, H, W, n, w0, h0);
+        InWindow win;
+        win.H = H, win.W = W, win.wx = w0 + (lane >> 2);
+        if (win.wx >= W) continue;
+        const bool inner = w0 > 0 && w0 + 8 < W;  // all taps of the strip's columns
+        win.col = x + n * H * W + win.wx;
+        win.start(h0);
+        for (int hu = h0; hu < min(H, h0 + kInRows); hu += 4)
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const int h = hu + u;
+            if (h >= H) break;
+            win.row(win.v[(u + 3) & 3], h + 2);
+            float2 o[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) o[j] = sb[j];
+            const bool all = h > 0 && h + 1 < H && inner;  // uniform over the warp
+            if (all) {
+#pragma unroll
+                for (int t = 0; t < 9; t++) {
+                    const float2 v = make_float2(win.tap(u, t), win.tap(u, t));
+#pragma unroll
+                    for (int j = 0; j < 4; j++) o[j] = __ffma2_rn(sw[j][t], v, o[j]);
+                }
+            } else {
 #pragma unroll
                 for (int t = 0; t < 9; t++)
-                    if (in[t]) s = fmaf(sw[c * 9 + t], v[t], s);
-                o[j] = tobf(fmaxf(s, 0.f));
+                    if (win.inside(h, t)) {
+                        const float2 v = make_float2(win.tap(u, t), win.tap(u, t));
+#pragma unroll
+                        for (int j = 0; j < 4; j++) o[j] = __ffma2_rn(sw[j][t], v, o[j]);
+                    }
             }
-            yp[q] = *reinterpret_cast<const uint4 *>(o);
+            __align__(16) __nv_bfloat162 r[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) r[j] = __floats2bfloat162_rn(fmaxf(o[j].x, 0.f), fmaxf(o[j].y, 0.f));
+            *reinterpret_cast<uint4 *>(y + ((n * H + h) * W + win.wx) * kInC + q * 8) =
+                *reinterpret_cast<const uint4 *>(r);
         }
     }
 }
 
-// weight/bias gradient of the first layer: gw[c][t] += sum_p dpre[p][c] * x[p+t]
-__global__ void k_conv_in_wgrad(const float *__restrict__ x, const __nv_bfloat16 *__restrict__ dpre,
-                                float *__restrict__ gw, float *__restrict__ gb, int N, int H, int W,
-                                int C) {
-    // one block per output channel c; threads over pixels, block reduction
-    const int c = blockIdx.x;
-    float acc[10];
+// Weight and bias gradient of the first layer from the gradient dy of its output y:
+// with dpre = dy where y > 0, gw[c][t] += sum_p dpre[p][c] x[p + t], gb[c] += sum_p
+// dpre[p][c] (pixels with dpre = 0 and taps outside the image skipped).  The sums of a
+// thread's 8 channels stay in registers over its strips; the block adds them at the
+// end, one FP32 atomic per value.  Bound by the reads of y and dy.  With a ReLU pass and a
+// kernel with one channel per block 111 + 342 us at 16 x 256^2, now 96.
+__global__ void __launch_bounds__(128, 4)
+    k_conv_in_bwd(const float *__restrict__ x, const __nv_bfloat16 *__restrict__ y,
+                  const __nv_bfloat16 *__restrict__ dy, float *__restrict__ gw, float *__restrict__ gb,
+                  int N, int H, int W, size_t strips) {
+    __shared__ float red[4][4][80];
+    const int lane = threadIdx.x & 31, q = lane & 3, warp = threadIdx.x >> 5;
+    float acc[8][10];
 #pragma unroll
-    for (int t = 0; t < 10; t++) acc[t] = 0.f;
-    const size_t P = (size_t)N * H * W;
-    for (size_t p = (size_t)blockIdx.y * blockDim.x + threadIdx.x; p < P;
-         p += (size_t)gridDim.y * blockDim.x) {
-        const float d = bf(dpre[p * C + c]);
-        if (d == 0.f) continue;
-        const int n = (int)(p / ((size_t)H * W)), h = (int)((p / W) % H), wx = (int)(p % W);
+    for (int j = 0; j < 8; j++)
 #pragma unroll
-        for (int t = 0; t < 9; t++) {
-            const int hh = h + t / 3 - 1, ww = wx + t % 3 - 1;
-            if (hh >= 0 && hh < H && ww >= 0 && ww < W)
-                acc[t] = fmaf(d, x[((size_t)n * H + hh) * W + ww], acc[t]);
+        for (int t = 0; t < 10; t++) acc[j][t] = 0.f;
+    for (size_t s = (size_t)blockIdx.x * 4 + warp; s < strips; s += (size_t)gridDim.x * 4) {
+        size_t n;
+        int w0, h0;
+        in_strip(s, H, W, n, w0, h0);
+        InWindow win;
+        win.H = H, win.W = W, win.wx = w0 + (lane >> 2);
+        if (win.wx >= W) continue;
+        win.col = x + n * H * W + win.wx;
+        win.start(h0);
+        for (int hu = h0; hu < min(H, h0 + kInRows); hu += 4)
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const int h = hu + u;
+            if (h >= H) break;
+            win.row(win.v[(u + 3) & 3], h + 2);
+            const size_t o = ((n * H + h) * W + win.wx) * kInC + q * 8;
+            const uint4 yv = *reinterpret_cast<const uint4 *>(y + o);
+            const uint4 dv = *reinterpret_cast<const uint4 *>(dy + o);
+            const __nv_bfloat16 *yb = reinterpret_cast<const __nv_bfloat16 *>(&yv);
+            const __nv_bfloat16 *db = reinterpret_cast<const __nv_bfloat16 *>(&dv);
+            float d[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                d[j] = bf(yb[j]) > 0.f ? bf(db[j]) : 0.f;
+                acc[j][9] += d[j];
+            }
+#pragma unroll
+            for (int t = 0; t < 9; t++)
+                if (win.inside(h, t)) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        if (d[j] != 0.f) acc[j][t] = fmaf(d[j], win.tap(u, t), acc[j][t]);
+                }
         }
-        acc[9] += d;
     }
-    __shared__ float red[10][256];
+    // lanes of the same channels, then the block's warps
 #pragma unroll
-    for (int t = 0; t < 10; t++) red[t][threadIdx.x] = acc[t];
+    for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int t = 0; t < 10; t++) {
+            float v = acc[j][t];
+            for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane < 4) red[warp][q][j * 10 + t] = v;
+        }
     __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o)
-#pragma unroll
-            for (int t = 0; t < 10; t++) red[t][threadIdx.x] += red[t][threadIdx.x + o];
-        __syncthreads();
+    for (int i = threadIdx.x; i < 320; i += 128) {
+        const int c = i / 10, t = i % 10;
+        float v = 0.f;
+        for (int k = 0; k < 4; k++) v += red[k][c / 8][c % 8 * 10 + t];
+        atomicAdd(t < 9 ? &gw[c * 9 + t] : &gb[c], v);
     }
-    if (threadIdx.x < 9) atomicAdd(&gw[c * 9 + threadIdx.x], red[threadIdx.x][0]);
-    if (threadIdx.x == 9) atomicAdd(&gb[c], red[9][0]);
 }
 
 // ---- last layer: 1x1, C -> 1, plus the residual input --------------------------------------
@@ -210,18 +302,39 @@ __global__ void k_maxpool(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__
     }
 }
 
-__global__ void k_maxpool_bwd(const __nv_bfloat16 *__restrict__ dy, const uint8_t *__restrict__ arg,
-                              float *__restrict__ dx_acc, int N, int H, int W, int C) {
-    // dx_acc (fp32, zeroed by the caller) += routed gradient
-    const int Ho = H / 2, Wo = W / 2;
-    const size_t n_out = (size_t)N * Ho * Wo * C;
+// Gradient of a level's skip tensor: dx = skip + (the pooled gradient dy at the arg
+// max of its 2 x 2 pixels, 0 elsewhere), summed in FP32, one thread per pooled pixel
+// and 8 channels.  Bound by its traffic (12 bytes per pooled value and pixel).  An
+// FP32 accumulator cleared, added to twice and rounded took 90 + 56 + 60 us and a
+// clearing pass at 16 x 256^2 x 32.
+__global__ void k_skip_grad(const __nv_bfloat16 *__restrict__ skip, const __nv_bfloat16 *__restrict__ dy,
+                            const uint8_t *__restrict__ arg, __nv_bfloat16 *__restrict__ dx, int N, int H,
+                            int W, int C) {
+    const int Ho = H / 2, Wo = W / 2, C8 = C / 8;
+    const size_t n_out = (size_t)N * Ho * Wo * C8;
     GRID_STRIDE(i, n_out) {
-        const int c = (int)(i % C);
-        const size_t po = i / C;
-        const int n = (int)(po / ((size_t)Ho * Wo)), ho = (int)((po / Wo) % Ho), wo = (int)(po % Wo);
-        const int t = arg[i];
-        const int h = 2 * ho + (t >> 1), w = 2 * wo + (t & 1);
-        dx_acc[(((size_t)n * H + h) * W + w) * C + c] += bf(dy[i]);
+        const int g = (int)(i % C8);
+        const size_t po = i / C8;
+        const int wo = (int)(po % Wo);
+        const size_t top = (2 * (po / Wo)) * W + 2 * wo;
+        const uint4 dv = *reinterpret_cast<const uint4 *>(dy + po * C + g * 8);
+        const uint2 av = *reinterpret_cast<const uint2 *>(arg + po * C + g * 8);
+        const __nv_bfloat16 *db = reinterpret_cast<const __nv_bfloat16 *>(&dv);
+        const uint8_t *ab = reinterpret_cast<const uint8_t *>(&av);
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            const size_t o = (top + (size_t)(t >> 1) * W + (t & 1)) * C + g * 8;
+            const uint4 sv = *reinterpret_cast<const uint4 *>(skip + o);
+            const __nv_bfloat16 *sb = reinterpret_cast<const __nv_bfloat16 *>(&sv);
+            __align__(16) __nv_bfloat16 r[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                float v = 0.f + bf(sb[j]);
+                if (ab[j] == t) v += bf(db[j]);
+                r[j] = tobf(v);
+            }
+            *reinterpret_cast<uint4 *>(dx + o) = *reinterpret_cast<const uint4 *>(r);
+        }
     }
 }
 
@@ -246,53 +359,55 @@ __global__ void k_upsample(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *_
     }
 }
 
-// dx[n][h][w][c] = sum over the 2x2 children of dy (channels [0, C) of a Cy-channel tensor)
+// dx[n][h][w][c] = sum over the 2x2 children of dy (channels [0, C) of a Cy-channel
+// tensor); one thread per pixel and 8 channels (one channel each: 112 us at
+// 16 x 128^2 x 64, a quarter of the sectors' bytes per load)
 __global__ void k_upsample_bwd(const __nv_bfloat16 *__restrict__ dy, __nv_bfloat16 *__restrict__ dx,
                                int N, int H, int W, int C, int Cy) {
-    const size_t n_in = (size_t)N * H * W * C;
+    const int C8 = C / 8;
+    const size_t n_in = (size_t)N * H * W * C8;
     GRID_STRIDE(i, n_in) {
-        const int c = (int)(i % C);
-        const size_t p = i / C;
-        const int n = (int)(p / ((size_t)H * W)), h = (int)((p / W) % H), w = (int)(p % W);
-        float s = 0.f;
+        const int g = (int)(i % C8);
+        const size_t p = i / C8;
+        const int w = (int)(p % W);
+        const size_t nh = p / W;  // n * H + h
+        const size_t o0 = ((2 * nh) * (2 * W) + 2 * w) * Cy + g * 8;  // row 2h, column 2w
+        float s[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) s[j] = 0.f;
 #pragma unroll
         for (int t = 0; t < 4; t++) {
-            const int hh = 2 * h + (t >> 1), ww = 2 * w + (t & 1);
-            s += bf(dy[(((size_t)n * 2 * H + hh) * 2 * W + ww) * Cy + c]);
+            const uint4 v = *reinterpret_cast<const uint4 *>(dy + o0 + (size_t)(t >> 1) * 2 * W * Cy +
+                                                             (t & 1) * Cy);
+            const __nv_bfloat16 *b = reinterpret_cast<const __nv_bfloat16 *>(&v);
+#pragma unroll
+            for (int j = 0; j < 8; j++) s[j] += bf(b[j]);
         }
-        dx[i] = tobf(s);
+        __align__(16) __nv_bfloat16 r[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) r[j] = tobf(s[j]);
+        *reinterpret_cast<uint4 *>(dx + p * C + g * 8) = *reinterpret_cast<const uint4 *>(r);
     }
 }
 
-// copy x [P][C] into channels [off, off+C) of y [P][Cy]
-__global__ void k_chan_copy(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ y,
-                            size_t P, int C, int Cy, int off) {
-    const int C8 = C / 8;  // 16-byte vectors (C, Cy, off multiples of 8)
+// y [P][C] = channels [off, off + C) of x [P][Cx]
+__global__ void k_chan_take(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ y,
+                            size_t P, int C, int Cx, int off) {
+    const int C8 = C / 8;  // 16-byte vectors (C, Cx, off multiples of 8)
     GRID_STRIDE(i, P * C8) {
         const size_t p = i / C8;
         const int g = (int)(i % C8);
-        *reinterpret_cast<uint4 *>(y + p * Cy + off + g * 8) =
-            *reinterpret_cast<const uint4 *>(x + p * C + g * 8);
+        *reinterpret_cast<uint4 *>(y + p * C + g * 8) =
+            *reinterpret_cast<const uint4 *>(x + p * Cx + off + g * 8);
     }
-}
-
-// dst[P][C] (fp32 accumulator) += channels [off, off+C) of src [P][Cs]
-__global__ void k_chan_add(const __nv_bfloat16 *__restrict__ src, float *__restrict__ dst, size_t P,
-                           int C, int Cs, int off) {
-    GRID_STRIDE(i, P * C) { dst[i] += bf(src[(i / C) * Cs + off + (i % C)]); }
 }
 
 __global__ void k_f32_to_bf16(const float *__restrict__ a, __nv_bfloat16 *__restrict__ b, size_t n) {
     GRID_STRIDE(i, n) { b[i] = tobf(a[i]); }
 }
 
-// dpre = dy * (y > 0) (ReLU backward on the post-activation output)
-__global__ void k_relu_bwd(const __nv_bfloat16 *__restrict__ y, const __nv_bfloat16 *__restrict__ dy,
-                           __nv_bfloat16 *__restrict__ dpre, size_t n) {
-    GRID_STRIDE(i, n) { dpre[i] = bf(y[i]) > 0.f ? dy[i] : tobf(0.f); }
-}
-
-// The same with row strides, and the bias gradient gb[c] += sum_p dpre[p][c].
+// dpre = dy * (y > 0) (ReLU backward on the post-activation output; row strides) and
+// the bias gradient gb[c] += sum_p dpre[p][c].
 // One thread per pixel and 8 channels (16-byte vectors); a thread keeps its
 // channels over its pixels, so the sums stay in registers until the block adds
 // them (FP32, one atomic per channel and block).  C a power of two in [32, 256].
@@ -480,14 +595,16 @@ __global__ void k_sumsq_partial(const float *__restrict__ a, size_t n, double *_
 // ---- host launchers -----------------------------------------------------------------------
 void conv_in(const float *x, const float *w, const float *b, __nv_bfloat16 *y, int N, int H, int W,
              int C, cudaStream_t st) {
-    if (C != 32) return;  // the network's first layer (32 channels)
-    k_conv_in<32><<<blocks_for((size_t)N * H * W), 256, 0, st>>>(x, w, b, y, N, H, W);
+    if (C != kInC) return;  // the network's first layer (32 channels)
+    const size_t strips = in_strips(N, H, W);
+    k_conv_in<<<(int)std::min<size_t>((strips + 3) / 4, 152 * 16), 128, 0, st>>>(x, w, b, y, N, H, W, strips);
 }
-void conv_in_wgrad(const float *x, const __nv_bfloat16 *dpre, float *gw, float *gb, int N, int H,
-                   int W, int C, cudaStream_t st) {
-    const size_t P = (size_t)N * H * W;
-    int gy = (int)std::min<size_t>(64, (P + 255) / 256);
-    k_conv_in_wgrad<<<dim3(C, gy), 256, 0, st>>>(x, dpre, gw, gb, N, H, W, C);
+void conv_in_bwd(const float *x, const __nv_bfloat16 *y, const __nv_bfloat16 *dy, float *gw, float *gb,
+                 int N, int H, int W, int C, cudaStream_t st) {
+    if (C != kInC) return;
+    const size_t strips = in_strips(N, H, W);
+    k_conv_in_bwd<<<(int)std::min<size_t>((strips + 3) / 4, 152 * 4), 128, 0, st>>>(x, y, dy, gw, gb, N, H,
+                                                                                    W, strips);
 }
 void conv_out(const __nv_bfloat16 *h, const float *w, const float *b, const float *x0, float *y,
               size_t P, int C, cudaStream_t st) {
@@ -506,9 +623,9 @@ void maxpool(const __nv_bfloat16 *x, __nv_bfloat16 *y, uint8_t *arg, int N, int 
     k_maxpool<<<blocks_for((size_t)N * H * W * C / 32), 256, 0, st>>>(x, y, arg, N, H, W, C,
                                                                       xs > 0 ? xs : C);
 }
-void maxpool_bwd(const __nv_bfloat16 *dy, const uint8_t *arg, float *dx_acc, int N, int H, int W,
-                 int C, cudaStream_t st) {
-    k_maxpool_bwd<<<blocks_for((size_t)N * H * W * C / 4), 256, 0, st>>>(dy, arg, dx_acc, N, H, W, C);
+void skip_grad(const __nv_bfloat16 *skip, const __nv_bfloat16 *dy, const uint8_t *arg, __nv_bfloat16 *dx,
+               int N, int H, int W, int C, cudaStream_t st) {
+    k_skip_grad<<<blocks_for((size_t)N * H * W * C / 32), 256, 0, st>>>(skip, dy, arg, dx, N, H, W, C);
 }
 void upsample(const __nv_bfloat16 *x, __nv_bfloat16 *y, int N, int H, int W, int C, int Cy,
               cudaStream_t st) {
@@ -516,22 +633,14 @@ void upsample(const __nv_bfloat16 *x, __nv_bfloat16 *y, int N, int H, int W, int
 }
 void upsample_bwd(const __nv_bfloat16 *dy, __nv_bfloat16 *dx, int N, int H, int W, int C, int Cy,
                   cudaStream_t st) {
-    k_upsample_bwd<<<blocks_for((size_t)N * H * W * C), 256, 0, st>>>(dy, dx, N, H, W, C, Cy);
+    k_upsample_bwd<<<blocks_for((size_t)N * H * W * C / 8), 256, 0, st>>>(dy, dx, N, H, W, C, Cy);
 }
-void chan_copy(const __nv_bfloat16 *x, __nv_bfloat16 *y, size_t P, int C, int Cy, int off,
+void chan_take(const __nv_bfloat16 *x, __nv_bfloat16 *y, size_t P, int C, int Cx, int off,
                cudaStream_t st) {
-    k_chan_copy<<<blocks_for(P * C / 8), 256, 0, st>>>(x, y, P, C, Cy, off);
-}
-void chan_add(const __nv_bfloat16 *src, float *dst, size_t P, int C, int Cs, int off,
-              cudaStream_t st) {
-    k_chan_add<<<blocks_for(P * C), 256, 0, st>>>(src, dst, P, C, Cs, off);
+    k_chan_take<<<blocks_for(P * C / 8), 256, 0, st>>>(x, y, P, C, Cx, off);
 }
 void f32_to_bf16(const float *a, __nv_bfloat16 *b, size_t n, cudaStream_t st) {
     k_f32_to_bf16<<<blocks_for(n), 256, 0, st>>>(a, b, n);
-}
-void relu_bwd(const __nv_bfloat16 *y, const __nv_bfloat16 *dy, __nv_bfloat16 *dpre, size_t n,
-              cudaStream_t st) {
-    k_relu_bwd<<<blocks_for(n), 256, 0, st>>>(y, dy, dpre, n);
 }
 void relu_bwd_bias(const __nv_bfloat16 *y, int yys, const __nv_bfloat16 *dy, int dys,
                    __nv_bfloat16 *dpre, float *gb, size_t P, int C, cudaStream_t st) {
