@@ -195,8 +195,16 @@ __device__ __forceinline__ void cp_async_wait() {
 // 0)); the second piece of VEC = 8 is 128 floats further.
 template <int VEC>
 __device__ __forceinline__ void lds_lane_if(unsigned pred, unsigned a, float (&v)[VEC]) {
-    static_assert(VEC == 4 || VEC == 8, "one or two float4 pieces");
-    if constexpr (VEC == 8) {
+    if constexpr (VEC == 1) {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p ld.shared.f32 %0, [%2];\n\t}\n"
+                     : "+f"(v[0])
+                     : "r"(pred), "r"(a));
+    } else if constexpr (VEC == 2) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.shared.v2.f32 {%0, %1}, [%3];\n\t}\n"
+            : "+f"(v[0]), "+f"(v[1])
+            : "r"(pred), "r"(a));
+    } else if constexpr (VEC == 8) {
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %8, 0;\n\t"
             "@p ld.shared.v4.f32 {%0, %1, %2, %3}, [%9];\n\t"
@@ -246,7 +254,12 @@ __device__ __forceinline__ void fma_row(float (&acc)[VEC], float w, const float 
 constexpr int kBpAngles = 32;  // angles per weight chunk
 constexpr int kBpFoot = 12;    // staged footprint width in bins (an 8x4 tile spans <= 11)
 
-constexpr int kBpBuf = 3;  // footprint buffers in flight
+// Footprint buffers in flight: three where several blocks per SM hide a copy's
+// latency, eight for narrow plans (few slices: few blocks, short rows).
+template <int VEC>
+constexpr int bp_bufs() {
+    return VEC <= 2 ? 8 : 3;
+}
 
 // The back projector's plan for one angle of one 8x4-pixel tile; lanes = the
 // tile's 32 rays (lane = 8 * row + pixel; has: the lane's pixel is a ray of
@@ -366,7 +379,7 @@ __global__ void __launch_bounds__(256) k_fp_taps(OpArgs A, float4 *taps) {
 
 template <int VEC, int NSC>
 constexpr size_t bp_smem_bytes() {
-    return sizeof(float) * kBpBuf * kBpFoot * (NSC * 32 * VEC) + sizeof(float4) * kBpAngles * 32 +
+    return sizeof(float) * bp_bufs<VEC>() * kBpFoot * (NSC * 32 * VEC) + sizeof(float4) * kBpAngles * 32 +
            sizeof(int) * 2 * kBpAngles + sizeof(double) * (4 * NSC);
 }
 
@@ -429,7 +442,7 @@ template <int W, int VEC, int NSC>
 __global__ void __launch_bounds__(128 * NSC, NSC == 1 ? 4 : 1)
     bp_kernel(OpArgs A, const float *__restrict__ s, float *__restrict__ g,
               const __grid_constant__ CUtensorMap tms, int use_tma) {
-    constexpr int NCW = 4 * NSC, AC = kBpAngles, FW = kBpFoot, NB = kBpBuf;
+    constexpr int NCW = 4 * NSC, AC = kBpAngles, FW = kBpFoot, NB = bp_bufs<VEC>();
     constexpr int SPAN = NSC * 32 * VEC;  // slices per block
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[NB];
@@ -515,45 +528,22 @@ __global__ void __launch_bounds__(128 * NSC, NSC == 1 ? 4 : 1)
             if (ok && yok) {
                 const float *F = foot + (size_t)buf * FW * SPAN + yw;
                 // the ring (slots 0, 1, 2); a warp's first used ray loads all three
-                if constexpr (VEC >= 4) {
-                    // branch-free: each slot's load is predicated on its bit of
-                    // the plan's code; skipped rays have zero weights (and the
-                    // ring holds finite staged values), so their FMAs add nothing
-                    const unsigned Fa = smem_u32(F + lane_piece<VEC>(lane, 0));
+                // branch-free: each slot's load is predicated on its bit of
+                // the plan's code; skipped rays have zero weights (and the
+                // ring holds finite staged values), so their FMAs add nothing
+                const unsigned Fa = smem_u32(F + lane_piece<VEC>(lane, 0));
 #pragma unroll
-                    for (int r = 0; r < 8; r++) {
-                        const float4 e = sw[ai * 32 + rg * 8 + r];
-                        const unsigned code = (unsigned)__float_as_int(e.x), mask = code & 7u;
-                        const unsigned a = Fa + (code >> 8) * (SPAN * 4u);
-                        const unsigned step = mask == 7u ? SPAN * 4u : 0u;
-                        lds_lane_if<VEC>(mask & 1u, a, R0);
-                        lds_lane_if<VEC>(mask & 2u, a + step, R1);
-                        lds_lane_if<VEC>(mask & 4u, a + 2 * step, R2);
-                        fma_row<VEC>(acc[r], e.y, R0);
-                        fma_row<VEC>(acc[r], e.z, R1);
-                        fma_row<VEC>(acc[r], e.w, R2);
-                    }
-                } else {
-#pragma unroll
-                    for (int r = 0; r < 8; r++) {
-                        const float4 e = sw[ai * 32 + rg * 8 + r];
-                        const int code = __float_as_int(e.x), mask = code & 7;
-                        const float *row = F + (code >> 8) * SPAN;
-                        if (mask == 7) {
-                            lds_lane<VEC>(row, lane, R0);
-                            lds_lane<VEC>(row + SPAN, lane, R1);
-                            lds_lane<VEC>(row + 2 * SPAN, lane, R2);
-                        } else if (mask == 1) {
-                            lds_lane<VEC>(row, lane, R0);
-                        } else if (mask == 2) {
-                            lds_lane<VEC>(row, lane, R1);
-                        } else if (mask == 4) {
-                            lds_lane<VEC>(row, lane, R2);
-                        }
-                        fma_row<VEC>(acc[r], e.y, R0);
-                        fma_row<VEC>(acc[r], e.z, R1);
-                        fma_row<VEC>(acc[r], e.w, R2);
-                    }
+                for (int r = 0; r < 8; r++) {
+                    const float4 e = sw[ai * 32 + rg * 8 + r];
+                    const unsigned code = (unsigned)__float_as_int(e.x), mask = code & 7u;
+                    const unsigned a = Fa + (code >> 8) * (SPAN * 4u);
+                    const unsigned step = mask == 7u ? SPAN * 4u : 0u;
+                    lds_lane_if<VEC>(mask & 1u, a, R0);
+                    lds_lane_if<VEC>(mask & 2u, a + step, R1);
+                    lds_lane_if<VEC>(mask & 4u, a + 2 * step, R2);
+                    fma_row<VEC>(acc[r], e.y, R0);
+                    fma_row<VEC>(acc[r], e.z, R1);
+                    fma_row<VEC>(acc[r], e.w, R2);
                 }
             }
             __syncwarp();  // this warp's reads of the buffer are done
@@ -1176,7 +1166,9 @@ static __global__ void __launch_bounds__(64) k_lin_index(OpArgs A, int *off, int
 // Linear weighting, gather: one warp per (angle, bin, slice chunk); bin b
 // takes w0 of the rays whose first bin is b, then w1 of those whose first bin
 // is b - 1, each in ascending ray order, as the reference's per-ray products
-// added in float (arecproject.cpp:75-95).
+// added in float (arecproject.cpp:75-95).  The lanes fetch 32 rays' numbers and
+// weights at a time, and U rows are on their way together (bound by the latency
+// of the rows' reads from L2 and L1, one ray after the other before).
 template <int VEC>
 __global__ void __launch_bounds__(256) fp_lin_gather(OpArgs A, const float *__restrict__ x,
                                                      float *__restrict__ q) {
@@ -1193,6 +1185,8 @@ __global__ void __launch_bounds__(256) fp_lin_gather(OpArgs A, const float *__re
     const int *o = A.lin_off + (size_t)a * (A.nx + 2);
     const int *l = A.lin_list + (size_t)a * A.nrays;
     const AngleParams ap = A.ang[a];
+    constexpr int U = VEC >= 8 ? 4 : 8;
+    const float *xy = x + (yok ? y0 : 0);
     float acc[VEC];
 #pragma unroll
     for (int v = 0; v < VEC; v++) acc[v] = 0.f;
@@ -1200,15 +1194,29 @@ __global__ void __launch_bounds__(256) fp_lin_gather(OpArgs A, const float *__re
     for (int t = 0; t < 2; t++) {
         const int j = b + 1 - t;  // t = 0: first bin b (w0); t = 1: first bin b - 1 (w1)
         const int e = o[j + 1];
-        for (int i = o[j]; i < e; i++) {
-            const int k = l[i];
-            const Taps tp = ray_taps<ARECGB_LIN>(A.ray[k], ap, A.r_hi, A.r_lo);
-            const float w = t == 0 ? tp.w0 : tp.w1;
-            if (yok) {
-                float v[VEC];
-                ldv<VEC>(x + (size_t)k * A.ys + y0, v);
+        for (int i0 = o[j]; i0 < e; i0 += 32) {
+            const int m = min(32, e - i0);
+            int k = 0;
+            float w = 0.f;
+            if (lane < m) {
+                k = l[i0 + lane];
+                const Taps tp = ray_taps<ARECGB_LIN>(A.ray[k], ap, A.r_hi, A.r_lo);
+                w = t == 0 ? tp.w0 : tp.w1;
+            }
+            for (int i = 0; i < m; i += U) {
+                float v[U][VEC];
 #pragma unroll
-                for (int u = 0; u < VEC; u++) acc[u] = __fadd_rn(acc[u], __fmul_rn(w, v[u]));
+                for (int n = 0; n < U; n++) {
+                    const int kn = __shfl_sync(0xffffffffu, k, (i + n) & 31);
+                    ldv<VEC>(xy + (size_t)kn * A.ys, v[n]);  // beyond m: ray 0, not used below
+                }
+#pragma unroll
+                for (int n = 0; n < U; n++) {
+                    const float wn = __shfl_sync(0xffffffffu, w, (i + n) & 31);
+                    if (i + n < m)
+#pragma unroll
+                        for (int u = 0; u < VEC; u++) acc[u] = __fadd_rn(acc[u], __fmul_rn(wn, v[n][u]));
+                }
             }
         }
     }
