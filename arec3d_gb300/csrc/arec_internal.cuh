@@ -82,7 +82,7 @@ struct Plan {
     size_t table_bytes = 0;
     // tensor-core projectors (arec_project_mma.cu): groups, strips and segments
     // of the forward projection, tiles of the back projection, FP16 operands
-    int mma = 0;
+    int mma = 0;                  // 0: not used, 1: not in CGLS, 2: everywhere
     int4 *d_mgroups = nullptr;
     int2 *d_mstrips = nullptr, *d_msegs = nullptr;
     int *d_mshear = nullptr, *d_mslots = nullptr, *d_mpix = nullptr;
@@ -164,11 +164,11 @@ void plan_destroy(Plan *p);
 size_t vol_floats(const Plan *p);
 size_t sin_floats(const Plan *p);
 
-// Operators (arec_project.cu)
+// Operators (arec_project.cu); fp32: on the FP32 kernels in any case
 int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2,
-                    const int *d_skip, cudaStream_t st);
+                    const int *d_skip, cudaStream_t st, bool fp32 = false);
 int back_project(const Plan *p, const float *d_s, float *d_g, double *d_norm2,
-                 const int *d_skip, cudaStream_t st);
+                 const int *d_skip, cudaStream_t st, bool fp32 = false);
 int fp_grid_blocks(const Plan *p);
 int plan_timing(const Plan *p, int mode, double *fp_ms, long long *fp_calls, double *bp_ms,
                 long long *bp_calls);

@@ -114,7 +114,8 @@ __global__ void __launch_bounds__(256) k_zero_unless(float4 *q, size_t n4, const
 }
 
 int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2,
-                    const int *d_skip, cudaStream_t st) {
+                    const int *d_skip, cudaStream_t st, bool fp32) {
+    const bool mma = p->mma && !fp32;
     const OpArgs A = make_args(p, d_skip);
     const size_t nq = sin_floats(p);
     int rc = timing_mark(p, true, false, st);
@@ -127,7 +128,7 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
         // zero q, then each (orientation, line band) launch adds its part
         k_zero_unless<<<(unsigned)std::min<size_t>(152 * 8, (nq / 4 + 255) / 256), 256, 0, st>>>(
             reinterpret_cast<float4 *>(d_q), nq / 4, d_skip);
-        if (p->mma) {
+        if (mma) {
             rc = forward_project_mma(p, d_x, d_q, d_skip, st);
             if (rc) return rc;
         }
@@ -139,7 +140,7 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
         CUtensorMap tmx, tmxT;
         memset(&tmx, 0, sizeof(tmx));
         memset(&tmxT, 0, sizeof(tmxT));
-        if (A.taps && !p->mma) {
+        if (A.taps && !mma) {
             const int span = 32 * fp_vec(p);
             if (p->ngroups_o[1]) {
                 const int ys4 = p->ys / 4;
@@ -155,7 +156,7 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
                 return ARECGB_ERR_ARG;
             }
         }
-        for (int o = 0; o < 2 && !rc && !p->mma; o++) {
+        for (int o = 0; o < 2 && !rc && !mma; o++) {
             const int ngo = p->ngroups_o[o];
             if (!ngo) continue;
             const int g0 = o ? p->ngroups_o[0] : 0;
@@ -183,8 +184,8 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
 }
 
 int back_project(const Plan *p, const float *d_s, float *d_g, double *d_norm2,
-                 const int *d_skip, cudaStream_t st) {
-    if (p->mma) {
+                 const int *d_skip, cudaStream_t st, bool fp32) {
+    if (p->mma && !fp32) {
         int rc = timing_mark(p, false, false, st);
         if (!rc) rc = back_project_mma(p, d_s, d_g, d_skip, st);
         if (!rc && d_norm2) {
@@ -266,19 +267,21 @@ int plan_build_tables(Plan *p) {
     const char *env = getenv("ARECGB_PLAN_TABLES");
     if (env && env[0] == '0') return 0;
     const size_t b_recs = sizeof(float4) * (size_t)p->ngroups * p->nrays * 4;
-    // the tensor-core projectors read packed taps; the others taps and x's
-    // column-major copy
-    const size_t b_taps = b_recs + (p->mma ? 0 : sizeof(float) * (size_t)p->nrays * p->ys);
-    const size_t b_bpw = p->mma ? 0 : sizeof(float4) * (size_t)p->ntiles * p->na * 32;
-    const size_t b_bpf = p->mma ? 0 : sizeof(int2) * (size_t)p->ntiles * p->na;
+    // Plans all on the tensor cores read packed taps; the FP32 kernels taps and x's
+    // column-major copy (plans that have them for CGLS only: these, and the tensor-core
+    // kernels compute their taps, which costs them 3 to 20 %)
+    const bool mma = p->mma == 2;
+    const size_t b_taps = b_recs + (mma ? 0 : sizeof(float) * (size_t)p->nrays * p->ys);
+    const size_t b_bpw = mma ? 0 : sizeof(float4) * (size_t)p->ntiles * p->na * 32;
+    const size_t b_bpf = mma ? 0 : sizeof(int2) * (size_t)p->ntiles * p->na;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
     const size_t work = p->mma ? mma_work_bytes(p->nx, p->na, p->ys) : 0;  // in use already
     if ((double)(work + b_taps + b_bpw + b_bpf) > 0.4 * (double)(work + free_b)) return 0;
-    cudaError_t e = p->mma ? cudaMalloc(&p->d_ptaps, b_recs) : cudaMalloc(&p->d_taps, b_recs);
-    if (e == cudaSuccess && !p->mma) e = cudaMalloc(&p->d_xT, sizeof(float) * (size_t)p->nrays * p->ys);
-    if (e == cudaSuccess && !p->mma) e = cudaMalloc(&p->d_bpw, b_bpw);
-    if (e == cudaSuccess && !p->mma) e = cudaMalloc(&p->d_bpf, b_bpf);
+    cudaError_t e = mma ? cudaMalloc(&p->d_ptaps, b_recs) : cudaMalloc(&p->d_taps, b_recs);
+    if (e == cudaSuccess && !mma) e = cudaMalloc(&p->d_xT, sizeof(float) * (size_t)p->nrays * p->ys);
+    if (e == cudaSuccess && !mma) e = cudaMalloc(&p->d_bpw, b_bpw);
+    if (e == cudaSuccess && !mma) e = cudaMalloc(&p->d_bpf, b_bpf);
     if (e != cudaSuccess) {
         cudaGetLastError();  // an allocation failure is not sticky; run without tables
         cudaFree(p->d_taps);
@@ -295,7 +298,7 @@ int plan_build_tables(Plan *p) {
     }
     OpArgs A = make_args(p, nullptr);
     int rc = 0;
-    if (p->mma) {
+    if (mma) {
         rc = mma_build_taps(p, A);
         count_launches(1);
     } else {
@@ -323,7 +326,7 @@ int plan_build_tables(Plan *p) {
 // tensor-core projectors have one shape: they keep the plan's defaults.
 int plan_autotune(Plan *p, float *d_x, float *d_q, cudaStream_t st) {
     if (p->weighting == ARECGB_LIN) return 0;  // the linear pair has no shapes to choose
-    if (p->mma) {
+    if (p->mma == 2) {
         p->fp_vec = p->bp_vec = p->vec;
         p->bp_nsc = 1;
         p->tuned = 1;
@@ -360,7 +363,7 @@ int plan_autotune(Plan *p, float *d_x, float *d_q, cudaStream_t st) {
             if (band > 2 * p->nx && band != 32) continue;
             p->fp_band = band;
             float ms;
-            if ((rc = best_of([&] { return forward_project(p, d_x, d_q, nullptr, nullptr, st); },
+            if ((rc = best_of([&] { return forward_project(p, d_x, d_q, nullptr, nullptr, st, true); },
                               &ms)))
                 break;
             if (ms < best) {
@@ -385,7 +388,7 @@ int plan_autotune(Plan *p, float *d_x, float *d_q, cudaStream_t st) {
         p->bp_vec = v;
         p->bp_nsc = nsc;
         float ms;
-        if ((rc = best_of([&] { return back_project(p, d_q, d_x, nullptr, nullptr, st); }, &ms)))
+        if ((rc = best_of([&] { return back_project(p, d_q, d_x, nullptr, nullptr, st, true); }, &ms)))
             break;
         if (ms < best) {
             best = ms;

@@ -982,22 +982,30 @@ int upload(T **d, const std::vector<T> &h) {
 // x 64, 28.5, 28.5, 28.3 and 28.8 ms for CGLS at 401^2 x 300 x 75 (Kaiser-Bessel).
 static const int kMinBlocks = 10;
 
-// From 32 bins and 48 slices on.  Bins: 32 are two tiles across; there the forward
-// projection takes 0.049 against 0.077 ms and the back projection 0.045 against
-// 0.041 (36 angles, 64 slices); at 256^2 x 180 x 64 0.51 against 1.03 and 0.26
-// against 0.58 (the FP32 kernels with tables).  Slices: the blocks work on 128 at a
-// time and would pay from 8 on (0.49 against 0.94 ms at 256^2 x 180 x 8).  But a long
-// CGLS solve amplifies rounding (its residual goes its own way after about six
-// steps), and on slabs of a few slices, where solves are compared step by step with
-// the reference, the FP32 kernels sum in the reference's order; these do not, and
+// 2 (every projection of the plan) from 32 bins, 48 slices and 64 angles on, or
+// 4 million values in a volume: a back projection of a small volume is a chain over the
+// angles, 0.6 us each and 25 us of conversions and launches here against 1.1 us each
+// (65^2 x 90 x 64: 0.078 against 0.093 ms, forward 0.091 against 0.139; 256^2 x 180 x
+// 64: 0.26 against 0.58, forward 0.51 against 1.03; the FP32 kernels with tables).
+// 1 (all but CGLS) with fewer slices and 2.3 million rays and angles (twice that and
+// more for Kaiser-Bessel, whose taps cost more to compute): 160^2 x 90 x 16 0.094
+// against 0.107 ms, forward 0.20 against 0.36; 1024^2 x 600 x 8 10.7 against 17.8,
+// forward 11.5 against 36.6; at 96^2 x 24 x 8 it would be 0.043 against 0.029.  A long
+// CGLS solve amplifies rounding (its residual goes its own way after about six steps);
+// on slabs of a few slices, where solves are compared step by step with the reference,
+// it stays on the FP32 kernels, which sum in the reference's order: these do not, and
 // end closer to FP64 than to it.  4096 angles fill the back projector's table.
-bool mma_takes(int weighting, int nx, int ys, int na) {
-    return weighting != ARECGB_LIN && nx >= 32 && ys >= 48 && na <= BpMma::MAX_NA;
+int mma_takes(int weighting, int nx, int ys, int na) {
+    if (weighting == ARECGB_LIN || nx < 32 || na > BpMma::MAX_NA) return 0;
+    const double px = (double)nx * nx;
+    if (ys >= 48) return na >= 64 || px * ys >= 4e6 ? 2 : 0;
+    return px * na >= (weighting == ARECGB_KB ? 6e6 : 2.3e6) ? 1 : 0;
 }
 
 int mma_plan_create(Plan *p, const std::vector<int4> &g4, const std::vector<AngleParams> &ang,
                     const std::vector<RowInfo> &rows, const std::vector<ColInfo> &cols, bool spare) {
-    if (!mma_takes(p->weighting, p->nx, p->ys, p->na)) return 0;
+    const int use = mma_takes(p->weighting, p->nx, p->ys, p->na);
+    if (!use) return 0;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
     if (spare && (double)mma_work_bytes(p->nx, p->na, p->ys) > 0.4 * (double)free_b) return 0;
@@ -1079,7 +1087,7 @@ int mma_plan_create(Plan *p, const std::vector<int4> &g4, const std::vector<Angl
     }
     ARECGB_CUDA(cudaMemsetAsync(p->d_half[0], 0, bytes[0], p->stream));
     ARECGB_CUDA(cudaStreamSynchronize(p->stream));
-    p->mma = 1;
+    p->mma = use;
     return 0;
 }
 
@@ -1286,7 +1294,7 @@ int back_project_mma(const Plan *p, const float *d_s, float *d_g, const int *d_s
 
 MmaHold::MmaHold(Plan *const *plans, int n, cudaStream_t s) : st(s) {
     for (int i = 0; i < n; i++)
-        if (plans[i]->mma) held.push_back(plans[i]);
+        if (plans[i]->mma == 2) held.push_back(plans[i]);
     std::sort(held.begin(), held.end());  // one order for all holders
     for (Plan *p : held)
         for (int d = 0; d < 2; d++) {

@@ -52,8 +52,8 @@ struct MmaPlan {
     int ngroups, max_segs, max_strips, lblocks;
 };
 
-// Plans whose projections run on the tensor cores.
-bool mma_takes(int weighting, int nx, int ys, int na);
+// Which of a plan's projections run on the tensor cores (Plan::mma).
+int mma_takes(int weighting, int nx, int ys, int na);
 // spare: leave the plan to the FP32 kernels (p->mma = 0) when the operands would
 // take more than 40 % of the free memory.  It is left to them in any case when
 // they cannot be allocated.

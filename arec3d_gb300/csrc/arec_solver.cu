@@ -480,9 +480,10 @@ static int cgls_iteration(Plan *p, SolveState *S, double *hist, float *x, float 
     k_cgls_save<<<gv, 256, 0, st>>>(S, x, xs, nv / 4);
     k_cgls_save_done<<<1, 1, 0, st>>>(S);
     k_cgls_p<<<gv, 256, 0, st>>>(S, g, pd, nv / 4);
-    int rc = forward_project(p, pd, q, w || p->mma ? nullptr : &S->qnorm2, &S->done, st);
+    const bool mma = p->mma == 2;
+    int rc = forward_project(p, pd, q, w || mma ? nullptr : &S->qnorm2, &S->done, st, !mma);
     if (rc) return rc;
-    if (p->mma) {
+    if (mma) {
         const int nb = std::min(kRedBlocks, gs);
         k_cgls_dots<<<nb, 256, 0, st>>>(S, (const float4 *)q, (const float4 *)s, (const float4 *)w,
                                         ns / 4, p->d_partials);
@@ -494,9 +495,9 @@ static int cgls_iteration(Plan *p, SolveState *S, double *hist, float *x, float 
         if (rc) return rc;
         count_launches(2);
     }
-    if (!p->mma) k_cgls_alpha<<<1, 1, 0, st>>>(S);
+    if (!mma) k_cgls_alpha<<<1, 1, 0, st>>>(S);
     k_cgls_xs<<<gs, 256, 0, st>>>(S, x, pd, nv / 4, s, q, ns / 4, w);
-    rc = back_project(p, s, g, &S->gnorm2, &S->done, st);
+    rc = back_project(p, s, g, &S->gnorm2, &S->done, st, !mma);
     if (rc) return rc;
     k_cgls_gamma<<<1, 1, 0, st>>>(S, hist);
     count_launches(6);
@@ -607,7 +608,7 @@ int cgls_batch(Plan *const *plans, const float *const *d_b, float *const *d_x, c
         float *s_ = p->d_sin[0], *q = p->d_sin[1], *g = p->d_vol[0];
         const float *wi = d_w ? d_w[i] : nullptr;
         if (warm && warm[i]) {
-            rc = forward_project(p, d_x[i], q, nullptr, nullptr, cs);
+            rc = forward_project(p, d_x[i], q, nullptr, nullptr, cs, p->mma != 2);
             if (rc) break;
             if (wi)
                 k_sub_w<<<grid_for(ns, 16), 256, 0, cs>>>(d_b[i], q, wi, s_, ns);
@@ -623,7 +624,7 @@ int cgls_batch(Plan *const *plans, const float *const *d_b, float *const *d_x, c
                 cudaMemcpyAsync(s_, d_b[i], sizeof(float) * ns, cudaMemcpyDeviceToDevice, cs);
             }
         }
-        rc = back_project(p, s_, g, &S[i].gnorm2, nullptr, cs);
+        rc = back_project(p, s_, g, &S[i].gnorm2, nullptr, cs, p->mma != 2);
         if (rc) break;
         k_cgls_init<<<1, 1, 0, cs>>>(S + i, maxit, tol, rnorm_ref ? rnorm_ref[i] : 0.0);
         count_launches(1);

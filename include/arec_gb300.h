@@ -64,8 +64,8 @@ int arecgb_version(void);
 /* Geometry plan for one cylinder: radius (pixels, as arecAllocateCylImage,
  * AREC3D/AREC3D/arecImage.cpp:29), ny slices, nangles float radians (copied).
  * Allocates device tables on the current device, and for square-pixel and
- * Kaiser-Bessel plans with nx >= 32 and ys >= 48 (the tensor-core projectors)
- * room for one volume (of all nx nx pixels) and one sinogram as FP16 pairs,
+ * Kaiser-Bessel plans of more than a few angles and slices (those whose projections
+ * run on the tensor cores; with fewer than 48 slices CGLS keeps to FP32 kernels) room for one volume (of all nx nx pixels) and one sinogram as FP16 pairs,
  * unless that takes more than 40 % of the free memory (the FP32 projectors then).
  * A call captured into a graph brings this room as memory of the graph. */
 int arecgb_plan_create(arecgb_plan **plan, int weighting, double radius, int ny, int nangles,
@@ -153,8 +153,7 @@ int arecgb_plan_timing(arecgb_plan *plan, int mode, double *fp_ms, long long *fp
  * which it overwrites, and keeps the fastest; reports the band and the chunks
  * (either pointer may be NULL; arecgb_plan_shapes reports all four).  Results
  * do not depend on the choice beyond float summation order across bands.
- * Plans on the tensor cores (square-pixel and Kaiser-Bessel, nx >= 32, ys >= 48) have
- * one shape: the call reports their defaults and leaves the buffers alone.  No
+ * Plans all of whose projections run on the tensor cores have one shape: the call reports their defaults and leaves the buffers alone.  No
  * counterpart in the reference. */
 int arecgb_plan_autotune(arecgb_plan *plan, float *d_x, float *d_q, int *fp_band, int *bp_nsc,
                          void *stream);
@@ -166,8 +165,8 @@ int arecgb_plan_set_shapes(arecgb_plan *plan, int fp_band, int fp_vec, int bp_ve
 
 /* Device bytes of the plan's projector tables (0: none).  A plan for the
  * square-pixel or Kaiser-Bessel weighting stores the taps of every (ray,
- * angle) and, without the tensor-core projectors, the back projector's
- * per-tile ring plans when they take at most 40 % of the free device memory and the environment variable
+ * angle) and, where FP32 projectors are used, the back projector's per-tile
+ * ring plans when they take at most 40 % of the free device memory and the environment variable
  * ARECGB_PLAN_TABLES is not "0" at creation; the projectors compute the same
  * values without them (identical results).  No counterpart in the reference. */
 long long arecgb_plan_table_bytes(const arecgb_plan *plan);

@@ -1,5 +1,5 @@
-"""The tensor-core projectors (square-pixel and Kaiser-Bessel plans from 32
-bins and 48 slices on) at the sizes where their blocks end: slice tiles of 128 and 256, 16 x
+"""The tensor-core projectors (square-pixel and Kaiser-Bessel plans of all but
+small sizes) at the sizes where their blocks end: slice tiles of 128 and 256, 16 x
 16-pixel tiles, angle groups and pairs, and with operands that the FP16 pairs
 cannot hold.  References: the oracle with every sum in double.
 
@@ -23,7 +23,7 @@ TOL = {SQ: 1e-6, KB: 1e-5}
 
 def make(gb, nx, ny, ang, w=SQ):
     plan = gb.Plan(w, 0.5 * (nx - 1), ny, np.asarray(ang, np.float32))
-    assert plan.nx == nx and plan.ys >= 48
+    assert plan.nx == nx
     return plan
 
 
@@ -41,13 +41,17 @@ def backproject(plan, s):
     return vol_from_dev(plan, gd)
 
 
-ODD = [1.475, 21.123, 2.123, -0.3, 7.9, 0.785398, 0.7853982, 2.3561945, 3.1415927]
+ODD = np.concatenate([[1.475, 21.123, 2.123, -0.3, 7.9, 0.785398, 0.7853982, 2.3561945, 3.1415927],
+                      uniform_angles(60)]).astype(np.float32)
+FEW = [1e-4, 0.78, 0.79, 1.5707]
 CASES = [
-    (SQ, 32, 41, [0.3]), (SQ, 32, 48, uniform_angles(2)), (SQ, 33, 49, ODD),
-    (SQ, 34, 120, uniform_angles(7)), (SQ, 48, 128, uniform_angles(8)),
-    (SQ, 49, 129, uniform_angles(9)), (KB, 33, 136, uniform_angles(17)),
-    (SQ, 65, 256, uniform_angles(33)), (SQ, 64, 257, uniform_angles(5, 2 * np.pi)),
-    (KB, 65, 56, ODD), (SQ, 257, 44, uniform_angles(181)), (SQ, 530, 48, [1e-4, 0.78, 0.79, 1.5707]),
+    (SQ, 32, 41, ODD), (SQ, 33, 49, ODD), (SQ, 32, 48, uniform_angles(65)),
+    (SQ, 34, 120, uniform_angles(71)), (SQ, 48, 128, uniform_angles(72)),
+    (SQ, 49, 129, uniform_angles(73)), (KB, 33, 136, uniform_angles(65)),
+    (SQ, 65, 256, uniform_angles(64)), (SQ, 64, 257, uniform_angles(69, 2 * np.pi)),
+    (KB, 65, 56, ODD), (SQ, 257, 44, uniform_angles(181)), (SQ, 530, 48, FEW), (SQ, 360, 41, [0.3]),
+    # few slices, taps computed by the kernels
+    (SQ, 220, 1, ODD), (KB, 347, 8, ODD), (SQ, 1100, 20, FEW[:2]), (SQ, 96, 40, uniform_angles(250)),
 ]
 
 
@@ -81,7 +85,7 @@ def test_constant_sinogram_keeps_its_sum(gb, oc):
 def test_wide_values_stay_where_they_are(gb, oc, value):
     """One large or non-finite ray (or bin) of one slice: everything it does not
     reach is as without it, what it reaches is finite where the oracle's is."""
-    nx, ny, ang = 65, 42, uniform_angles(30)
+    nx, ny, ang = 65, 42, uniform_angles(64)
     plan = make(gb, nx, ny, ang)
     rng = np.random.default_rng(5)
     x = rng.random((plan.nrays, ny), dtype=np.float32)
@@ -107,7 +111,7 @@ def test_streams_and_graphs_share_a_plan(gb):
     beside eager calls, give what they give alone."""
     import torch
 
-    nx, ny, ang = 96, 44, uniform_angles(50)
+    nx, ny, ang = 96, 44, uniform_angles(64)
     plan = make(gb, nx, ny, ang)
     rng = np.random.default_rng(9)
     n = 6
@@ -153,7 +157,7 @@ def test_cgls_is_no_further_from_fp64_than_the_reference(gb, oc):
     """Twelve steps at 48 slices: steps computed from <s, q> keep the directions
     conjugate whatever A and A^T lose to rounding."""
     w, nx, ny, its = SQ, 65, 48, 12
-    ang, rng = uniform_angles(48), np.random.default_rng(31)
+    ang, rng = uniform_angles(64), np.random.default_rng(31)
     plan = make(gb, nx, ny, ang)
     with oc.op_threads():
         b = oc.project(w, 0.5 * (nx - 1), rng.random((plan.nrays, ny), dtype=np.float32), ang)
