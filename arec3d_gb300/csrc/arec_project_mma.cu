@@ -687,7 +687,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
     const int tid = threadIdx.x, warp = umma::uniform(tid >> 5), lane = tid & 31;
     if ((A.skip && *A.skip) || *nonfinite) return;  // uniform
     const int2 tile = M.tiles[blockIdx.x];
-    const int yb = blockIdx.y * 128, na = A.na, ns = (na + 1) / 2;
+    const int yb = blockIdx.y * 128, na = A.na;
+    // this block's pairs of angles: all, or one of two halves
+    const int pairs = ((na + 1) / 2 + gridDim.z - 1) / gridDim.z, a_lo = 2 * pairs * blockIdx.z;
+    const int ns = min(pairs, (na + 1) / 2 - pairs * (int)blockIdx.z);
     const float r = A.r_hi + A.r_lo;
 
     if (tid < 256) {
@@ -733,16 +736,16 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
         if (warp == kLoadWarp && lane == 0) {
             bool ok = true;
             for (int it = 0; it < ns && ok; it++) {
-                const int s = it % C::STAGES, n = min(2, na - 2 * it);
+                const int s = it % C::STAGES, a = a_lo + 2 * it, n = min(2, na - a);
                 if (it >= C::STAGES)
                     ok = umma::mbar_wait(&empty[s], (uint32_t)(it / C::STAGES - 1) & 1u, kMmaWait);
                 if (!ok) break;
                 umma::mbar_arrive_expect_tx(&afull[s], (uint32_t)(2 * n * C::PART));
                 for (int i = 0; i < n; i++) {
-                    const int f = (int)(s_ang[2 * it + i].x >> 16) - 64;
+                    const int f = (int)(s_ang[a + i].x >> 16) - 64;
                     unsigned char *d = sm + (size_t)s * C::STAGE + 2 * i * C::PART;
-                    umma::tma_load_4d(d, &tms, 8 * f, yb / 8, 2 * it + i, 0, &afull[s]);
-                    umma::tma_load_4d(d + C::PART, &tms, 8 * f, yb / 8, 2 * it + i, 1, &afull[s]);
+                    umma::tma_load_4d(d, &tms, 8 * f, yb / 8, a + i, 0, &afull[s]);
+                    umma::tma_load_4d(d + C::PART, &tms, 8 * f, yb / 8, a + i, 1, &afull[s]);
                 }
             }
             if (!ok) atomicOr(A.err, 16);
@@ -751,9 +754,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
             const uint32_t idesc = (1u << 4) | (1u << 15) | (8u << 17) | ((128u >> 4) << 24);
             bool ok = true;
             for (int it = 0; it < ns && ok; it++) {
-                const int s = it % C::STAGES, b = it & 1, n = min(2, na - 2 * it);
+                const int s = it % C::STAGES, b = it & 1, a0 = a_lo + 2 * it, n = min(2, na - a0);
                 const uint32_t ph = (uint32_t)(it / C::STAGES) & 1u;
-                const uint32_t win[2] = {umma::uniform(s_ang[2 * it].x), umma::uniform(s_ang[2 * it + 1].x)};
+                const uint32_t win[2] = {umma::uniform(s_ang[a0].x), umma::uniform(s_ang[a0 + 1].x)};
                 ok = umma::mbar_wait_warp(&bfull[s], ph, kMmaWait) &&
                      umma::mbar_wait_warp(&afull[s], ph, kMmaWait) &&
                      (it < 2 ||
@@ -805,9 +808,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
         auto fetch = [&](int it, uint4 (&e)[2]) {
 #pragma unroll
             for (int i = 0; i < 2; i++) {
-                const int a = 2 * it + i;
+                const int a = a_lo + 2 * it + i;
                 e[i] = make_uint4(0u, 0u, 0u, 0u);  // no ray: zero weights
-                if (a >= na || k < 0) continue;
+                if (it >= ns || a >= na || k < 0) continue;
                 if (M.taps) {
                     const int slot = (int)s_ang[a].y;
                     e[i] = __ldg(M.taps + ((size_t)((slot & INT_MAX) >> 2) * A.nrays + (slot < 0 ? kc : k)) *
@@ -827,8 +830,8 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
             unsigned char *d = sm + (size_t)s * C::STAGE + C::A + q * C::SUBW + ((t >> 3) & 7) * 256 + (t & 7) * 16;
 #pragma unroll
             for (int i = 0; i < 2; i++) {
-                if (2 * it + i >= na) break;
-                const unsigned win = s_ang[2 * it + i].x;
+                if (a_lo + 2 * it + i >= na) break;
+                const unsigned win = s_ang[a_lo + 2 * it + i].x;
                 int p = (int)e[i].x + 63 - (int)((win >> 16) + (win >> (4 * q) & 15u));
                 if (k < 0) p = 0;
                 if ((unsigned)p > (unsigned)kSpread) {
@@ -892,14 +895,28 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
                 uint32_t va, vb;
                 unpair(acc[i], va, vb);
                 const int ka = s_k[half * 128 + 2 * i], kb = s_k[half * 128 + 2 * i + 1];
-                if (ka >= 0) g[(size_t)ka * A.ys + y] = __uint_as_float(va) * inv;
-                if (kb >= 0) g[(size_t)kb * A.ys + y] = __uint_as_float(vb) * inv;
+                float *pa = g + (size_t)ka * A.ys + y, *pb = g + (size_t)kb * A.ys + y;
+                const float fa = __uint_as_float(va) * inv, fb = __uint_as_float(vb) * inv;
+                if (gridDim.z > 1) {  // two halves into zeros: the order does not matter
+                    if (ka >= 0) atomicAdd(pa, fa);
+                    if (kb >= 0) atomicAdd(pb, fb);
+                } else {
+                    if (ka >= 0) *pa = fa;
+                    if (kb >= 0) *pb = fb;
+                }
             }
         }
     }
     umma::fence_before_sync();
     __syncthreads();
     if (warp == kLoadWarp) umma::tmem_dealloc(tmem, C::COLS);
+}
+
+// v = 0 unless the solve has finished.
+__global__ void __launch_bounds__(256) k_clear_unless(float4 *v, size_t n, const int *skip) {
+    if (skip && *skip) return;
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256)
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // Back projection of a sinogram that holds an infinity or a NaN; returns at once
@@ -1248,7 +1265,17 @@ int launch_bp_mma(const Work &w, const OpArgs &A, const CUtensorMap &ts, const f
                                     (int)BpMma::smem(BpMma::MAX_NA));
     });
     ARECGB_CUDA(attr);
-    bp_mma_kernel<W><<<dim3(w.p->m_tiles, (A.ys + 127) / 128), kMmaThreads, BpMma::smem(A.na), w.st>>>(
+    // Two blocks per tile, half of the angles each, where the SMs' last wave gains: one
+    // wave lasts as long as its angles (256^2 x 180 x 64, 208 tiles: two waves of 90
+    // pairs or three of 45).
+    const int n = w.p->m_tiles * ((A.ys + 127) / 128);
+    const bool halves = A.na >= 32 && 10 * ((2 * n + 151) / 152) < 18 * ((n + 151) / 152);
+    if (halves) {
+        k_clear_unless<<<152 * 4, 256, 0, w.st>>>((float4 *)g, vol_floats(w.p) / 4, A.skip);
+        count_launches(1);
+    }
+    bp_mma_kernel<W><<<dim3(w.p->m_tiles, (A.ys + 127) / 128, halves ? 2 : 1), kMmaThreads,
+                       BpMma::smem(A.na), w.st>>>(
         A, make_plan(w.p), ts, g, w.smax, w.wide);
     bp_any_kernel<W><<<152 * 4, 128, 0, w.st>>>(A, s, g, w.wide);
     count_launches(2);
