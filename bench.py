@@ -852,8 +852,8 @@ def main():
     traffic = profiled_traffic().get(dom)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": traffic,
-                "kernel": "fp_band_kernel (one forward projection)" if dom == "fp"
-                else "bp_kernel (one back projection)",
+                "kernel": "fp_mma_kernel (one forward projection)" if dom == "fp"
+                else "bp_mma_kernel (one back projection)",
                 "peak_source": peak_kind,
                 "algorithmic_bytes_per_projection": algo_bytes,
                 "fp32": {"achieved_tflops": flops / t_dom / 1e12,
