@@ -68,6 +68,7 @@ static int choose_vec(int ys) {
 
 int plan_create(Plan **out, int weighting, double radius, int ny, int nangles,
                 const float *angles_host, bool tables) {
+    scratch_trim();  // the alignment's scratch, before memory is measured below
     *out = nullptr;
     if (weighting < ARECGB_LIN || weighting > ARECGB_SQ) {
         set_error("plan_create: weighting must be 1 (LIN), 2 (KB) or 3 (SQ)");

@@ -161,6 +161,7 @@ constexpr int kFpBins = 8;             // detector bins per forward-projection b
 int plan_create(Plan **out, int weighting, double radius, int ny, int nangles,
                 const float *angles_host, bool tables = true);
 void plan_destroy(Plan *p);
+void scratch_trim();  // arec_ccorr.cu: gives unused alignment scratch back
 size_t vol_floats(const Plan *p);
 size_t sin_floats(const Plan *p);
 
