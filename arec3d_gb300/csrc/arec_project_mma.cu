@@ -1023,6 +1023,8 @@ int mma_plan_create(Plan *p, const std::vector<int4> &g4, const std::vector<Angl
                     const std::vector<RowInfo> &rows, const std::vector<ColInfo> &cols, bool spare) {
     const int use = mma_takes(p->weighting, p->nx, p->ys, p->na);
     if (!use) return 0;
+    for (const AngleParams &a : ang)
+        if (!std::isfinite(a.c) || !std::isfinite(a.s)) return 0;  // no strips to follow
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
     if (spare && (double)mma_work_bytes(p->nx, p->na, p->ys) > 0.4 * (double)free_b) return 0;

@@ -50,6 +50,7 @@ CASES = [
     (SQ, 49, 129, uniform_angles(73)), (KB, 33, 136, uniform_angles(65)),
     (SQ, 65, 256, uniform_angles(64)), (SQ, 64, 257, uniform_angles(69, 2 * np.pi)),
     (KB, 65, 56, ODD), (SQ, 257, 44, uniform_angles(181)), (SQ, 530, 48, FEW), (SQ, 360, 41, [0.3]),
+    (SQ, 32, 41, uniform_angles(4096)),  # the back projector's table of windows is full
     # few slices, taps computed by the kernels
     (SQ, 220, 1, ODD), (KB, 347, 8, ODD), (SQ, 1100, 20, FEW[:2]), (SQ, 96, 40, uniform_angles(250)),
 ]
