@@ -13,7 +13,7 @@ int launch_fp_lin(const OpArgs &A, int vec, const float *x, float *q, cudaStream
 }
 
 int launch_lin_index(const OpArgs &A, int *off, int *list, cudaStream_t st) {
-    k_lin_index<<<(A.na + 63) / 64, 64, 0, st>>>(A, off, list);
+    k_lin_index<<<A.na, kLinIndexThreads, 0, st>>>(A, off, list);
     return 0;
 }
 
