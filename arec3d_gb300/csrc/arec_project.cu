@@ -126,11 +126,13 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
         count_launches(1);
     } else {
         // zero q, then each (orientation, line band) launch adds its part
-        k_zero_unless<<<(unsigned)std::min<size_t>(152 * 8, (nq / 4 + 255) / 256), 256, 0, st>>>(
-            reinterpret_cast<float4 *>(d_q), nq / 4, d_skip);
         if (mma) {
             rc = forward_project_mma(p, d_x, d_q, d_skip, st);
             if (rc) return rc;
+        } else {
+            k_zero_unless<<<(unsigned)std::min<size_t>(152 * 8, (nq / 4 + 255) / 256), 256, 0, st>>>(
+                reinterpret_cast<float4 *>(d_q), nq / 4, d_skip);
+            count_launches(1);
         }
         const int ntile = (p->nx + kFpBins - 1) / kFpBins;
         rc = 0;
@@ -169,7 +171,6 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
                 count_launches(1);
             }
         }
-        count_launches(1);
     }
     ARECGB_CUDA(cudaGetLastError());
     if (rc) return ARECGB_ERR_ARG;

@@ -21,6 +21,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <numeric>
 #include <vector>
 
 #include "arec_project_mma.cuh"
@@ -51,6 +52,25 @@ constexpr int kSegBlocks = 64;  // line blocks of a segment at most
 
 // ---------------------------------------------------------------------------
 // FP16 pairs.
+
+// A pair keeps its 22 bits down to 2^-29 of the slice's largest magnitude (scaled:
+// 2^14 .. 2^15).  A slice more than 1/32 of whose nonzero values lie below kSmall
+// (2^-30 of the largest, or a little more) would lose bits that FP32 keeps: a fill
+// value or a hot pixel beside ordinary data.  Fewer do not matter: values spread
+// around zero reach below it in about 2^-28 of the cases, the rounding noise that an
+// FP32 transform leaves on a background of zeros (2^-25 of the largest) in 2 %.
+constexpr float kSmall = 1.f / 32768.f;
+constexpr int kScoreSmall = 31;
+constexpr int kScoreShared = 4096;  // slices whose scores a block adds up in shared memory
+
+// Per plan and direction, beside the operand: zeroed before the largest magnitudes are
+// taken; mma_stats_bytes.
+struct HalfStats {
+    unsigned *maxb;              // [ys] largest magnitude per slice
+    unsigned long long *score;   // [ys] kScoreSmall for a small value, -1 for any other
+    int *wide;                   // set when one is positive: the operand takes FP32 kernels
+    int ys;
+};
 
 // Largest magnitude per slice (as ordered integers; an infinity or NaN is >=
 // 0x7f800000) of rows [n][ys]; out zeroed by the caller.
@@ -92,15 +112,23 @@ __device__ __forceinline__ unsigned pack_half(float a, float b, float &ra, float
     return (unsigned)__half_as_ushort(ha) | ((unsigned)__half_as_ushort(hb) << 16);
 }
 
-// Eight slices: scaled, high and low halves.
-__device__ __forceinline__ void half_pair(const float4 *v, const uint4 *maxb, uint4 &hi, uint4 &lo) {
+// Eight slices: scaled, high and low halves.  score: a nonzero value below kSmall
+// adds kScoreSmall, any other nonzero one takes 1.
+__device__ __forceinline__ void half_pair(const float4 *v, const uint4 &ma, const uint4 &mb, uint4 &hi,
+                                          uint4 &lo, int (&score)[8]) {
     const float4 a = v[0], b = v[1];
-    const uint4 ma = maxb[0], mb = maxb[1];
-    float l[8], d0, d1;
-    hi.x = pack_half(a.x * pow2f(half_shift(ma.x)), a.y * pow2f(half_shift(ma.y)), l[0], l[1]);
-    hi.y = pack_half(a.z * pow2f(half_shift(ma.z)), a.w * pow2f(half_shift(ma.w)), l[2], l[3]);
-    hi.z = pack_half(b.x * pow2f(half_shift(mb.x)), b.y * pow2f(half_shift(mb.y)), l[4], l[5]);
-    hi.w = pack_half(b.z * pow2f(half_shift(mb.z)), b.w * pow2f(half_shift(mb.w)), l[6], l[7]);
+    const float raw[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    const unsigned m[8] = {ma.x, ma.y, ma.z, ma.w, mb.x, mb.y, mb.z, mb.w};
+    float f[8], l[8], d0, d1;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        f[i] = raw[i] * pow2f(half_shift(m[i]));
+        if (raw[i] != 0.f) score[i] += fabsf(f[i]) < kSmall ? kScoreSmall : -1;
+    }
+    hi.x = pack_half(f[0], f[1], l[0], l[1]);
+    hi.y = pack_half(f[2], f[3], l[2], l[3]);
+    hi.z = pack_half(f[4], f[5], l[4], l[5]);
+    hi.w = pack_half(f[6], f[7], l[6], l[7]);
 #pragma unroll
     for (int i = 0; i < 8; i++) l[i] *= kLowScale;
     lo.x = pack_half(l[0], l[1], d0, d1);
@@ -109,53 +137,100 @@ __device__ __forceinline__ void half_pair(const float4 *v, const uint4 *maxb, ui
     lo.w = pack_half(l[6], l[7], d0, d1);
 }
 
-// Rows [n][ys] as FP16 pairs [2][rows][ys], row r at place[r] (r itself when
-// null).  flag: set when a slice holds an infinity, a NaN or values from 2^40 on.
-__global__ void __launch_bounds__(256)
-    k_to_half(const float4 *__restrict__ v, size_t n, int ys8, const unsigned *__restrict__ maxb,
-              const int *__restrict__ place, size_t rows, uint4 *__restrict__ out, int *flag,
-              const int *skip) {
+// A conversion's end: the scores of the block's lanes lane mod step (slices 8 m ..,
+// m < 0: none) to the slices' sums.  cnt: shared memory (zeroed, a barrier later), a
+// counter per slice where kScoreShared of them are enough.
+__device__ __forceinline__ void start_scores(const HalfStats &S, int *cnt) {
+    if (S.ys <= kScoreShared)
+        for (int i = threadIdx.x; i < S.ys; i += 256) cnt[i] = 0;
+    __syncthreads();
+}
+__device__ __forceinline__ void add_scores(const HalfStats &S, int m, int step, int (&score)[8], int *cnt) {
+    const bool sm = S.ys <= kScoreShared;
+    for (int o = 16; o >= step; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < 8; i++) score[i] += __shfl_xor_sync(0xffffffffu, score[i], o);
+    if (m >= 0 && (int)(threadIdx.x & 31) < step)
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            if (sm) atomicAdd(&cnt[8 * m + i], score[i]);
+            else if (score[i]) atomicAdd(S.score + 8 * m + i, (unsigned long long)(long long)score[i]);
+        }
+    __syncthreads();
+    if (sm)
+        for (int i = threadIdx.x; i < S.ys; i += 256)
+            if (cnt[i]) atomicAdd(S.score + i, (unsigned long long)(long long)cnt[i]);
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < S.ys; i += 256)
+            if (S.maxb[i] >= kWideBits) atomicAdd(S.score + i, 1ull << 62);
+}
+
+// v = 0 unless the solve has finished; and the operand's flag (a block of the
+// conversion that waited for the others to set it would cost 3 us, the projectors'
+// blocks 1 us each if they added the scores up to it themselves).
+__global__ void __launch_bounds__(256) k_clear(float4 *v, size_t n, const int *skip, const HalfStats S) {
     if (skip && *skip) return;
     if (blockIdx.x == 0)
-        for (int i = threadIdx.x; i < 8 * ys8; i += 256)
-            if (maxb[i] >= kWideBits) *flag = 1;
-    const size_t total = n * ys8;
-    for (size_t t = (size_t)blockIdx.x * 256 + threadIdx.x; t < total; t += (size_t)gridDim.x * 256) {
-        const size_t r = t / ys8;
-        const int m = (int)(t - r * ys8);
+        for (int i = threadIdx.x; i < S.ys; i += 256)
+            if ((long long)S.score[i] > 0) *S.wide = 1;
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256)
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// Rows [n][ys] as FP16 pairs [2][rows][ys], row r at place[r].  The grid's threads are a
+// multiple of ys8: each keeps its slices.
+__global__ void __launch_bounds__(256)
+    k_to_half(const float4 *__restrict__ v, size_t n, int ys8, const HalfStats S,
+              const int *__restrict__ place, size_t rows, uint4 *__restrict__ out, const int *skip) {
+    extern __shared__ int sm_score[];
+    if (skip && *skip) return;
+    start_scores(S, sm_score);
+    const size_t total = n * ys8, t0 = (size_t)blockIdx.x * 256 + threadIdx.x;
+    const int m = (int)(t0 % ys8);
+    const uint4 ma = reinterpret_cast<const uint4 *>(S.maxb)[2 * m];
+    const uint4 mb = reinterpret_cast<const uint4 *>(S.maxb)[2 * m + 1];
+    int score[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (size_t t = t0; t < total; t += (size_t)gridDim.x * 256) {
         uint4 hi, lo;
-        half_pair(v + 2 * t, reinterpret_cast<const uint4 *>(maxb) + 2 * m, hi, lo);
-        const size_t o = (place ? (size_t)place[r] : r) * ys8 + m;
+        half_pair(v + 2 * t, ma, mb, hi, lo, score);
+        const size_t o = (size_t)place[t / ys8] * ys8 + m;
         out[o] = hi;
         out[rows * ys8 + o] = lo;
     }
+    add_scores(S, m, 32 % ys8 ? 32 : ys8, score, sm_score);
 }
 
 // The sinogram [na][nx][ys] as FP16 pairs [2][na][ys/8][nx][8] (the back
 // projector's windows start at any bin: eight slices of neighbouring bins lie in
 // one row).  A warp takes 8 bins x 4 slice groups: 128-byte pieces on both sides.
+// The grid's warps are a multiple of the groups of four: each keeps its own.
 __global__ void __launch_bounds__(256)
-    k_sino_to_half(const float4 *__restrict__ v, int na, int nx, int ys8,
-                   const unsigned *__restrict__ maxb, uint4 *__restrict__ out, int *flag,
-                   const int *skip) {
+    k_sino_to_half(const float4 *__restrict__ v, int na, int nx, int ys8, const HalfStats S,
+                   uint4 *__restrict__ out, const int *skip) {
+    extern __shared__ int sm_score[];
     if (skip && *skip) return;
-    if (blockIdx.x == 0)
-        for (int i = threadIdx.x; i < 8 * ys8; i += 256)
-            if (maxb[i] >= kWideBits) *flag = 1;
+    start_scores(S, sm_score);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nmb = (ys8 + 3) / 4, nbb = (nx + 7) / 8;
     const size_t total = (size_t)na * nbb * nmb, half = (size_t)na * ys8 * nx;
-    for (size_t t = (size_t)blockIdx.x * 8 + warp; t < total; t += (size_t)gridDim.x * 8) {
-        const int m = (int)(t % nmb) * 4 + (lane & 3);
-        const int b = (int)(t / nmb % nbb) * 8 + (lane >> 2);
-        const size_t a = t / nmb / nbb;
-        if (m >= ys8 || b >= nx) continue;
-        uint4 hi, lo;
-        half_pair(v + ((a * nx + b) * ys8 + m) * 2, reinterpret_cast<const uint4 *>(maxb) + 2 * m, hi, lo);
-        const size_t o = (a * ys8 + m) * nx + b;
-        out[o] = hi;
-        out[half + o] = lo;
+    const size_t t0 = (size_t)blockIdx.x * 8 + warp;
+    const int m = (int)(t0 % nmb) * 4 + (lane & 3);
+    int score[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (m < ys8) {
+        const uint4 ma = reinterpret_cast<const uint4 *>(S.maxb)[2 * m];
+        const uint4 mb = reinterpret_cast<const uint4 *>(S.maxb)[2 * m + 1];
+        for (size_t t = t0; t < total; t += (size_t)gridDim.x * 8) {
+            const int b = (int)(t / nmb % nbb) * 8 + (lane >> 2);
+            const size_t a = t / nmb / nbb;
+            if (b >= nx) continue;
+            uint4 hi, lo;
+            half_pair(v + ((a * nx + b) * ys8 + m) * 2, ma, mb, hi, lo, score);
+            const size_t o = (a * ys8 + m) * nx + b;
+            out[o] = hi;
+            out[half + o] = lo;
+        }
     }
+    add_scores(S, m < ys8 ? m : -1, 4, score, sm_score);
 }
 
 // ---------------------------------------------------------------------------
@@ -278,7 +353,7 @@ struct FpMma {
 template <int W, int MT>
 __global__ void __launch_bounds__(kMmaThreads, 1)
     fp_mma_kernel(OpArgs A, MmaPlan M, const __grid_constant__ CUtensorMap tmx, float *__restrict__ q,
-                  const unsigned *__restrict__ maxb, const int *__restrict__ nonfinite, int seg,
+                  const unsigned *__restrict__ maxb, const int *__restrict__ wide, int seg,
                   int color) {
     using C = FpMma<MT>;
     extern __shared__ unsigned char sm_raw[];
@@ -296,7 +371,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
     const int g = blockIdx.x % M.ngroups, strip = blockIdx.x / M.ngroups * 3 + color;
     const int4 G = M.groups[g];
     const int2 js = M.strips[g], sg = M.segs[g * M.max_segs + seg];
-    const int bad = *nonfinite, skip = A.skip ? *A.skip : 0;
+    const int bad = *wide, skip = A.skip ? *A.skip : 0;
     if (bad || skip || seg >= G.w || strip >= js.y) return;  // uniform
     const int j8 = 8 * (js.x + strip), orient = G.z, NA = G.y, N = kWin * NA;
     const int *shear = M.shear + (size_t)g * M.lblocks;
@@ -565,8 +640,8 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
 template <int W>
 __global__ void __launch_bounds__(128)
     fp_any_kernel(OpArgs A, const float *__restrict__ x, float *__restrict__ q,
-                  const int *__restrict__ nonfinite) {
-    if ((A.skip && *A.skip) || !*nonfinite) return;
+                  const int *__restrict__ wide) {
+    if ((A.skip && *A.skip) || !*wide) return;
     const float r = A.r_hi + A.r_lo;
     for (long long t = blockIdx.x; t < (long long)A.na * A.nx; t += gridDim.x) {
         const int a = (int)(t / A.nx), b = (int)(t % A.nx);
@@ -677,7 +752,7 @@ __device__ __forceinline__ void two_sum(unsigned long long *acc, uint32_t *va, u
 template <int W>
 __global__ void __launch_bounds__(kMmaThreads, 1)
     bp_mma_kernel(OpArgs A, MmaPlan M, const __grid_constant__ CUtensorMap tms, float *__restrict__ g,
-                  const unsigned *__restrict__ maxb, const int *__restrict__ nonfinite) {
+                  const unsigned *__restrict__ maxb, const int *__restrict__ wide) {
     using C = BpMma;
     extern __shared__ unsigned char sm_raw[];
     __shared__ __align__(8) uint64_t afull[C::STAGES], bfull[C::STAGES], empty[C::STAGES];
@@ -685,7 +760,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
     __shared__ uint32_t tmem_base;
     __shared__ int s_k[256];                // rays of the tile (-1: none), sub-block by sub-block
     const int tid = threadIdx.x, warp = umma::uniform(tid >> 5), lane = tid & 31;
-    if ((A.skip && *A.skip) || *nonfinite) return;  // uniform
+    if ((A.skip && *A.skip) || *wide) return;  // uniform
     const int2 tile = M.tiles[blockIdx.x];
     const int yb = blockIdx.y * 128, na = A.na;
     // this block's pairs of angles: all, or one of two halves
@@ -912,20 +987,13 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
     if (warp == kLoadWarp) umma::tmem_dealloc(tmem, C::COLS);
 }
 
-// v = 0 unless the solve has finished.
-__global__ void __launch_bounds__(256) k_clear_unless(float4 *v, size_t n, const int *skip) {
-    if (skip && *skip) return;
-    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256)
-        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-}
-
 // Back projection of a sinogram that holds an infinity or a NaN; returns at once
 // otherwise.
 template <int W>
 __global__ void __launch_bounds__(128)
     bp_any_kernel(OpArgs A, const float *__restrict__ s, float *__restrict__ g,
-                  const int *__restrict__ nonfinite) {
-    if ((A.skip && *A.skip) || !*nonfinite) return;
+                  const int *__restrict__ wide) {
+    if ((A.skip && *A.skip) || !*wide) return;
     for (int k = blockIdx.x; k < A.nrays; k += gridDim.x)
         for (int y = threadIdx.x; y < A.ys; y += blockDim.x) {
             float v = 0.f;
@@ -1097,7 +1165,7 @@ int mma_plan_create(Plan *p, const std::vector<int4> &g4, const std::vector<Angl
     const size_t bytes[2] = {sizeof(float) * (size_t)p->nx * p->nx * p->ys, sizeof(float) * sin_floats(p)};
     for (int d = 0; d < 2; d++) {
         if (cudaMalloc(&p->d_half[d], bytes[d]) != cudaSuccess ||
-            cudaMalloc(&p->d_smax[d], sizeof(unsigned) * (p->ys + 4)) != cudaSuccess) {
+            cudaMalloc(&p->d_smax[d], mma_stats_bytes(p->ys)) != cudaSuccess) {
             cudaGetLastError();  // not sticky: run without
             mma_plan_destroy(p);
             return 0;
@@ -1158,7 +1226,7 @@ namespace {
 struct Work {
     void *half = nullptr;
     unsigned *smax = nullptr;
-    int *wide = nullptr;  // the flag behind the maxima
+    HalfStats stats{};
     const Plan *p = nullptr;
     int dir = 0;
     cudaStream_t st = nullptr;
@@ -1175,7 +1243,7 @@ struct Work {
         if (own) {
             const size_t bytes = sizeof(float) * (dir ? sin_floats(p) : (size_t)p->nx * p->nx * p->ys);
             ARECGB_CUDA(cudaMallocAsync(&half, bytes, st));
-            ARECGB_CUDA(cudaMallocAsync((void **)&smax, sizeof(unsigned) * (p->ys + 4), st));
+            ARECGB_CUDA(cudaMallocAsync((void **)&smax, mma_stats_bytes(p->ys), st));
             if (dir == 0) ARECGB_CUDA(cudaMemsetAsync(half, 0, bytes, st));
         }
         if (eager) {
@@ -1186,7 +1254,7 @@ struct Work {
                 ARECGB_CUDA(e);
             }
         }
-        wide = (int *)(smax + p->ys);
+        stats = {smax, (unsigned long long *)(smax + p->ys), (int *)(smax + 3 * p->ys), p->ys};
         return 0;
     }
     int end() {
@@ -1203,16 +1271,22 @@ struct Work {
     }
 };
 
-// Largest magnitude per slice of rows [n][ys], the flag cleared.
+// Largest magnitude per slice of rows [n][ys], the scores cleared.
 int slice_max(const Work &w, const float *v, size_t n, const int *skip) {
     const int ys4 = w.p->ys / 4, nv = std::min(ys4, 256), rb = 256 / nv;
-    ARECGB_CUDA(cudaMemsetAsync(w.smax, 0, sizeof(unsigned) * (w.p->ys + 4), w.st));
+    ARECGB_CUDA(cudaMemsetAsync(w.smax, 0, mma_stats_bytes(w.p->ys), w.st));
     k_slice_max<<<(int)std::min<size_t>(152 * 8, (n + rb - 1) / rb), 256, 16 * nv, w.st>>>(
         (const float4 *)v, n, ys4, w.smax, skip);
     count_launches(1);
     ARECGB_CUDA(cudaGetLastError());
     return 0;
 }
+
+// About `blocks` of them, a multiple of `unit`.
+unsigned blocks_of(int unit, size_t blocks) {
+    return (unsigned)((blocks + unit - 1) / unit * unit);
+}
+size_t score_bytes(int ys) { return ys <= kScoreShared ? sizeof(int) * ys : 0; }
 
 template <int W, int MT>
 int launch_fp_mma(const Work &w, const OpArgs &A, const MmaPlan &M, const CUtensorMap &tx,
@@ -1228,8 +1302,8 @@ int launch_fp_mma(const Work &w, const OpArgs &A, const MmaPlan &M, const CUtens
     for (int seg = 0; seg < M.max_segs; seg++)
         for (int color = 0; color < 3; color++)
             fp_mma_kernel<W, MT><<<grid, kMmaThreads, FpMma<MT>::SMEM, w.st>>>(A, M, tx, q, w.smax,
-                                                                               w.wide, seg, color);
-    fp_any_kernel<W><<<152 * 4, 128, 0, w.st>>>(A, x, q, w.wide);
+                                                                               w.stats.wide, seg, color);
+    fp_any_kernel<W><<<152 * 4, 128, 0, w.st>>>(A, x, q, w.stats.wide);
     count_launches(3 * M.max_segs + 1);
     ARECGB_CUDA(cudaGetLastError());
     return 0;
@@ -1240,10 +1314,14 @@ int fp_steps(const Work &w, const OpArgs &A, const float *d_x, float *d_q) {
     const int ys8 = p->ys / 8;
     const size_t n = p->nrays, total = n * ys8;
     if (int rc = slice_max(w, d_x, n, A.skip)) return rc;
-    k_to_half<<<(unsigned)std::min<size_t>(152 * 16, (total + 255) / 256), 256, 0, w.st>>>(
-        (const float4 *)d_x, n, ys8, w.smax, p->d_mpix, (size_t)p->nx * p->nx, (uint4 *)w.half, w.wide,
-        A.skip);
-    count_launches(1);
+    const int unit = ys8 / std::gcd(ys8, 256);  // blocks whose threads are a multiple of ys8
+    k_to_half<<<blocks_of(unit, std::min<size_t>(152 * 4, (total + 255) / 256)), 256, score_bytes(p->ys),
+                w.st>>>((const float4 *)d_x, n, ys8, w.stats, p->d_mpix, (size_t)p->nx * p->nx,
+                        (uint4 *)w.half, A.skip);
+    const size_t nq = sin_floats(p) / 4;
+    k_clear<<<(unsigned)std::min<size_t>(152 * 8, (nq + 255) / 256), 256, 0, w.st>>>((float4 *)d_q, nq,
+                                                                                    A.skip, w.stats);
+    count_launches(2);
     CUtensorMap tx;
     if (!encode_half_map(&tx, w.half, p->ys, p->nx, p->nx, 8, 8)) {
         set_error("forward_project: tensor map encoding failed");
@@ -1272,14 +1350,13 @@ int launch_bp_mma(const Work &w, const OpArgs &A, const CUtensorMap &ts, const f
     // pairs or three of 45).
     const int n = w.p->m_tiles * ((A.ys + 127) / 128);
     const bool halves = A.na >= 32 && 10 * ((2 * n + 151) / 152) < 18 * ((n + 151) / 152);
-    if (halves) {
-        k_clear_unless<<<152 * 4, 256, 0, w.st>>>((float4 *)g, vol_floats(w.p) / 4, A.skip);
-        count_launches(1);
-    }
+    k_clear<<<halves ? 152 * 4 : 1, 256, 0, w.st>>>((float4 *)g, halves ? vol_floats(w.p) / 4 : 0, A.skip,
+                                                    w.stats);
+    count_launches(1);
     bp_mma_kernel<W><<<dim3(w.p->m_tiles, (A.ys + 127) / 128, halves ? 2 : 1), kMmaThreads,
                        BpMma::smem(A.na), w.st>>>(
-        A, make_plan(w.p), ts, g, w.smax, w.wide);
-    bp_any_kernel<W><<<152 * 4, 128, 0, w.st>>>(A, s, g, w.wide);
+        A, make_plan(w.p), ts, g, w.smax, w.stats.wide);
+    bp_any_kernel<W><<<152 * 4, 128, 0, w.st>>>(A, s, g, w.stats.wide);
     count_launches(2);
     ARECGB_CUDA(cudaGetLastError());
     return 0;
@@ -1289,9 +1366,10 @@ int bp_steps(const Work &w, const OpArgs &A, const float *d_s, float *d_g) {
     const Plan *p = w.p;
     const int ys8 = p->ys / 8;
     if (int rc = slice_max(w, d_s, (size_t)p->na * p->nx, A.skip)) return rc;
-    const size_t warps = (size_t)p->na * ((p->nx + 7) / 8) * ((ys8 + 3) / 4);
-    k_sino_to_half<<<(unsigned)std::min<size_t>(152 * 8, (warps + 7) / 8), 256, 0, w.st>>>(
-        (const float4 *)d_s, p->na, p->nx, ys8, w.smax, (uint4 *)w.half, w.wide, A.skip);
+    const int nmb = (ys8 + 3) / 4, unit = nmb / std::gcd(nmb, 8);
+    const size_t warps = (size_t)p->na * ((p->nx + 7) / 8) * nmb;
+    k_sino_to_half<<<blocks_of(unit, std::min<size_t>(152 * 4, (warps + 7) / 8)), 256, score_bytes(p->ys),
+                     w.st>>>((const float4 *)d_s, p->na, p->nx, ys8, w.stats, (uint4 *)w.half, A.skip);
     count_launches(1);
     CUtensorMap ts;
     if (!encode_foot_map(&ts, w.half, p->nx, ys8, p->na, kFoot)) {
@@ -1304,7 +1382,7 @@ int bp_steps(const Work &w, const OpArgs &A, const float *d_s, float *d_g) {
 
 }  // namespace
 
-// q (zeroed by the caller) = A x.
+// q = A x.
 int forward_project_mma(const Plan *p, const float *d_x, float *d_q, const int *d_skip,
                         cudaStream_t st) {
     Work w;

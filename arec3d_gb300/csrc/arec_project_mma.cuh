@@ -23,13 +23,12 @@ namespace arecgb {
 // the slice's value times 2^half_shift(the slice's largest magnitude).  The low
 // halves' own scale (taken back by the MMA that adds hi*hi, D = A B + D 2^-11)
 // keeps them normal: 22 bits down to 2^-29 of the slice's largest magnitude, an
-// error of 2^-51 of it below.
+// error of 2^-51 of it below.  An operand with a slice that spans more than that
+// (see kSmall in arec_project_mma.cu) takes FP32 kernels.
 constexpr float kWeightScale = 4096.f;
 constexpr int kLowBits = 11;
 constexpr float kLowScale = 2048.f;
-// Slices with values from 2^40 on (fill values, infinities, NaN) have neighbours
-// that these pairs cannot hold: such an operand takes the kernels that work ray
-// by ray in FP32.
+// So does one with values from 2^40 on, an infinity or a NaN.
 constexpr unsigned kWideBits = (127u + 40u) << 23;
 
 __device__ __forceinline__ int half_shift(unsigned max_bits) {
@@ -82,9 +81,11 @@ class MmaHold {
     cudaStream_t st;
 };
 
-// Bytes of the FP16 operands and maxima of a plan.
+// Bytes of an operand's maxima and scores, and of both FP16 operands of a plan
+// with theirs.
+inline size_t mma_stats_bytes(size_t ys) { return sizeof(unsigned) * (3 * ys + 4); }
 inline size_t mma_work_bytes(size_t nx, size_t na, size_t ys) {
-    return sizeof(float) * (nx * nx * ys + na * nx * ys + 2 * (ys + 4));
+    return sizeof(float) * (nx * nx * ys + na * nx * ys) + 2 * mma_stats_bytes(ys);
 }
 
 }  // namespace arecgb
