@@ -30,6 +30,14 @@ struct OpArgs {
     const int *kinv;     // column-major ray index -> ray index
 };
 
+// What a projection does about an operand that FP16 pairs cannot hold (operand_wide in
+// arec_project_impl.cuh): [ys] scores, the flag, float4 of the output to clear otherwise.
+struct WideArgs {
+    const long long *score;
+    int *wide;
+    size_t n_clear;
+};
+
 inline OpArgs make_args(const Plan *p, const int *skip) {
     OpArgs A;
     A.ray = p->d_ray;

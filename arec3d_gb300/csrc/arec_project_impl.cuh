@@ -32,6 +32,7 @@
 #include <cuda.h>  // CUtensorMap (the forward projector's row tiles)
 
 #include <climits>
+#include <cstring>
 
 #include "arec_project_args.cuh"
 #include "arec_umma.cuh"
@@ -438,10 +439,13 @@ __device__ __forceinline__ void bp_stage(const OpArgs &A, const float *__restric
 // warp, so 4 blocks fit per SM.  Each warp walks its 8 rays through a
 // three-row register ring (one shared-memory row read per ray instead of
 // three).  Bins off the detector add nothing, as the reference skips them.
-template <int W, int VEC, int NSC>
-__global__ void __launch_bounds__(128 * NSC, NSC == 1 ? 4 : 1)
-    bp_kernel(OpArgs A, const float *__restrict__ s, float *__restrict__ g,
-              const __grid_constant__ CUtensorMap tms, int use_tma) {
+//
+// Tile bx, slice block by; true unless a wait gave up.  AGAIN: the block has done
+// another tile before (after a barrier).
+template <int W, int VEC, int NSC, bool AGAIN>
+__device__ __forceinline__ bool bp_block(const OpArgs &A, const float *__restrict__ s,
+                                         float *__restrict__ g, const CUtensorMap *tms, int use_tma,
+                                         int bx, int by, bool again) {
     constexpr int NCW = 4 * NSC, AC = kBpAngles, FW = kBpFoot, NB = bp_bufs<VEC>();
     constexpr int SPAN = NSC * 32 * VEC;  // slices per block
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -452,12 +456,11 @@ __global__ void __launch_bounds__(128 * NSC, NSC == 1 ? 4 : 1)
     int *fb = reinterpret_cast<int *>(sw + AC * 32);                 // [AC] first bin
     int *fn = fb + AC;                                               // [AC] bins spanned
     double *red = reinterpret_cast<double *>(fn + AC);               // [NCW]
-    if (A.skip && *A.skip) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int k = tile_lane_ray(A, A.tiles[blockIdx.x], lane);
+    const int k = tile_lane_ray(A, A.tiles[bx], lane);
     const float4 myray = k >= 0 && !A.bpw ? A.ray[k] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int rg = warp & 3, sc = warp >> 2;
-    const int yb = blockIdx.y * SPAN;                  // first slice of the block
+    const int yb = by * SPAN;                  // first slice of the block
     const int yw = sc * 32 * VEC;                        // this warp's slices within the block
     const bool yok = yb + yw + lane_piece<VEC>(lane, 0) < A.ys;
     const size_t ys = (size_t)A.ys;
@@ -465,6 +468,7 @@ __global__ void __launch_bounds__(128 * NSC, NSC == 1 ? 4 : 1)
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int b = 0; b < NB; b++) {
+            if (AGAIN && again) umma::mbar_inval(&full[b]);
             umma::mbar_init(&full[b], 1);
             released[b] = 0;
         }
@@ -487,11 +491,11 @@ __global__ void __launch_bounds__(128 * NSC, NSC == 1 ? 4 : 1)
         const int nac = min(AC, A.na - a0);
         if (A.bpw) {
             // the plan's precomputed entries for this tile and chunk
-            const float4 *src = A.bpw + ((size_t)blockIdx.x * A.na + a0) * 32;
+            const float4 *src = A.bpw + ((size_t)bx * A.na + a0) * 32;
             for (int i = threadIdx.x; i < nac * 32; i += blockDim.x) cp_async16(sw + i, src + i, true);
             cp_async_commit();
             for (int i = threadIdx.x; i < nac; i += blockDim.x) {
-                const int2 f = A.bpf[(size_t)blockIdx.x * A.na + a0 + i];
+                const int2 f = A.bpf[(size_t)bx * A.na + a0 + i];
                 fb[i] = f.x;
                 fn[i] = f.y;
             }
@@ -515,7 +519,7 @@ __global__ void __launch_bounds__(128 * NSC, NSC == 1 ? 4 : 1)
         if (warp == 0) {
             for (int ai = 0; ai < min(NB, nac); ai++) {
                 const int buf = (t0 + ai) % NB;
-                bp_stage<FW, SPAN>(A, s, foot + (size_t)buf * FW * SPAN, &full[buf], &tms,
+                bp_stage<FW, SPAN>(A, s, foot + (size_t)buf * FW * SPAN, &full[buf], tms,
                                    use_tma != 0, a0 + ai, fb[ai], fn[ai], yb, row_bytes, ok, lane);
             }
         }
@@ -552,7 +556,7 @@ __global__ void __launch_bounds__(128 * NSC, NSC == 1 ? 4 : 1)
             if (lane == 0) last = (atomicAdd(&released[buf], 1) + 1) % NCW == 0;
             last = __shfl_sync(0xffffffffu, last, 0);
             if (last && ai + NB < nac)
-                bp_stage<FW, SPAN>(A, s, foot + (size_t)buf * FW * SPAN, &full[buf], &tms,
+                bp_stage<FW, SPAN>(A, s, foot + (size_t)buf * FW * SPAN, &full[buf], tms,
                                    use_tma != 0, a0 + ai + NB, fb[ai + NB], fn[ai + NB], yb,
                                    row_bytes, ok, lane);
         }
@@ -575,7 +579,49 @@ __global__ void __launch_bounds__(128 * NSC, NSC == 1 ? 4 : 1)
             for (int q = 0; q < VEC; q++) s2 += (double)__fmul_rn(acc[r][q], acc[r][q]);
         }
     }
-    block_sum_to<NCW>(s2, red, A.partials + (size_t)blockIdx.y * gridDim.x + blockIdx.x);
+    if constexpr (!AGAIN) block_sum_to<NCW>(s2, red, A.partials + (size_t)by * gridDim.x + bx);
+    return ok;
+}
+
+template <int W, int VEC, int NSC>
+__global__ void __launch_bounds__(128 * NSC, NSC == 1 ? 4 : 1)
+    bp_kernel(OpArgs A, const float *__restrict__ s, float *__restrict__ g,
+              const __grid_constant__ CUtensorMap tms, int use_tma) {
+    if (A.skip && *A.skip) return;
+    bp_block<W, VEC, NSC, false>(A, s, g, &tms, use_tma, blockIdx.x, blockIdx.y, false);
+}
+
+// Before a projection on the tensor cores, once its operand is in FP16 pairs: whether a
+// slice's score says that they cannot hold it (see arec_project_mma.cu).  If so the kernel
+// sets *wide, which sends the tensor-core kernel home, and does the projection, its
+// blocks taking turns at the tiles; if not it clears n float4 of the output.
+__device__ __forceinline__ bool operand_wide(const OpArgs &A, const long long *score, int *wide,
+                                             float *out, size_t n) {
+    bool w = false;
+    for (int i = threadIdx.x; i < A.ys; i += blockDim.x) w |= score[i] > 0;
+    if (__syncthreads_or(w)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *wide = 1;
+        return true;
+    }
+    float4 *v = reinterpret_cast<float4 *>(out);
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    return false;
+}
+
+template <int W, int VEC>
+__global__ void __launch_bounds__(128, 4)
+    bp_wide_kernel(OpArgs A, const float *__restrict__ s, float *__restrict__ g,
+                   const __grid_constant__ CUtensorMap tms, int use_tma, int ntiles, int slice_blocks,
+                   const long long *score, int *wide, size_t n_clear) {
+    if (A.skip && *A.skip) return;
+    if (!operand_wide(A, score, wide, g, n_clear)) return;
+    const int n = ntiles * slice_blocks;
+    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+        const bool ok = bp_block<W, VEC, 1, true>(A, s, g, &tms, use_tma, i % ntiles, i / ntiles,
+                                                  i != (int)blockIdx.x);
+        if (__syncthreads_or(!ok)) return;
+    }
 }
 
 // Linear weighting: its ray coordinates are the reference's shifted table
@@ -764,11 +810,13 @@ __device__ __forceinline__ void fp_entry(float (&acc)[BT][VEC], const int GG, co
     if (GG <= BT - 1) fma_row<VEC>(acc[GG <= BT - 1 ? GG : 0], e.w, v);
 }
 
-template <int W, int VEC, int BT>
-__global__ void __launch_bounds__(kFpThreads, 3)
-    fp_band_kernel(OpArgs A, const float *__restrict__ x, float *__restrict__ q, int g0, int ngo,
-                   int band_lo, int band_hi, const __grid_constant__ CUtensorMap tmx,
-                   const __grid_constant__ CUtensorMap tmxT) {
+// Angle group g0 + bx % ngo, bins from BT (bx / ngo) on, slice block by; true unless a
+// wait gave up.  AGAIN: as in bp_block, and without the plan's tables.
+template <int W, int VEC, int BT, bool AGAIN>
+__device__ __forceinline__ bool fp_band_block(const OpArgs &A, const float *__restrict__ x,
+                                              float *__restrict__ q, int g0, int ngo, int band_lo,
+                                              int band_hi, const CUtensorMap *tmx, const CUtensorMap *tmxT,
+                                              int bx, int by, bool again) {
     constexpr int NA = kGroupAngles, NG = BT + 2, SPAN = 32 * VEC, US = kFpStage;
     static_assert(NG <= 16, "two slot rows of 16 buckets per warp list");
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -781,22 +829,21 @@ __global__ void __launch_bounds__(kFpThreads, 3)
     int *lrange = reinterpret_cast<int *>(rayb + 2 * US * NA);       // [NA][2]
     int *uinfo = lrange + 2 * NA;                                    // [2][2] (first pixel, rows)
     int2 *linfo = reinterpret_cast<int2 *>(uinfo + 4);               // [band lines] (first ray, rows)
-    if (A.skip && *A.skip) return;
     if (band_hi - band_lo > kFpMaxBand) {  // the host keeps bands within kFpMaxBand lines
         if (threadIdx.x == 0) atomicOr(A.err, 1);
-        return;
+        return false;
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool stager = warp == NA;
     const int ai = stager ? 0 : warp;
-    const int grp = g0 + blockIdx.x % ngo, b0 = (blockIdx.x / ngo) * BT;
+    const int grp = g0 + bx % ngo, b0 = (bx / ngo) * BT;
     const int4 G = A.groups[grp];
     const int orient = G.z;
     const float r = A.r_hi + A.r_lo;
     const float T1 = (float)b0 - 1.5f - 0.02f - r;
     const float T2 = (float)(b0 + BT) + 0.5f + 0.02f - r;
     const float R = r + 1.5f;
-    const int yb = blockIdx.y * SPAN;
+    const int yb = by * SPAN;
     const size_t ys = (size_t)A.ys;
     const uint32_t row_bytes = (uint32_t)min(SPAN, A.ys - yb) * 4u;
     const bool angle_ok = !stager && ai < G.y;
@@ -818,6 +865,11 @@ __global__ void __launch_bounds__(kFpThreads, 3)
         lrange[2 * ai + 1] = hi;
     }
     if (threadIdx.x == 0) {
+        if (AGAIN && again)
+            for (int b = 0; b < 2; b++) {
+                umma::mbar_inval(&full[b]);
+                umma::mbar_inval(&empty[b]);
+            }
         umma::mbar_init(&full[0], 1);
         umma::mbar_init(&full[1], 1);
         umma::mbar_init(&empty[0], NA);
@@ -831,7 +883,7 @@ __global__ void __launch_bounds__(kFpThreads, 3)
         L0 = min(L0, lrange[2 * i]);
         L1 = max(L1, lrange[2 * i + 1]);
     }
-    if (L0 > L1) return;  // the strip misses this band (uniform over the block)
+    if (L0 > L1) return true;  // the strip misses this band (uniform over the block)
     bool ok = true;
 
     if (stager) {
@@ -845,7 +897,7 @@ __global__ void __launch_bounds__(kFpThreads, 3)
             q_lo = lrange[2 * lane];
             q_hi = lrange[2 * lane + 1];
         }
-        if (A.taps) {
+        if (!AGAIN && A.taps) {
             // With the plan's tables every line's staging (first ray of the
             // union of the group's candidates, rows) is worked out up front,
             // lanes = lines, so the per-line loop below carries no dependent
@@ -920,13 +972,13 @@ __global__ void __launch_bounds__(kFpThreads, 3)
                 __syncwarp();
                 if (lane < nbox)
                     umma::tma_load_2d(stg + ((size_t)buf * US + lane * kFpBox) * SPAN,
-                                      orient ? &tmxT : &tmx, yb, lf.x + lane * kFpBox, &full[buf]);
+                                      orient ? tmxT : tmx, yb, lf.x + lane * kFpBox, &full[buf]);
                 if (lane == 0 && n)
                     umma::bulk_g2s(rayb + buf * US * NA, A.taps + ((size_t)grp * A.nrays + lf.x) * NA,
                                    (uint32_t)n * 16u * NA, &full[buf]);
                 __syncwarp();
             }
-            return;
+            return ok;
         }
         for (int li = L0; li <= L1; li++) {
             const int it = li - L0, buf = it & 1;
@@ -970,7 +1022,7 @@ __global__ void __launch_bounds__(kFpThreads, 3)
                 umma::bulk_g2s(rayb + (buf * US + lane) * NA, A.ray + k, 16u, &full[buf]);
             }
         }
-        return;
+        return ok;
     }
 
     const int my_lo = lrange[2 * ai], my_hi = lrange[2 * ai + 1];
@@ -994,7 +1046,7 @@ __global__ void __launch_bounds__(kFpThreads, 3)
         if (angle_ok && lane < un && li >= my_lo && li <= my_hi) {
             const int row = ca > 0.f ? lane : un - 1 - lane;
             Taps t;
-            if (A.taps) {
+            if (!AGAIN && A.taps) {
                 const float4 tt = rayb[(buf * US + row) * NA + ai];
                 t.iqx = __float_as_int(tt.x);
                 t.w0 = tt.y;
@@ -1092,13 +1144,57 @@ __global__ void __launch_bounds__(kFpThreads, 3)
         // a wait gave up: let the copies still in flight land before the block exits
         for (int it = max(0, L1 - L0 - 1); it <= L1 - L0; it++)
             umma::mbar_wait(&full[it & 1], (uint32_t)(it >> 1) & 1u, kFpWait);
-        return;
+        return false;
     }
     if (angle_ok) {
         float *qa = q + (size_t)(G.x + ai) * A.nx * ys + yb;
 #pragma unroll
         for (int j = 0; j < BT; j++)
             if (b0 + j < A.nx) add_lane<VEC>(qa + (size_t)(b0 + j) * ys, lane, acc[j], A.ys - yb);
+    }
+    return true;
+}
+
+template <int W, int VEC, int BT>
+__global__ void __launch_bounds__(kFpThreads, 3)
+    fp_band_kernel(OpArgs A, const float *__restrict__ x, float *__restrict__ q, int g0, int ngo,
+                   int band_lo, int band_hi, const __grid_constant__ CUtensorMap tmx,
+                   const __grid_constant__ CUtensorMap tmxT) {
+    if (A.skip && *A.skip) return;
+    fp_band_block<W, VEC, BT, false>(A, x, q, g0, ngo, band_lo, band_hi, &tmx, &tmxT, blockIdx.x,
+                                     blockIdx.y, false);
+}
+
+// The whole forward projection in one launch (see operand_wide): a block takes the same
+// bins and angles in every band, band after band, so each output is added up by one
+// block in the order of the launches above.
+template <int W, int VEC, int BT>
+__global__ void __launch_bounds__(kFpThreads, 3)
+    fp_wide_kernel(OpArgs A, const float *__restrict__ x, float *__restrict__ q, int ngo0, int slice_blocks,
+                   int band, const long long *score, int *wide, size_t n_clear) {
+    if (A.skip && *A.skip) return;
+    if (!operand_wide(A, score, wide, q, n_clear)) return;
+    const int ntile = (A.nx + BT - 1) / BT;
+    bool again = false;
+    for (int o = 0; o < 2; o++) {
+        const int ngo = o ? A.ngroups - ngo0 : ngo0, g0 = o ? ngo0 : 0, n = ngo * ntile;
+        for (int i = blockIdx.x; i < n * slice_blocks; i += gridDim.x) {  // q = 0
+            const int4 G = A.groups[g0 + i % n % ngo];
+            const int b0 = i % n / ngo * BT, nb = min(BT, A.nx - b0);
+            const int y0 = i / n * 32 * VEC, ny = min(32 * VEC, A.ys - y0);
+            for (int t = threadIdx.x; t < G.y * nb * ny; t += kFpThreads)
+                q[((size_t)(G.x + t / (nb * ny)) * A.nx + b0 + t / ny % nb) * A.ys + y0 + t % ny] = 0.f;
+        }
+        __syncthreads();
+        for (int lo = 0; lo < A.nx; lo += band)
+            for (int i = blockIdx.x; i < n * slice_blocks; i += gridDim.x) {
+                const bool ok = fp_band_block<W, VEC, BT, true>(A, x, q, g0, ngo, lo, min(A.nx, lo + band),
+                                                                nullptr, nullptr, i % n, i / n, again);
+                // this item's reads of shared memory before the next one's copies
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                if (__syncthreads_or(!ok)) return;
+                again = true;
+            }
     }
 }
 
@@ -1343,6 +1439,43 @@ int launch_fpb(const OpArgs &A, int vec, dim3 grid, const float *x, float *q, in
     if (vec == 2) return launch_fpb_one<W, 2, BT>(A, grid, x, q, g0, ngo, lo, hi, tmx, tmxT, st);
     if (vec == 4) return launch_fpb_one<W, 4, BT>(A, grid, x, q, g0, ngo, lo, hi, tmx, tmxT, st);
     return launch_fpb_one<W, 8, BT>(A, grid, x, q, g0, ngo, lo, hi, tmx, tmxT, st);
+}
+
+// fp_wide_kernel or bp_wide_kernel: as many blocks as run at a time.
+template <int W, int V>
+int launch_wide_one(const OpArgs &A, int ntiles, int ngo0, int band, const float *in, float *out, bool back,
+                    const WideArgs &w, cudaStream_t st) {
+    constexpr size_t smem = bp_smem_bytes<V, 1>(), fsmem = fpb_smem_bytes<V>();
+    static bool configured = false;  // per instantiation, once per process
+    if (!configured) {
+        if (cudaFuncSetAttribute(bp_wide_kernel<W, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem) != cudaSuccess ||
+            cudaFuncSetAttribute(fp_wide_kernel<W, V, kFpBins>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)fsmem) != cudaSuccess)
+            return -2;
+        configured = true;
+    }
+    const int slices = (A.ys + 32 * V - 1) / (32 * V);
+    if (back) {
+        CUtensorMap tms;
+        memset(&tms, 0, sizeof(tms));
+        const int use_tma = encode_sino_map(&tms, in, A.ys, A.nx, A.na, 32 * V, kBpFoot);
+        bp_wide_kernel<W, V><<<152 * 4, 128, smem, st>>>(A, in, out, tms, use_tma, ntiles, slices, w.score,
+                                                         w.wide, w.n_clear);
+    } else {
+        fp_wide_kernel<W, V, kFpBins><<<152 * 3, kFpThreads, fsmem, st>>>(A, in, out, ngo0, slices, band,
+                                                                          w.score, w.wide, w.n_clear);
+    }
+    return 0;
+}
+
+template <int W>
+int launch_wide(const OpArgs &A, int vec, int ntiles, int ngo0, int band, const float *in, float *out,
+                bool back, const WideArgs &w, cudaStream_t st) {
+    if (vec == 1) return launch_wide_one<W, 1>(A, ntiles, ngo0, band, in, out, back, w, st);
+    if (vec == 2) return launch_wide_one<W, 2>(A, ntiles, ngo0, band, in, out, back, w, st);
+    if (vec == 4) return launch_wide_one<W, 4>(A, ntiles, ngo0, band, in, out, back, w, st);
+    return launch_wide_one<W, 8>(A, ntiles, ngo0, band, in, out, back, w, st);
 }
 
 // Linear weighting: the gather when the plan has its ray index, else the

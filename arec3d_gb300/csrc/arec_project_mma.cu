@@ -34,6 +34,11 @@ namespace arecgb {
 
 bool encode_half_map(CUtensorMap *m, const void *base, int ys, int n1, int n2, int box1, int box2);
 bool encode_foot_map(CUtensorMap *m, const void *base, int nx, int groups, int na, int box_bins);
+// arec_project_{kb,sq}.cu
+int launch_wide_kb(const OpArgs &, int, int, int, int, const float *, float *, bool, const WideArgs &,
+                   cudaStream_t);
+int launch_wide_sq(const OpArgs &, int, int, int, int, const float *, float *, bool, const WideArgs &,
+                   cudaStream_t);
 
 namespace {
 
@@ -60,14 +65,14 @@ constexpr int kSegBlocks = 64;  // line blocks of a segment at most
 // around zero reach below it in about 2^-28 of the cases, the rounding noise that an
 // FP32 transform leaves on a background of zeros (2^-25 of the largest) in 2 %.
 constexpr float kSmall = 1.f / 32768.f;
-constexpr int kScoreSmall = 31;
+constexpr int kScoreSmall = 32;
 constexpr int kScoreShared = 4096;  // slices whose scores a block adds up in shared memory
 
 // Per plan and direction, beside the operand: zeroed before the largest magnitudes are
 // taken; mma_stats_bytes.
 struct HalfStats {
     unsigned *maxb;              // [ys] largest magnitude per slice
-    unsigned long long *score;   // [ys] kScoreSmall for a small value, -1 for any other
+    unsigned long long *score;   // [ys] see add_score
     int *wide;                   // set when one is positive: the operand takes FP32 kernels
     int ys;
 };
@@ -112,69 +117,75 @@ __device__ __forceinline__ unsigned pack_half(float a, float b, float &ra, float
     return (unsigned)__half_as_ushort(ha) | ((unsigned)__half_as_ushort(hb) << 16);
 }
 
-// Eight slices: scaled, high and low halves.  score: a nonzero value below kSmall
-// adds kScoreSmall, any other nonzero one takes 1.
-__device__ __forceinline__ void half_pair(const float4 *v, const uint4 &ma, const uint4 &mb, uint4 &hi,
-                                          uint4 &lo, int (&score)[8]) {
-    const float4 a = v[0], b = v[1];
-    const float raw[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    const unsigned m[8] = {ma.x, ma.y, ma.z, ma.w, mb.x, mb.y, mb.z, mb.w};
-    float f[8], l[8], d0, d1;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        f[i] = raw[i] * pow2f(half_shift(m[i]));
-        if (raw[i] != 0.f) score[i] += fabsf(f[i]) < kSmall ? kScoreSmall : -1;
-    }
-    hi.x = pack_half(f[0], f[1], l[0], l[1]);
-    hi.y = pack_half(f[2], f[3], l[2], l[3]);
-    hi.z = pack_half(f[4], f[5], l[4], l[5]);
-    hi.w = pack_half(f[6], f[7], l[6], l[7]);
-#pragma unroll
-    for (int i = 0; i < 8; i++) l[i] *= kLowScale;
-    lo.x = pack_half(l[0], l[1], d0, d1);
-    lo.y = pack_half(l[2], l[3], d0, d1);
-    lo.z = pack_half(l[4], l[5], d0, d1);
-    lo.w = pack_half(l[6], l[7], d0, d1);
+// A slice's score: kScoreSmall for every nonzero value below kSmall, less 1 for every
+// nonzero value.  A block adds it up in shared memory (cnt: a counter per slice), or
+// straight in S.score when there are too many slices for that.
+__device__ __forceinline__ void add_score(const HalfStats &S, int *cnt, int slice, int v) {
+    if (S.ys <= kScoreShared) atomicAdd(cnt + slice, v);
+    else atomicAdd(S.score + slice, (unsigned long long)(long long)v);
 }
 
-// A conversion's end: the scores of the block's lanes lane mod step (slices 8 m ..,
-// m < 0: none) to the slices' sums.  cnt: shared memory (zeroed, a barrier later), a
-// counter per slice where kScoreShared of them are enough.
+// A thread's eight slices 8 m ..: their scales and its nonzero values, two counts of 16
+// bits to a register (a thread of a grid as large as those below has less than 2^16
+// rows of anything that fits the memory).
+struct HalfLane {
+    float scale[8];
+    unsigned count[4] = {0, 0, 0, 0};
+    int m;
+
+    __device__ __forceinline__ HalfLane(const HalfStats &S, int m_) : m(m_) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) scale[i] = pow2f(half_shift(S.maxb[8 * m + i]));
+    }
+    // Scaled, high and low halves.
+    __device__ __forceinline__ void pair(const float4 *v, const HalfStats &S, int *cnt, uint4 &hi, uint4 &lo) {
+        const float4 a = v[0], b = v[1];
+        const float raw[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        float f[8], l[8], d0, d1;
+        unsigned small = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            f[i] = raw[i] * scale[i];
+            if (raw[i] != 0.f) {
+                count[i >> 1] += i & 1 ? 0x10000u : 1u;
+                if (fabsf(f[i]) < kSmall) small |= 1u << i;
+            }
+        }
+        hi.x = pack_half(f[0], f[1], l[0], l[1]);
+        hi.y = pack_half(f[2], f[3], l[2], l[3]);
+        hi.z = pack_half(f[4], f[5], l[4], l[5]);
+        hi.w = pack_half(f[6], f[7], l[6], l[7]);
+#pragma unroll
+        for (int i = 0; i < 8; i++) l[i] *= kLowScale;
+        lo.x = pack_half(l[0], l[1], d0, d1);
+        lo.y = pack_half(l[2], l[3], d0, d1);
+        lo.z = pack_half(l[4], l[5], d0, d1);
+        lo.w = pack_half(l[6], l[7], d0, d1);
+        for (; small; small &= small - 1) add_score(S, cnt, 8 * m + __ffs(small) - 1, kScoreSmall);
+    }
+    __device__ __forceinline__ void finish(const HalfStats &S, int *cnt) const {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int n = (int)(count[i >> 1] >> (i & 1 ? 16 : 0) & 0xffffu);
+            if (n) add_score(S, cnt, 8 * m + i, -n);
+        }
+    }
+};
+
+// Before the block's first and after its last values.
 __device__ __forceinline__ void start_scores(const HalfStats &S, int *cnt) {
     if (S.ys <= kScoreShared)
         for (int i = threadIdx.x; i < S.ys; i += 256) cnt[i] = 0;
     __syncthreads();
 }
-__device__ __forceinline__ void add_scores(const HalfStats &S, int m, int step, int (&score)[8], int *cnt) {
-    const bool sm = S.ys <= kScoreShared;
-    for (int o = 16; o >= step; o >>= 1)
-#pragma unroll
-        for (int i = 0; i < 8; i++) score[i] += __shfl_xor_sync(0xffffffffu, score[i], o);
-    if (m >= 0 && (int)(threadIdx.x & 31) < step)
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            if (sm) atomicAdd(&cnt[8 * m + i], score[i]);
-            else if (score[i]) atomicAdd(S.score + 8 * m + i, (unsigned long long)(long long)score[i]);
-        }
+__device__ __forceinline__ void finish_scores(const HalfStats &S, const int *cnt) {
     __syncthreads();
-    if (sm)
+    if (S.ys <= kScoreShared)
         for (int i = threadIdx.x; i < S.ys; i += 256)
             if (cnt[i]) atomicAdd(S.score + i, (unsigned long long)(long long)cnt[i]);
     if (blockIdx.x == 0)
         for (int i = threadIdx.x; i < S.ys; i += 256)
             if (S.maxb[i] >= kWideBits) atomicAdd(S.score + i, 1ull << 62);
-}
-
-// v = 0 unless the solve has finished; and the operand's flag (a block of the
-// conversion that waited for the others to set it would cost 3 us, the projectors'
-// blocks 1 us each if they added the scores up to it themselves).
-__global__ void __launch_bounds__(256) k_clear(float4 *v, size_t n, const int *skip, const HalfStats S) {
-    if (skip && *skip) return;
-    if (blockIdx.x == 0)
-        for (int i = threadIdx.x; i < S.ys; i += 256)
-            if ((long long)S.score[i] > 0) *S.wide = 1;
-    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256)
-        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // Rows [n][ys] as FP16 pairs [2][rows][ys], row r at place[r].  The grid's threads are a
@@ -187,17 +198,16 @@ __global__ void __launch_bounds__(256)
     start_scores(S, sm_score);
     const size_t total = n * ys8, t0 = (size_t)blockIdx.x * 256 + threadIdx.x;
     const int m = (int)(t0 % ys8);
-    const uint4 ma = reinterpret_cast<const uint4 *>(S.maxb)[2 * m];
-    const uint4 mb = reinterpret_cast<const uint4 *>(S.maxb)[2 * m + 1];
-    int score[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    HalfLane h(S, m);
     for (size_t t = t0; t < total; t += (size_t)gridDim.x * 256) {
         uint4 hi, lo;
-        half_pair(v + 2 * t, ma, mb, hi, lo, score);
+        h.pair(v + 2 * t, S, sm_score, hi, lo);
         const size_t o = (size_t)place[t / ys8] * ys8 + m;
         out[o] = hi;
         out[rows * ys8 + o] = lo;
     }
-    add_scores(S, m, 32 % ys8 ? 32 : ys8, score, sm_score);
+    h.finish(S, sm_score);
+    finish_scores(S, sm_score);
 }
 
 // The sinogram [na][nx][ys] as FP16 pairs [2][na][ys/8][nx][8] (the back
@@ -215,22 +225,21 @@ __global__ void __launch_bounds__(256)
     const size_t total = (size_t)na * nbb * nmb, half = (size_t)na * ys8 * nx;
     const size_t t0 = (size_t)blockIdx.x * 8 + warp;
     const int m = (int)(t0 % nmb) * 4 + (lane & 3);
-    int score[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (m < ys8) {
-        const uint4 ma = reinterpret_cast<const uint4 *>(S.maxb)[2 * m];
-        const uint4 mb = reinterpret_cast<const uint4 *>(S.maxb)[2 * m + 1];
+        HalfLane h(S, m);
         for (size_t t = t0; t < total; t += (size_t)gridDim.x * 8) {
             const int b = (int)(t / nmb % nbb) * 8 + (lane >> 2);
             const size_t a = t / nmb / nbb;
             if (b >= nx) continue;
             uint4 hi, lo;
-            half_pair(v + ((a * nx + b) * ys8 + m) * 2, ma, mb, hi, lo, score);
+            h.pair(v + ((a * nx + b) * ys8 + m) * 2, S, sm_score, hi, lo);
             const size_t o = (a * ys8 + m) * nx + b;
             out[o] = hi;
             out[half + o] = lo;
         }
+        h.finish(S, sm_score);
     }
-    add_scores(S, m < ys8 ? m : -1, 4, score, sm_score);
+    finish_scores(S, sm_score);
 }
 
 // ---------------------------------------------------------------------------
@@ -634,39 +643,6 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
     if (warp == kLoadWarp) umma::tmem_dealloc(tmem, C::COLS);
 }
 
-// Forward projection of a volume that holds an infinity or a NaN (the blocks'
-// dense products would spread it to neighbouring bins): per output, the rays of
-// each line near the bin.  Returns at once otherwise.
-template <int W>
-__global__ void __launch_bounds__(128)
-    fp_any_kernel(OpArgs A, const float *__restrict__ x, float *__restrict__ q,
-                  const int *__restrict__ wide) {
-    if ((A.skip && *A.skip) || !*wide) return;
-    const float r = A.r_hi + A.r_lo;
-    for (long long t = blockIdx.x; t < (long long)A.na * A.nx; t += gridDim.x) {
-        const int a = (int)(t / A.nx), b = (int)(t % A.nx);
-        const AngleParams ap = A.ang[a];
-        const int orient = ap.orient;
-        const float ca = orient ? ap.s : ap.c, cl = orient ? ap.c : ap.s;
-        for (int y = threadIdx.x; y < A.ys; y += blockDim.x) {
-            float s = 0.f;
-            for (int li = 0; li < A.nx; li++) {
-                int st, lo, hi;
-                line_info(A, orient, li, st, lo, hi);
-                const float pc = ((float)b - r - ((float)li - r) * cl) / ca + r;
-                for (int P = max(lo, (int)floorf(pc) - 3); P <= min(hi, (int)floorf(pc) + 4); P++) {
-                    const int k = orient ? A.kinv[st + P - lo] : st + P - lo;
-                    const Taps tp = ray_taps<W>(A.ray[k], ap, A.r_hi, A.r_lo);
-                    const int d = b - (tp.iqx - 1);
-                    if (d >= 0 && d < 3)
-                        s = fmaf(d == 0 ? tp.w0 : (d == 1 ? tp.w1 : tp.w2), x[(size_t)k * A.ys + y], s);
-                }
-            }
-            q[(size_t)t * A.ys + y] = s;
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Back projection  g[k][y] = sum_a sum_j w_j(k, a) s[a][b(k, a) + j][y].
 //   D[y][k] += sum over a window of 16 bins of S[y][b] W[b][k]:
@@ -987,30 +963,6 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
     if (warp == kLoadWarp) umma::tmem_dealloc(tmem, C::COLS);
 }
 
-// Back projection of a sinogram that holds an infinity or a NaN; returns at once
-// otherwise.
-template <int W>
-__global__ void __launch_bounds__(128)
-    bp_any_kernel(OpArgs A, const float *__restrict__ s, float *__restrict__ g,
-                  const int *__restrict__ wide) {
-    if ((A.skip && *A.skip) || !*wide) return;
-    for (int k = blockIdx.x; k < A.nrays; k += gridDim.x)
-        for (int y = threadIdx.x; y < A.ys; y += blockDim.x) {
-            float v = 0.f;
-            for (int a = 0; a < A.na; a++) {
-                const Taps t = ray_taps<W>(A.ray[k], A.ang[a], A.r_hi, A.r_lo);
-                const float *sa = s + (size_t)a * A.nx * A.ys + y;
-#pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    const int b = t.iqx - 1 + j;
-                    if ((unsigned)b < (unsigned)A.nx)
-                        v = fmaf(j == 0 ? t.w0 : (j == 1 ? t.w1 : t.w2), sa[(size_t)b * A.ys], v);
-                }
-            }
-            g[(size_t)k * A.ys + y] = v;
-        }
-}
-
 // ---------------------------------------------------------------------------
 // Plan: groups, strips and segments.
 
@@ -1289,8 +1241,7 @@ unsigned blocks_of(int unit, size_t blocks) {
 size_t score_bytes(int ys) { return ys <= kScoreShared ? sizeof(int) * ys : 0; }
 
 template <int W, int MT>
-int launch_fp_mma(const Work &w, const OpArgs &A, const MmaPlan &M, const CUtensorMap &tx,
-                  const float *x, float *q) {
+int launch_fp_mma(const Work &w, const OpArgs &A, const MmaPlan &M, const CUtensorMap &tx, float *q) {
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;
     std::call_once(once, [] {
@@ -1303,10 +1254,28 @@ int launch_fp_mma(const Work &w, const OpArgs &A, const MmaPlan &M, const CUtens
         for (int color = 0; color < 3; color++)
             fp_mma_kernel<W, MT><<<grid, kMmaThreads, FpMma<MT>::SMEM, w.st>>>(A, M, tx, q, w.smax,
                                                                                w.stats.wide, seg, color);
-    fp_any_kernel<W><<<152 * 4, 128, 0, w.st>>>(A, x, q, w.stats.wide);
-    count_launches(3 * M.max_segs + 1);
+    count_launches(3 * M.max_segs);
     ARECGB_CUDA(cudaGetLastError());
     return 0;
+}
+
+// An operand that the pairs cannot hold is projected here, on the FP32 kernels (without
+// the plan's tables); for any other n_clear float4 of the output are cleared.  One value
+// of 1e12 or an infinity at 512^2 x 360 x 128: 10.8 ms forward and 4.4 back (1.9 and 1.6
+// on the tensor cores, 7.0 and 3.2 on the FP32 kernels with tables, as a plan with few
+// angles or slices has them); at 1024^2 x 1200 x 512 240 and 146 (44, 73; 160, 209).  A
+// kernel of its own that took the rays one by one for each output was 361 and 46 at the
+// first size.
+int wide_step(const Work &w, OpArgs A, const float *in, float *out, bool back, size_t n_clear) {
+    const Plan *p = w.p;
+    A.taps = nullptr;
+    const auto launch = p->weighting == ARECGB_KB ? launch_wide_kb : launch_wide_sq;
+    const int vec = back ? (p->bp_vec ? p->bp_vec : p->vec) : (p->fp_vec ? p->fp_vec : p->vec);
+    const WideArgs wa{(const long long *)w.stats.score, w.stats.wide, n_clear};
+    const int rc = launch(A, vec, p->ntiles, p->ngroups_o[0], p->fp_band, in, out, back, wa, w.st);
+    count_launches(1);
+    ARECGB_CUDA(cudaGetLastError());
+    return rc ? ARECGB_ERR_ARG : 0;
 }
 
 int fp_steps(const Work &w, const OpArgs &A, const float *d_x, float *d_q) {
@@ -1318,10 +1287,8 @@ int fp_steps(const Work &w, const OpArgs &A, const float *d_x, float *d_q) {
     k_to_half<<<blocks_of(unit, std::min<size_t>(152 * 4, (total + 255) / 256)), 256, score_bytes(p->ys),
                 w.st>>>((const float4 *)d_x, n, ys8, w.stats, p->d_mpix, (size_t)p->nx * p->nx,
                         (uint4 *)w.half, A.skip);
-    const size_t nq = sin_floats(p) / 4;
-    k_clear<<<(unsigned)std::min<size_t>(152 * 8, (nq + 255) / 256), 256, 0, w.st>>>((float4 *)d_q, nq,
-                                                                                    A.skip, w.stats);
-    count_launches(2);
+    count_launches(1);
+    if (int rc = wide_step(w, A, d_x, d_q, false, sin_floats(p) / 4)) return rc;
     CUtensorMap tx;
     if (!encode_half_map(&tx, w.half, p->ys, p->nx, p->nx, 8, 8)) {
         set_error("forward_project: tensor map encoding failed");
@@ -1330,14 +1297,12 @@ int fp_steps(const Work &w, const OpArgs &A, const float *d_x, float *d_q) {
     const MmaPlan M = make_plan(p);
     const bool kb = p->weighting == ARECGB_KB;
     if (p->ys > 128)
-        return kb ? launch_fp_mma<ARECGB_KB, 2>(w, A, M, tx, d_x, d_q)
-                  : launch_fp_mma<ARECGB_SQ, 2>(w, A, M, tx, d_x, d_q);
-    return kb ? launch_fp_mma<ARECGB_KB, 1>(w, A, M, tx, d_x, d_q)
-              : launch_fp_mma<ARECGB_SQ, 1>(w, A, M, tx, d_x, d_q);
+        return kb ? launch_fp_mma<ARECGB_KB, 2>(w, A, M, tx, d_q) : launch_fp_mma<ARECGB_SQ, 2>(w, A, M, tx, d_q);
+    return kb ? launch_fp_mma<ARECGB_KB, 1>(w, A, M, tx, d_q) : launch_fp_mma<ARECGB_SQ, 1>(w, A, M, tx, d_q);
 }
 
 template <int W>
-int launch_bp_mma(const Work &w, const OpArgs &A, const CUtensorMap &ts, const float *s, float *g) {
+int launch_bp_mma(const Work &w, const OpArgs &A, const CUtensorMap &ts, float *g, bool halves) {
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;
     std::call_once(once, [] {
@@ -1345,19 +1310,10 @@ int launch_bp_mma(const Work &w, const OpArgs &A, const CUtensorMap &ts, const f
                                     (int)BpMma::smem(BpMma::MAX_NA));
     });
     ARECGB_CUDA(attr);
-    // Two blocks per tile, half of the angles each, where the SMs' last wave gains: one
-    // wave lasts as long as its angles (256^2 x 180 x 64, 208 tiles: two waves of 90
-    // pairs or three of 45).
-    const int n = w.p->m_tiles * ((A.ys + 127) / 128);
-    const bool halves = A.na >= 32 && 10 * ((2 * n + 151) / 152) < 18 * ((n + 151) / 152);
-    k_clear<<<halves ? 152 * 4 : 1, 256, 0, w.st>>>((float4 *)g, halves ? vol_floats(w.p) / 4 : 0, A.skip,
-                                                    w.stats);
-    count_launches(1);
     bp_mma_kernel<W><<<dim3(w.p->m_tiles, (A.ys + 127) / 128, halves ? 2 : 1), kMmaThreads,
                        BpMma::smem(A.na), w.st>>>(
         A, make_plan(w.p), ts, g, w.smax, w.stats.wide);
-    bp_any_kernel<W><<<152 * 4, 128, 0, w.st>>>(A, s, g, w.stats.wide);
-    count_launches(2);
+    count_launches(1);
     ARECGB_CUDA(cudaGetLastError());
     return 0;
 }
@@ -1376,8 +1332,14 @@ int bp_steps(const Work &w, const OpArgs &A, const float *d_s, float *d_g) {
         set_error("back_project: tensor map encoding failed");
         return ARECGB_ERR_ARG;
     }
-    return p->weighting == ARECGB_KB ? launch_bp_mma<ARECGB_KB>(w, A, ts, d_s, d_g)
-                                     : launch_bp_mma<ARECGB_SQ>(w, A, ts, d_s, d_g);
+    // Two blocks per tile, half of the angles each, where the SMs' last wave gains: one
+    // wave lasts as long as its angles (256^2 x 180 x 64, 208 tiles: two waves of 90
+    // pairs or three of 45).
+    const int n = p->m_tiles * ((A.ys + 127) / 128);
+    const bool halves = A.na >= 32 && 10 * ((2 * n + 151) / 152) < 18 * ((n + 151) / 152);
+    if (int rc = wide_step(w, A, d_s, d_g, true, halves ? vol_floats(p) / 4 : 0)) return rc;
+    return p->weighting == ARECGB_KB ? launch_bp_mma<ARECGB_KB>(w, A, ts, d_g, halves)
+                                     : launch_bp_mma<ARECGB_SQ>(w, A, ts, d_g, halves);
 }
 
 }  // namespace

@@ -18,4 +18,9 @@ int launch_tables_sq(const OpArgs &A, int ntiles, float4 *taps, float4 *bpw, int
     return launch_tables<ARECGB_SQ>(A, ntiles, taps, bpw, bpf, st);
 }
 
+int launch_wide_sq(const OpArgs &A, int vec, int ntiles, int ngo0, int band, const float *in, float *out,
+                   bool back, const WideArgs &w, cudaStream_t st) {
+    return launch_wide<ARECGB_SQ>(A, vec, ntiles, ngo0, band, in, out, back, w, st);
+}
+
 }  // namespace arecgb

@@ -172,6 +172,10 @@ __device__ __forceinline__ void tmem_wait_st() {
 }
 
 // --- mbarrier -------------------------------------------------------------------------------
+// Before a barrier that has been used is initialised again.
+__device__ __forceinline__ void mbar_inval(uint64_t *mbar) {
+    asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_addr(mbar)) : "memory");
+}
 __device__ __forceinline__ void mbar_init(uint64_t *mbar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(mbar)), "r"(count)
                  : "memory");
