@@ -49,10 +49,16 @@ constexpr uint32_t kMmaWait = 1u << 22;
 // idle: registers are handed over by groups of four warps).
 constexpr int kTakers = 8, kBuilders = 8, kLoadWarp = 16, kMmaWarp = 17;
 constexpr int kMmaThreads = 32 * 20;
-// Of a block's sum over 64 rays of one sign the tensor core's rounding toward zero
-// takes 8e-8 on average (measured at 256 to 1024 pixels), of two angles' 5.5e-8:
-// the takers give it back, by this factor on 5 of 8 and on every second sum.
-constexpr float kUnbias = 1.f + 1.1920929e-7f;
+// The tensor core's rounding toward zero takes part of every sum: at 129 to 512 pixels
+// 8.8e-8 of a forward projection of data of one sign, 6.9e-8 with both signs, 3.8e-8 at
+// 5 % of the rays (back 4.9e-8, 4.5e-8, 3.6e-8), nothing of sums that are exact.  The
+// conversion adds this share of a value to its low half: the same for every ray and
+// angle, so A and A^T stay transposes of each other but for their scale.  Errors
+// against FP64 at 256 pixels, 64 angles: dense 6.5e-8 and 4.3e-8 back (1.09e-7 and 6.4e-8
+// without, FP32 kernels 1.34e-7 and 1.66e-7), 5 % of the rays 6.4e-8 and 5.2e-8 (7.0e-8,
+// 6.3e-8; 4.8e-8, 5.2e-8), single rays 8.6e-8 and 5.3e-8 (5.4e-8, 5.3e-8; 4.3e-8, 4.0e-8):
+// what lost nothing is off by the share and its rounding, less than one last place.
+constexpr float kLostForward = 8e-8f, kLostBack = 4.5e-8f;
 constexpr int kSegBlocks = 64;  // line blocks of a segment at most
 
 // ---------------------------------------------------------------------------
@@ -137,8 +143,9 @@ struct HalfLane {
 #pragma unroll
         for (int i = 0; i < 8; i++) scale[i] = pow2f(half_shift(S.maxb[8 * m + i]));
     }
-    // Scaled, high and low halves.
-    __device__ __forceinline__ void pair(const float4 *v, const HalfStats &S, int *cnt, uint4 &hi, uint4 &lo) {
+    // Scaled, high and low halves (with `share` of the value more).
+    __device__ __forceinline__ void pair(const float4 *v, float share, const HalfStats &S, int *cnt, uint4 &hi,
+                                         uint4 &lo) {
         const float4 a = v[0], b = v[1];
         const float raw[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
         float f[8], l[8], d0, d1;
@@ -156,7 +163,7 @@ struct HalfLane {
         hi.z = pack_half(f[4], f[5], l[4], l[5]);
         hi.w = pack_half(f[6], f[7], l[6], l[7]);
 #pragma unroll
-        for (int i = 0; i < 8; i++) l[i] *= kLowScale;
+        for (int i = 0; i < 8; i++) l[i] = fmaf(f[i], share, l[i]) * kLowScale;
         lo.x = pack_half(l[0], l[1], d0, d1);
         lo.y = pack_half(l[2], l[3], d0, d1);
         lo.z = pack_half(l[4], l[5], d0, d1);
@@ -201,7 +208,7 @@ __global__ void __launch_bounds__(256)
     HalfLane h(S, m);
     for (size_t t = t0; t < total; t += (size_t)gridDim.x * 256) {
         uint4 hi, lo;
-        h.pair(v + 2 * t, S, sm_score, hi, lo);
+        h.pair(v + 2 * t, kLostForward, S, sm_score, hi, lo);
         const size_t o = (size_t)place[t / ys8] * ys8 + m;
         out[o] = hi;
         out[rows * ys8 + o] = lo;
@@ -232,7 +239,7 @@ __global__ void __launch_bounds__(256)
             const size_t a = t / nmb / nbb;
             if (b >= nx) continue;
             uint4 hi, lo;
-            h.pair(v + ((a * nx + b) * ys8 + m) * 2, S, sm_score, hi, lo);
+            h.pair(v + ((a * nx + b) * ys8 + m) * 2, kLostBack, S, sm_score, hi, lo);
             const size_t o = (a * ys8 + m) * nx + b;
             out[o] = hi;
             out[half + o] = lo;
@@ -604,7 +611,6 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
                             umma::mbar_wait(&accfull[b], (uint32_t)(it / 2) & 1u, kMmaWait));
             if (!ok) break;
             umma::fence_after_sync();
-            const float unbias = (it & 7) < 5 ? kUnbias : 1.f;
             const uint32_t col = tmem + ((uint32_t)(32 * quarter) << 16) +
                                  (uint32_t)((b * MT + mt) * 128 + c0);
 #pragma unroll
@@ -613,7 +619,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
                     float v[16];
                     umma::tmem_ld16(col + 16 * c, v);
 #pragma unroll
-                    for (int i = 0; i < 16; i++) acc[16 * c + i] = fmaf(v[i], unbias, acc[16 * c + i]);
+                    for (int i = 0; i < 16; i++) acc[16 * c + i] += v[i];
                 }
             umma::fence_before_sync();
             __syncwarp();
@@ -913,8 +919,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
         unsigned long long acc[64];
 #pragma unroll
         for (int i = 0; i < 64; i++) acc[i] = 0ull;
-        const uint32_t f0 = __float_as_uint(kLowScale), f1 = __float_as_uint(kLowScale * kUnbias);
-        const unsigned long long scale0 = pair(f0, f0), scale1 = pair(f1, f1);
+        const unsigned long long scale = pair(__float_as_uint(kLowScale), __float_as_uint(kLowScale));
         bool ok = true;
         for (int it = 0; it < ns; it++) {
             const int b = it & 1;
@@ -923,7 +928,6 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
             if (!ok) break;
             umma::fence_after_sync();
             const uint32_t col = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(b * 256 + half * 128);
-            const unsigned long long scale = it & 1 ? scale1 : scale0;
 #pragma unroll
             for (int c = 0; c < 8; c++) {
                 uint32_t v[16];
