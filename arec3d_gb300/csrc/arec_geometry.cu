@@ -252,9 +252,13 @@ int plan_create(Plan **out, int weighting, double radius, int ny, int nangles,
         // ntiles x ceil(ys / (32 max(1, vec / 2))) blocks
         const int hv = std::max(1, p->vec / 2);
         const int bp_max = p->ntiles * ((p->ys + 32 * hv - 1) / (32 * hv));
-        p->n_partials = std::max(std::max(fp_grid_blocks(p), bp_grid_blocks(p)), bp_max);
-        e = cudaMalloc(&p->d_partials, sizeof(double) * (size_t)p->n_partials);
+        p->n_partials = std::max(bp_grid_blocks(p), bp_max);
+        e = cudaMalloc(&p->d_partials,
+                       sizeof(double) * ((size_t)fp_grid_blocks(p) + std::max(p->n_partials, kNormBlocks)));
+        if (e == cudaSuccess) p->d_bp_partials = p->d_partials + fp_grid_blocks(p);
     }
+    for (auto &ev : p->turn_ev)
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
         set_error(std::string("plan_create: ") + cudaGetErrorString(e));
@@ -297,6 +301,8 @@ void plan_destroy(Plan *p) {
     cudaFree(p->d_bpw);
     cudaFree(p->d_bpf);
     mma_plan_destroy(p);
+    for (auto &ev : p->turn_ev)
+        if (ev) cudaEventDestroy(ev);
     cudaFree(p->d_err);
     cudaFree(p->d_partials);
     for (auto &v : p->d_vol) cudaFree(v);

@@ -91,12 +91,13 @@ struct Plan {
     int2 *d_mtiles = nullptr;     // back projection: 16 x 16-pixel tiles
     int m_tiles = 0;
     // FP16 pairs of the volume and of the sinogram, [0] forward and [1] back
-    // projection; per slice the largest magnitude, then the wide-range flag; the
-    // end of the last call that used them
+    // projection, and their HalfStats
     void *d_half[2] = {nullptr, nullptr};
     unsigned *d_smax[2] = {nullptr, nullptr};
-    cudaEvent_t half_ev[2] = {nullptr, nullptr};
-    mutable std::mutex half_lock[2];
+    // scratch of a projection in either direction (Turn): the end of the last call
+    // that used it, and the call that is being launched
+    cudaEvent_t turn_ev[2] = {nullptr, nullptr};
+    mutable std::mutex turn_lock[2];
     int tuned = 0;                // launch shapes chosen by plan_autotune
     int2 *d_tiles = nullptr;      // back-projection ray tiles: (ix0, iz0) of 8x4-pixel tiles
     int ntiles = 0;
@@ -107,8 +108,9 @@ struct Plan {
     int fp_bins = 16;             // detector bins per forward-projection block
     int bp_rays = 32;             // rays per back-projection block
 
-    // FP64 reduction partial sums (one per block of FP / BP)
-    double *d_partials = nullptr;
+    // FP64 reduction partial sums: one per block for the solvers (and the forward
+    // projection's norm), then the back projection's
+    double *d_partials = nullptr, *d_bp_partials = nullptr;
     int n_partials = 0;
 
     // scratch owned by the plan for the reference-compatible entry points
@@ -165,11 +167,29 @@ void scratch_trim();  // arec_ccorr.cu: gives unused alignment scratch back
 size_t vol_floats(const Plan *p);
 size_t sin_floats(const Plan *p);
 
+// A projection's turn at its plan's scratch (FP16 operands, the volume's column-major
+// copy, partial sums).  Eager calls wait for the last one's on the device; a captured
+// call takes none.  Held from begin to the end of the object's life.
+class Turn {
+  public:
+    int begin(const Plan *plan, int direction, cudaStream_t stream);
+    ~Turn();
+    Turn() = default;
+    Turn(const Turn &) = delete;
+    Turn &operator=(const Turn &) = delete;
+
+  private:
+    const Plan *p = nullptr;
+    int dir = 0;
+    cudaStream_t st = nullptr;
+};
+
 // Operators (arec_project.cu); fp32: on the FP32 kernels in any case
 int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2,
                     const int *d_skip, cudaStream_t st, bool fp32 = false);
 int back_project(const Plan *p, const float *d_s, float *d_g, double *d_norm2,
                  const int *d_skip, cudaStream_t st, bool fp32 = false);
+constexpr int kNormBlocks = 1024;  // partial sums of a norm
 int fp_grid_blocks(const Plan *p);
 int plan_timing(const Plan *p, int mode, double *fp_ms, long long *fp_calls, double *bp_ms,
                 long long *bp_calls);

@@ -39,8 +39,6 @@ static int slice_blocks(const Plan *p) {
     return (p->ys + span - 1) / span;
 }
 
-constexpr int kNormBlocks = 1024;
-
 // Forward projection (banded kernels): floats per lane.
 static int fp_vec(const Plan *p) { return p->fp_vec ? p->fp_vec : p->vec; }
 
@@ -113,12 +111,31 @@ __global__ void __launch_bounds__(256) k_zero_unless(float4 *q, size_t n4, const
         q[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
+int Turn::begin(const Plan *plan, int direction, cudaStream_t stream) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    ARECGB_CUDA(cudaStreamIsCapturing(stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return 0;
+    plan->turn_lock[direction].lock();
+    p = plan, dir = direction, st = stream;
+    ARECGB_CUDA(cudaStreamWaitEvent(st, p->turn_ev[dir], 0));
+    return 0;
+}
+
+Turn::~Turn() {
+    if (!p) return;
+    cudaEventRecord(p->turn_ev[dir], st);
+    p->turn_lock[dir].unlock();
+}
+
 int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2,
                     const int *d_skip, cudaStream_t st, bool fp32) {
     const bool mma = p->mma && !fp32;
     const OpArgs A = make_args(p, d_skip);
     const size_t nq = sin_floats(p);
-    int rc = timing_mark(p, true, false, st);
+    Turn turn;
+    int rc = 0;
+    if (mma || d_norm2 || (A.taps && p->ngroups_o[1])) rc = turn.begin(p, 0, st);
+    if (!rc) rc = timing_mark(p, true, false, st);
     if (rc) return rc;
     if (p->weighting == ARECGB_LIN) {
         ARECGB_CUDA(cudaMemsetAsync(d_q, 0, sizeof(float) * nq, st));
@@ -186,17 +203,21 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
 
 int back_project(const Plan *p, const float *d_s, float *d_g, double *d_norm2,
                  const int *d_skip, cudaStream_t st, bool fp32) {
+    Turn turn;
+    if ((p->mma && !fp32) || d_norm2)
+        if (int rc = turn.begin(p, 1, st)) return rc;
     if (p->mma && !fp32) {
         int rc = timing_mark(p, false, false, st);
         if (!rc) rc = back_project_mma(p, d_s, d_g, d_skip, st);
         if (!rc && d_norm2) {
-            rc = sumsq_partials(d_g, vol_floats(p), p->d_partials, kNormBlocks, st);
-            if (!rc) rc = reduce_partials(p->d_partials, kNormBlocks, d_norm2, st);
+            rc = sumsq_partials(d_g, vol_floats(p), p->d_bp_partials, kNormBlocks, st);
+            if (!rc) rc = reduce_partials(p->d_bp_partials, kNormBlocks, d_norm2, st);
             count_launches(2);
         }
         return rc ? rc : timing_mark(p, false, true, st);
     }
-    const OpArgs A = make_args(p, d_skip);
+    OpArgs A = make_args(p, d_skip);
+    if (!d_norm2) A.partials = nullptr;
     const int nsc = slice_chunks(p);
     dim3 grid(p->ntiles, slice_blocks(p));
     // the footprint of an angle as one TMA tile (kBpFoot bins x the block's slices,
@@ -222,7 +243,7 @@ int back_project(const Plan *p, const float *d_s, float *d_g, double *d_norm2,
     ARECGB_CUDA(cudaGetLastError());
     if (rc) return ARECGB_ERR_ARG;
     if (d_norm2) {
-        rc = reduce_partials(p->d_partials, grid.x * grid.y, d_norm2, st);
+        rc = reduce_partials(p->d_bp_partials, grid.x * grid.y, d_norm2, st);
         if (rc) return rc;
     }
     return timing_mark(p, false, true, st);

@@ -53,7 +53,7 @@ inline OpArgs make_args(const Plan *p, const int *skip) {
     A.ngroups = p->ngroups;
     A.r_hi = p->r_hi;
     A.r_lo = p->r_lo;
-    A.partials = p->d_partials;
+    A.partials = p->d_bp_partials;
     A.skip = skip;
     A.err = p->d_err;
     A.taps = p->d_taps;

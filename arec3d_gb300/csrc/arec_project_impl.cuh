@@ -579,7 +579,8 @@ __device__ __forceinline__ bool bp_block(const OpArgs &A, const float *__restric
             for (int q = 0; q < VEC; q++) s2 += (double)__fmul_rn(acc[r][q], acc[r][q]);
         }
     }
-    if constexpr (!AGAIN) block_sum_to<NCW>(s2, red, A.partials + (size_t)by * gridDim.x + bx);
+    if constexpr (!AGAIN)
+        if (A.partials) block_sum_to<NCW>(s2, red, A.partials + (size_t)by * gridDim.x + bx);
     return ok;
 }
 
@@ -691,7 +692,7 @@ __global__ void __launch_bounds__(128 * NSC)
             for (int q = 0; q < VEC; q++) s2 += (double)__fmul_rn(acc[r][q], acc[r][q]);
         }
     }
-    block_sum_to<NWARP>(s2, red, A.partials + (size_t)blockIdx.y * gridDim.x + blockIdx.x);
+    if (A.partials) block_sum_to<NWARP>(s2, red, A.partials + (size_t)blockIdx.y * gridDim.x + blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------

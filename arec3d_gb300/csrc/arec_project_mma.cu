@@ -1126,7 +1126,6 @@ int mma_plan_create(Plan *p, const std::vector<int4> &g4, const std::vector<Angl
             mma_plan_destroy(p);
             return 0;
         }
-        ARECGB_CUDA(cudaEventCreateWithFlags(&p->half_ev[d], cudaEventDisableTiming));
     }
     ARECGB_CUDA(cudaMemsetAsync(p->d_half[0], 0, bytes[0], p->stream));
     ARECGB_CUDA(cudaStreamSynchronize(p->stream));
@@ -1162,8 +1161,6 @@ void mma_plan_destroy(Plan *p) {
     for (int d = 0; d < 2; d++) {
         drop(p->d_half[d]);
         drop(p->d_smax[d]);
-        if (p->half_ev[d]) cudaEventDestroy(p->half_ev[d]);
-        p->half_ev[d] = nullptr;
     }
     p->mma = 0;
 }
@@ -1176,9 +1173,9 @@ static MmaPlan make_plan(const Plan *p) {
 namespace {
 
 // The operands of one projection (dir 0 forward, 1 back) on stream st.  An eager
-// call takes the plan's, after the last call that did; a captured one gets its own
-// from the graph (its replays are ordered with nothing else), except within a
-// solver (d_skip), which launches its graph under MmaHold.
+// call takes the plan's, in its turn; a captured one gets its own from the graph (its
+// replays are ordered with nothing else), except within a solver (d_skip), which
+// launches its graph under MmaHold.
 struct Work {
     void *half = nullptr;
     unsigned *smax = nullptr;
@@ -1186,14 +1183,13 @@ struct Work {
     const Plan *p = nullptr;
     int dir = 0;
     cudaStream_t st = nullptr;
-    bool eager = false, own = false;
+    bool own = false;
 
     int begin(const Plan *plan, int d, const int *d_skip, cudaStream_t stream) {
         p = plan, dir = d, st = stream;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         ARECGB_CUDA(cudaStreamIsCapturing(st, &cap));
-        eager = cap == cudaStreamCaptureStatusNone;
-        own = !eager && !d_skip;
+        own = cap != cudaStreamCaptureStatusNone && !d_skip;
         half = p->d_half[dir];
         smax = p->d_smax[dir];
         if (own) {
@@ -1202,14 +1198,6 @@ struct Work {
             ARECGB_CUDA(cudaMallocAsync((void **)&smax, mma_stats_bytes(p->ys), st));
             if (dir == 0) ARECGB_CUDA(cudaMemsetAsync(half, 0, bytes, st));
         }
-        if (eager) {
-            p->half_lock[dir].lock();
-            const cudaError_t e = cudaStreamWaitEvent(st, p->half_ev[dir], 0);
-            if (e != cudaSuccess) {
-                p->half_lock[dir].unlock();
-                ARECGB_CUDA(e);
-            }
-        }
         stats = {smax, (unsigned long long *)(smax + p->ys), (int *)(smax + 3 * p->ys), p->ys};
         return 0;
     }
@@ -1217,11 +1205,6 @@ struct Work {
         if (own) {
             ARECGB_CUDA(cudaFreeAsync(half, st));
             ARECGB_CUDA(cudaFreeAsync(smax, st));
-        }
-        if (eager) {
-            const cudaError_t e = cudaEventRecord(p->half_ev[dir], st);
-            p->half_lock[dir].unlock();
-            ARECGB_CUDA(e);
         }
         return 0;
     }
@@ -1371,16 +1354,16 @@ MmaHold::MmaHold(Plan *const *plans, int n, cudaStream_t s) : st(s) {
     std::sort(held.begin(), held.end());  // one order for all holders
     for (Plan *p : held)
         for (int d = 0; d < 2; d++) {
-            p->half_lock[d].lock();
-            cudaStreamWaitEvent(st, p->half_ev[d], 0);
+            p->turn_lock[d].lock();
+            cudaStreamWaitEvent(st, p->turn_ev[d], 0);
         }
 }
 
 MmaHold::~MmaHold() {
     for (Plan *p : held)
         for (int d = 0; d < 2; d++) {
-            cudaEventRecord(p->half_ev[d], st);
-            p->half_lock[d].unlock();
+            cudaEventRecord(p->turn_ev[d], st);
+            p->turn_lock[d].unlock();
         }
 }
 

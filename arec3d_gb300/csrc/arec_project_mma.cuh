@@ -66,9 +66,8 @@ int forward_project_mma(const Plan *p, const float *d_x, float *d_q, const int *
                         cudaStream_t st);
 int back_project_mma(const Plan *p, const float *d_s, float *d_g, const int *d_skip, cudaStream_t st);
 
-// A plan's FP16 operands serve one forward and one back projection at a time:
-// eager calls on other streams or threads wait for the last one's (on the device).
-// Held around launches of graphs whose projections use them.
+// A plan's turns in both directions, held around launches of graphs whose projections
+// use its operands.
 class MmaHold {
   public:
     MmaHold(Plan *const *plans, int n, cudaStream_t st);
