@@ -68,7 +68,8 @@ static int choose_vec(int ys) {
 
 int plan_create(Plan **out, int weighting, double radius, int ny, int nangles,
                 const float *angles_host, bool tables) {
-    scratch_trim();  // the alignment's scratch, before memory is measured below
+    scratch_trim();  // scratch that nothing uses, before memory is measured below
+    graph_memory_trim();
     *out = nullptr;
     if (weighting < ARECGB_LIN || weighting > ARECGB_SQ) {
         set_error("plan_create: weighting must be 1 (LIN), 2 (KB) or 3 (SQ)");
@@ -283,6 +284,7 @@ void plan_destroy(Plan *p) {
     cudaGetDevice(&cur);
     if (cur != p->device) cudaSetDevice(p->device);
     if (p->stream) cudaStreamSynchronize(p->stream);
+    graph_memory_trim();
     cudaFree(p->d_ray);
     cudaFree(p->d_ang);
     cudaFree(p->d_rows);

@@ -94,6 +94,14 @@ struct Plan {
     // projection, and their HalfStats
     void *d_half[2] = {nullptr, nullptr};
     unsigned *d_smax[2] = {nullptr, nullptr};
+    // the last captured call's operand in either direction (mma_operand)
+    struct GraphOperand {
+        unsigned long long capture = 0;
+        cudaStream_t stream = nullptr;
+        void *ptr = nullptr;
+    };
+    mutable GraphOperand graph_op[2];
+    mutable std::mutex graph_lock;
     // scratch of a projection in either direction (Turn): the end of the last call
     // that used it, and the call that is being launched
     cudaEvent_t turn_ev[2] = {nullptr, nullptr};
@@ -164,6 +172,7 @@ int plan_create(Plan **out, int weighting, double radius, int ny, int nangles,
                 const float *angles_host, bool tables = true);
 void plan_destroy(Plan *p);
 void scratch_trim();  // arec_ccorr.cu: gives unused alignment scratch back
+void graph_memory_trim();  // arec_project_mma.cu: and what graphs that are gone held
 size_t vol_floats(const Plan *p);
 size_t sin_floats(const Plan *p);
 

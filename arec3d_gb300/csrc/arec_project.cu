@@ -129,7 +129,12 @@ Turn::~Turn() {
 
 int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2,
                     const int *d_skip, cudaStream_t st, bool fp32) {
-    const bool mma = p->mma && !fp32;
+    bool mma = p->mma && !fp32;
+    MmaOperand op;
+    if (mma) {
+        if (int rc = mma_operand(p, 0, d_skip, st, &op)) return rc;
+        mma = op.half != nullptr;
+    }
     const OpArgs A = make_args(p, d_skip);
     const size_t nq = sin_floats(p);
     Turn turn;
@@ -144,7 +149,7 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
     } else {
         // zero q, then each (orientation, line band) launch adds its part
         if (mma) {
-            rc = forward_project_mma(p, d_x, d_q, d_skip, st);
+            rc = forward_project_mma(p, op, d_x, d_q, d_skip, st);
             if (rc) return rc;
         } else {
             k_zero_unless<<<(unsigned)std::min<size_t>(152 * 8, (nq / 4 + 255) / 256), 256, 0, st>>>(
@@ -203,12 +208,18 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
 
 int back_project(const Plan *p, const float *d_s, float *d_g, double *d_norm2,
                  const int *d_skip, cudaStream_t st, bool fp32) {
+    bool mma = p->mma && !fp32;
+    MmaOperand op;
+    if (mma) {
+        if (int rc = mma_operand(p, 1, d_skip, st, &op)) return rc;
+        mma = op.half != nullptr;
+    }
     Turn turn;
-    if ((p->mma && !fp32) || d_norm2)
+    if (mma || d_norm2)
         if (int rc = turn.begin(p, 1, st)) return rc;
-    if (p->mma && !fp32) {
+    if (mma) {
         int rc = timing_mark(p, false, false, st);
-        if (!rc) rc = back_project_mma(p, d_s, d_g, d_skip, st);
+        if (!rc) rc = back_project_mma(p, op, d_s, d_g, d_skip, st);
         if (!rc && d_norm2) {
             rc = sumsq_partials(d_g, vol_floats(p), p->d_bp_partials, kNormBlocks, st);
             if (!rc) rc = reduce_partials(p->d_bp_partials, kNormBlocks, d_norm2, st);

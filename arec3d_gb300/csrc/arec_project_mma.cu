@@ -1172,41 +1172,18 @@ static MmaPlan make_plan(const Plan *p) {
 
 namespace {
 
-// The operands of one projection (dir 0 forward, 1 back) on stream st.  An eager
-// call takes the plan's, in its turn; a captured one gets its own from the graph (its
-// replays are ordered with nothing else), except within a solver (d_skip), which
-// launches its graph under MmaHold.
+// One projection (dir 0 forward, 1 back) on stream st and its operand.
 struct Work {
-    void *half = nullptr;
-    unsigned *smax = nullptr;
-    HalfStats stats{};
-    const Plan *p = nullptr;
-    int dir = 0;
-    cudaStream_t st = nullptr;
-    bool own = false;
+    const Plan *p;
+    int dir;
+    cudaStream_t st;
+    void *half;
+    unsigned *smax;
+    HalfStats stats;
 
-    int begin(const Plan *plan, int d, const int *d_skip, cudaStream_t stream) {
-        p = plan, dir = d, st = stream;
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        ARECGB_CUDA(cudaStreamIsCapturing(st, &cap));
-        own = cap != cudaStreamCaptureStatusNone && !d_skip;
-        half = p->d_half[dir];
-        smax = p->d_smax[dir];
-        if (own) {
-            const size_t bytes = sizeof(float) * (dir ? sin_floats(p) : (size_t)p->nx * p->nx * p->ys);
-            ARECGB_CUDA(cudaMallocAsync(&half, bytes, st));
-            ARECGB_CUDA(cudaMallocAsync((void **)&smax, mma_stats_bytes(p->ys), st));
-            if (dir == 0) ARECGB_CUDA(cudaMemsetAsync(half, 0, bytes, st));
-        }
+    Work(const Plan *plan, int d, const MmaOperand &op, cudaStream_t stream)
+        : p(plan), dir(d), st(stream), half(op.half), smax(op.stats) {
         stats = {smax, (unsigned long long *)(smax + p->ys), (int *)(smax + 3 * p->ys), p->ys};
-        return 0;
-    }
-    int end() {
-        if (own) {
-            ARECGB_CUDA(cudaFreeAsync(half, st));
-            ARECGB_CUDA(cudaFreeAsync(smax, st));
-        }
-        return 0;
     }
 };
 
@@ -1332,20 +1309,109 @@ int bp_steps(const Work &w, const OpArgs &A, const float *d_s, float *d_g) {
 }  // namespace
 
 // q = A x.
-int forward_project_mma(const Plan *p, const float *d_x, float *d_q, const int *d_skip,
-                        cudaStream_t st) {
-    Work w;
-    if (int rc = w.begin(p, 0, d_skip, st)) return rc;
-    const int rc = fp_steps(w, make_args(p, d_skip), d_x, d_q), rc2 = w.end();
-    return rc ? rc : rc2;
+int forward_project_mma(const Plan *p, const MmaOperand &op, const float *d_x, float *d_q,
+                        const int *d_skip, cudaStream_t st) {
+    return fp_steps(Work(p, 0, op, st), make_args(p, d_skip), d_x, d_q);
 }
 
 // g = A^T s.
-int back_project_mma(const Plan *p, const float *d_s, float *d_g, const int *d_skip, cudaStream_t st) {
-    Work w;
-    if (int rc = w.begin(p, 1, d_skip, st)) return rc;
-    const int rc = bp_steps(w, make_args(p, d_skip), d_s, d_g), rc2 = w.end();
-    return rc ? rc : rc2;
+int back_project_mma(const Plan *p, const MmaOperand &op, const float *d_s, float *d_g,
+                     const int *d_skip, cudaStream_t st) {
+    return bp_steps(Work(p, 1, op, st), make_args(p, d_skip), d_s, d_g);
+}
+
+// ---------------------------------------------------------------------------
+// Operands of captured calls.  A graph's replays are ordered with nothing else, so it
+// has memory of its own, which lives as long as it, its clones and its instances (a
+// user object they hold).  Allocation nodes would do that too, but not in a graph that
+// is cloned, a child of another or instantiated twice.  Calls captured on one stream
+// follow one another and share it.
+namespace {
+
+struct GraphMemory {
+    int device = 0;
+    void *ptr = nullptr;
+    size_t bytes = 0;
+};
+std::mutex g_graph_mu;
+std::vector<GraphMemory> g_graph_free;  // of graphs that are gone
+
+// May not call into CUDA: the memory is taken again, or freed by graph_memory_trim.
+void graph_memory_drop(void *m) {
+    std::lock_guard<std::mutex> lk(g_graph_mu);
+    g_graph_free.push_back(*static_cast<GraphMemory *>(m));
+    delete static_cast<GraphMemory *>(m);
+}
+
+// `bytes` held by `graph`, or null.
+void *graph_memory(cudaGraph_t graph, size_t bytes) {
+    GraphMemory *m = new GraphMemory;
+    if (cudaGetDevice(&m->device) == cudaSuccess) {
+        std::lock_guard<std::mutex> lk(g_graph_mu);
+        for (size_t i = 0; i < g_graph_free.size() && !m->ptr; i++)
+            if (g_graph_free[i].device == m->device && g_graph_free[i].bytes == bytes) {
+                *m = g_graph_free[i];
+                g_graph_free.erase(g_graph_free.begin() + i);
+            }
+    }
+    if (!m->ptr) {
+        m->bytes = bytes;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // this capture is no bar
+        const bool relaxed = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+        if (!relaxed || cudaMalloc(&m->ptr, bytes) != cudaSuccess) m->ptr = nullptr;
+        if (relaxed) cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    cudaUserObject_t obj = nullptr;
+    if (!m->ptr) {
+        delete m;
+    } else if (cudaUserObjectCreate(&obj, m, graph_memory_drop, 1, cudaUserObjectNoDestructorSync) !=
+               cudaSuccess) {
+        graph_memory_drop(m);
+    } else {
+        void *ptr = m->ptr;
+        if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) == cudaSuccess) return ptr;
+        cudaUserObjectRelease(obj, 1);
+    }
+    cudaGetLastError();  // not sticky
+    return nullptr;
+}
+
+}  // namespace
+
+void graph_memory_trim() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    std::lock_guard<std::mutex> lk(g_graph_mu);
+    for (size_t i = g_graph_free.size(); i-- > 0;)
+        if (g_graph_free[i].device == dev) {
+            cudaFree(g_graph_free[i].ptr);
+            g_graph_free.erase(g_graph_free.begin() + i);
+        }
+}
+
+int mma_operand(const Plan *p, int dir, const int *d_skip, cudaStream_t st, MmaOperand *op) {
+    *op = {p->d_half[dir], p->d_smax[dir]};
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    cudaGraph_t graph = nullptr;
+    ARECGB_CUDA(cudaStreamGetCaptureInfo(st, &cap, &id, &graph));
+    if (cap == cudaStreamCaptureStatusNone || d_skip) return 0;  // eager, or a solver's (MmaHold)
+    std::lock_guard<std::mutex> lk(p->graph_lock);
+    const size_t half = sizeof(float) * (dir ? sin_floats(p) : (size_t)p->nx * p->nx * p->ys);
+    Plan::GraphOperand &g = p->graph_op[dir];
+    if (g.capture != id || g.stream != st || !g.ptr) {
+        g.ptr = graph_memory(graph, half + mma_stats_bytes(p->ys));
+        g.capture = id;
+        g.stream = st;
+        if (!g.ptr) {
+            *op = {};
+            return 0;
+        }
+        // pixels outside the disk are read and never written
+        if (dir == 0) ARECGB_CUDA(cudaMemsetAsync(g.ptr, 0, half, st));
+    }
+    *op = {g.ptr, (unsigned *)((char *)g.ptr + half)};
+    return 0;
 }
 
 MmaHold::MmaHold(Plan *const *plans, int n, cudaStream_t s) : st(s) {

@@ -62,9 +62,19 @@ int mma_plan_create(Plan *p, const std::vector<int4> &groups4,
 struct OpArgs;
 int mma_build_taps(Plan *p, const OpArgs &A);
 void mma_plan_destroy(Plan *p);
-int forward_project_mma(const Plan *p, const float *d_x, float *d_q, const int *d_skip,
-                        cudaStream_t st);
-int back_project_mma(const Plan *p, const float *d_s, float *d_g, const int *d_skip, cudaStream_t st);
+// Memory of one projection: its operand as FP16 pairs and what HalfStats holds.
+struct MmaOperand {
+    void *half = nullptr;
+    unsigned *stats = nullptr;
+};
+// The operand of a projection (dir 0 forward, 1 back) on stream st: the plan's, or in a
+// capture (but a solver's: d_skip) one that the graph holds; half null when there is no
+// memory for that, and the call takes the FP32 kernels.
+int mma_operand(const Plan *p, int dir, const int *d_skip, cudaStream_t st, MmaOperand *op);
+int forward_project_mma(const Plan *p, const MmaOperand &op, const float *d_x, float *d_q,
+                        const int *d_skip, cudaStream_t st);
+int back_project_mma(const Plan *p, const MmaOperand &op, const float *d_s, float *d_g,
+                     const int *d_skip, cudaStream_t st);
 
 // A plan's turns in both directions, held around launches of graphs whose projections
 // use its operands.
