@@ -824,23 +824,6 @@ struct Scratch {
     }
 };
 
-static std::mutex g_smem_mu;
-static std::map<std::pair<int, const void *>, size_t> g_smem;  // (device, kernel) -> limit set
-
-// Raises a kernel's dynamic shared-memory limit to at least `bytes` and never
-// lowers it: the limit is process-wide, so a caller on another host thread
-// with smaller images cannot drop it between this caller's set and launch.
-static int set_smem(const void *fn, size_t bytes) {
-    int dev = 0;
-    ARECGB_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lk(g_smem_mu);
-    size_t &cur = g_smem[{dev, fn}];
-    if (bytes <= cur) return 0;
-    ARECGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    cur = bytes;
-    return 0;
-}
-
 // Calls f with the length as a compile-time constant (0: not a power of two
 // from 16).
 template <typename F>

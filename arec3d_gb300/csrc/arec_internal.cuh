@@ -171,6 +171,9 @@ constexpr int kFpBins = 8;             // detector bins per forward-projection b
 int plan_create(Plan **out, int weighting, double radius, int ny, int nangles,
                 const float *angles_host, bool tables = true);
 void plan_destroy(Plan *p);
+// Dynamic shared memory a kernel may use on the current device: at least `bytes` from
+// now on (arec_project.cu).
+int set_smem(const void *kernel, size_t bytes);
 void scratch_trim();  // arec_ccorr.cu: gives unused alignment scratch back
 void graph_memory_trim();  // arec_project_mma.cu: and what graphs that are gone held
 size_t vol_floats(const Plan *p);

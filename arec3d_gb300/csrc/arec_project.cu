@@ -3,6 +3,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "arec_limits.h"
 #include "arec_project_impl.cuh"
 #include "arec_project_mma.cuh"
 
@@ -109,6 +110,16 @@ __global__ void __launch_bounds__(256) k_zero_unless(float4 *q, size_t n4, const
     if (skip && *skip) return;
     for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256)
         q[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+int set_smem(const void *kernel, size_t bytes) {
+    static RaisedLimits limits;
+    int dev = 0;
+    ARECGB_CUDA(cudaGetDevice(&dev));
+    return limits.raise(dev, kernel, bytes, [&](size_t n) -> int {
+        ARECGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n));
+        return 0;
+    });
 }
 
 int Turn::begin(const Plan *plan, int direction, cudaStream_t stream) {

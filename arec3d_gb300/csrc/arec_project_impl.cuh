@@ -1371,13 +1371,7 @@ int launch_bp_one(const OpArgs &A, dim3 grid, const float *s, float *g, const CU
         bp_lin_kernel<V, N><<<grid, 128 * N, 0, st>>>(A, s, g);
     } else {
         constexpr size_t smem = bp_smem_bytes<V, N>();
-        static bool configured = false;  // per instantiation, once per process
-        if (!configured) {
-            if (cudaFuncSetAttribute(bp_kernel<W, V, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem) != cudaSuccess)
-                return -2;
-            configured = true;
-        }
+        if (set_smem((const void *)bp_kernel<W, V, N>, smem)) return -2;
         bp_kernel<W, V, N><<<grid, 128 * N, smem, st>>>(A, s, g, tms, use_tma);
     }
     return 0;
@@ -1422,13 +1416,7 @@ template <int W, int V, int BT>
 int launch_fpb_one(const OpArgs &A, dim3 grid, const float *x, float *q, int g0, int ngo, int lo,
                    int hi, const CUtensorMap &tmx, const CUtensorMap &tmxT, cudaStream_t st) {
     constexpr size_t smem = fpb_smem_bytes<V>();
-    static bool configured = false;  // per instantiation, once per process
-    if (!configured) {
-        if (cudaFuncSetAttribute(fp_band_kernel<W, V, BT>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return -2;
-        configured = true;
-    }
+    if (set_smem((const void *)fp_band_kernel<W, V, BT>, smem)) return -2;
     fp_band_kernel<W, V, BT><<<grid, kFpThreads, smem, st>>>(A, x, q, g0, ngo, lo, hi, tmx, tmxT);
     return 0;
 }
@@ -1447,15 +1435,9 @@ template <int W, int V>
 int launch_wide_one(const OpArgs &A, int ntiles, int ngo0, int band, const float *in, float *out, bool back,
                     const WideArgs &w, cudaStream_t st) {
     constexpr size_t smem = bp_smem_bytes<V, 1>(), fsmem = fpb_smem_bytes<V>();
-    static bool configured = false;  // per instantiation, once per process
-    if (!configured) {
-        if (cudaFuncSetAttribute(bp_wide_kernel<W, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem) != cudaSuccess ||
-            cudaFuncSetAttribute(fp_wide_kernel<W, V, kFpBins>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)fsmem) != cudaSuccess)
-            return -2;
-        configured = true;
-    }
+    if (set_smem(back ? (const void *)bp_wide_kernel<W, V> : (const void *)fp_wide_kernel<W, V, kFpBins>,
+                 back ? smem : fsmem))
+        return -2;
     const int slices = (A.ys + 32 * V - 1) / (32 * V);
     if (back) {
         CUtensorMap tms;

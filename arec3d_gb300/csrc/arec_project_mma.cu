@@ -1206,13 +1206,7 @@ size_t score_bytes(int ys) { return ys <= kScoreShared ? sizeof(int) * ys : 0; }
 
 template <int W, int MT>
 int launch_fp_mma(const Work &w, const OpArgs &A, const MmaPlan &M, const CUtensorMap &tx, float *q) {
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(fp_mma_kernel<W, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    FpMma<MT>::SMEM);
-    });
-    ARECGB_CUDA(attr);
+    if (int rc = set_smem((const void *)fp_mma_kernel<W, MT>, FpMma<MT>::SMEM)) return rc;
     const dim3 grid(M.ngroups * ((M.max_strips + 2) / 3), (A.ys + 128 * MT - 1) / (128 * MT));
     for (int seg = 0; seg < M.max_segs; seg++)
         for (int color = 0; color < 3; color++)
@@ -1267,13 +1261,7 @@ int fp_steps(const Work &w, const OpArgs &A, const float *d_x, float *d_q) {
 
 template <int W>
 int launch_bp_mma(const Work &w, const OpArgs &A, const CUtensorMap &ts, float *g, bool halves) {
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(bp_mma_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)BpMma::smem(BpMma::MAX_NA));
-    });
-    ARECGB_CUDA(attr);
+    if (int rc = set_smem((const void *)bp_mma_kernel<W>, BpMma::smem(BpMma::MAX_NA))) return rc;
     bp_mma_kernel<W><<<dim3(w.p->m_tiles, (A.ys + 127) / 128, halves ? 2 : 1), kMmaThreads,
                        BpMma::smem(A.na), w.st>>>(
         A, make_plan(w.p), ts, g, w.smax, w.stats.wide);

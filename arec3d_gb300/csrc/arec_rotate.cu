@@ -505,7 +505,7 @@ int rot_cc_angles(const float *d1, const float *d2, int nz, int ny, int nx, int 
     }
     ARECGB_CUDA(cudaGetLastError());
     const size_t smem = sizeof(float) * 4 * (size_t)n;
-    ARECGB_CUDA(cudaFuncSetAttribute(k_rot_peak, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = set_smem((const void *)k_rot_peak, smem)) return rc;
     k_rot_peak<<<nz, kPeakThreads, smem, st>>>(prof, nz, n, d_angles);
     count_launches(1);
     ARECGB_CUDA(cudaGetLastError());
@@ -536,8 +536,7 @@ int profile_shifts(const float *d_prof, int prof_y, int prof_x, int pad, int suc
         count_launches(1);
     }
     const size_t smem = sizeof(float) * 4 * (size_t)L;
-    ARECGB_CUDA(cudaFuncSetAttribute(k_profile_peak, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
+    if (int rc = set_smem((const void *)k_profile_peak, smem)) return rc;
     k_profile_peak<<<prof_y, kPeakThreads, smem, st>>>(d_prof, prof_x, pad, L,
                                                       successive ? nullptr : d_mean, d_out);
     count_launches(1);

@@ -163,12 +163,7 @@ static int launch_conv(const __nv_bfloat16 *X, const __nv_bfloat16 *Wt, const fl
                        __nv_bfloat16 *Y, int H, int Wd, int Cin, int P, int relu, int ystride,
                        int *err, cudaStream_t st) {
     using Cfg = ConvCfg<COUT>;
-    static bool configured = false;
-    if (!configured) {
-        ARECGB_CUDA(cudaFuncSetAttribute(conv3x3_umma_kernel<COUT, LBO, SBO>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
-        configured = true;
-    }
+    if (int rc = set_smem((const void *)conv3x3_umma_kernel<COUT, LBO, SBO>, Cfg::SMEM)) return rc;
     conv3x3_umma_kernel<COUT, LBO, SBO><<<(P + 127) / 128, 128, Cfg::SMEM, st>>>(
         X, Wt, bias, Y, H, Wd, Cin, P, relu, ystride, err);
     ARECGB_CUDA(cudaGetLastError());
@@ -574,13 +569,7 @@ static int launch_conv_pipe(const __nv_bfloat16 *x, const __nv_bfloat16 *w, cons
     if (!conv_tensor_maps(x, w, y, N, H, Wd, Cin, COUT, ystride, 1 << lw, BAND ? R + 2 : hb, KC,
                           &m))
         return -1;
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(conv3x3_pipe_kernel<COUT, R, BAND, KC, ST>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
-    });
-    ARECGB_CUDA(attr);
+    if (int rc = set_smem((const void *)conv3x3_pipe_kernel<COUT, R, BAND, KC, ST>, Cfg::SMEM)) return rc;
     const int wt = (Wd + (1 << lw) - 1) >> lw, ht = (H + hb - 1) / hb, ntiles = N * wt * ht;
     const int sms = sm_count();
     conv3x3_pipe_kernel<COUT, R, BAND, KC, ST><<<ntiles < sms ? ntiles : sms, kPipeThreads, Cfg::SMEM, st>>>(

@@ -34,7 +34,6 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "arec_internal.cuh"
 #include "arec_umma.cuh"
@@ -251,13 +250,7 @@ Operand make_operand(int blocks, int rows) {
 template <int NDY, int TILES>
 int launch_wgrad(const CUtensorMap &tx, const CUtensorMap &td, float *gw, int Cin, const WgradJob &J,
                  int *err, cudaStream_t st) {
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(k_wgrad_mma<NDY, TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kSmemStages + kSlack + 1024);
-    });
-    ARECGB_CUDA(attr);
+    if (int rc = set_smem((const void *)k_wgrad_mma<NDY, TILES>, kSmemStages + kSlack + 1024)) return rc;
     const int jobs = J.ci_jobs * J.co_jobs * (3 / NDY);
     const int splits = std::max(1, std::min(J.chunks, 152 / jobs));
     k_wgrad_mma<NDY, TILES><<<dim3(splits, jobs), kWgThreads, J.stages * J.stage + kSlack + 1024, st>>>(
