@@ -55,7 +55,7 @@ struct MmaPlan {
 int mma_takes(int weighting, int nx, int ys, int na);
 // spare: leave the plan to the FP32 kernels (p->mma = 0) when the operands would
 // take more than 40 % of the free memory.  It is left to them in any case when
-// they cannot be allocated.
+// they cannot be allocated or would leave no room for a solve.
 int mma_plan_create(Plan *p, const std::vector<int4> &groups4,
                     const std::vector<AngleParams> &ang, const std::vector<RowInfo> &rows,
                     const std::vector<ColInfo> &cols, bool spare);

@@ -66,7 +66,8 @@ int arecgb_version(void);
  * Allocates device tables on the current device, and for square-pixel and
  * Kaiser-Bessel plans of more than a few angles and slices (those whose projections
  * run on the tensor cores; with fewer than 48 slices CGLS keeps to FP32 kernels) room for one volume (of all nx nx pixels) and one sinogram as FP16 pairs,
- * unless that takes more than 40 % of the free memory (the FP32 projectors then).
+ * unless that takes more than 40 % of the free memory or leaves no room for a solve's
+ * workspace (the FP32 projectors then).
  * The first call captured into a graph on a stream allocates this room again, for the
  * graph, its clones and instances (freed with a later plan_create or plan_destroy once
  * they are gone; FP32 projectors if it does not fit). */
