@@ -385,7 +385,7 @@ int cached_plan(Plan **out, int w, double radius, int ny, int na, const float *a
 
 int ensure(float **buf, size_t n) {
     if (*buf) return 0;
-    ARECGB_CUDA(cudaMalloc(buf, sizeof(float) * std::max<size_t>(n, 1)));
+    ARECGB_CUDA(arecgb::dev_malloc(buf, sizeof(float) * std::max<size_t>(n, 1)));
     ARECGB_CUDA(cudaMemset(*buf, 0, sizeof(float) * std::max<size_t>(n, 1)));
     return 0;
 }
@@ -395,7 +395,7 @@ int ensure_stage(Plan *p, size_t n) {
     cudaFree(p->d_stage);
     p->d_stage = nullptr;
     p->stage_floats = 0;
-    ARECGB_CUDA(cudaMalloc(&p->d_stage, sizeof(float) * std::max<size_t>(n, 1)));
+    ARECGB_CUDA(arecgb::dev_malloc(&p->d_stage, sizeof(float) * std::max<size_t>(n, 1)));
     p->stage_floats = n;
     return 0;
 }
@@ -709,7 +709,7 @@ int arecgb_reconstruct_host(arecgb_plan *plan, const float *b_host, float *x_hos
                 v = nullptr;
             }
             p->img_floats = 0;
-            for (auto &v : p->d_img) ARECGB_CUDA(cudaMalloc(&v, sizeof(float) * n));
+            for (auto &v : p->d_img) ARECGB_CUDA(arecgb::dev_malloc(&v, sizeof(float) * n));
             p->img_floats = n;
         }
     }
@@ -939,9 +939,9 @@ int arecgb_arecCCImages(MPI_Comm, arecImage i1, arecImage i2, float *sx, float *
     cudaStream_t st = nullptr;
     int rc = 0;
     cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&d1, sizeof(float) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&d2, sizeof(float) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&dsx, sizeof(float) * 2 * nz);
+    if (e == cudaSuccess) e = arecgb::dev_malloc(&d1, sizeof(float) * n);
+    if (e == cudaSuccess) e = arecgb::dev_malloc(&d2, sizeof(float) * n);
+    if (e == cudaSuccess) e = arecgb::dev_malloc(&dsx, sizeof(float) * 2 * nz);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d1, i1.data, sizeof(float) * n, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d2, i2.data, sizeof(float) * n, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) {
@@ -981,9 +981,9 @@ static int rot_host(const char *who, int kind, const arecImage &a, const arecIma
     cudaStream_t st = nullptr;
     int rc = 0;
     cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&d1, sizeof(float) * n);
-    if (e == cudaSuccess && two) e = cudaMalloc(&d2, sizeof(float) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&da, sizeof(float) * nz);
+    if (e == cudaSuccess) e = arecgb::dev_malloc(&d1, sizeof(float) * n);
+    if (e == cudaSuccess && two) e = arecgb::dev_malloc(&d2, sizeof(float) * n);
+    if (e == cudaSuccess) e = arecgb::dev_malloc(&da, sizeof(float) * nz);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d1, a.data, sizeof(float) * n, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && two)
         e = cudaMemcpyAsync(d2, b->data, sizeof(float) * n, cudaMemcpyHostToDevice, st);
@@ -1067,7 +1067,7 @@ static int pre_host(const char *who, int kind, float *data, size_t n, int nz, in
     int rc = 0;
     const size_t nbuf = kind == 2 ? 2 * n : n;
     cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&d, sizeof(float) * nbuf);
+    if (e == cudaSuccess) e = arecgb::dev_malloc(&d, sizeof(float) * nbuf);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d, data, sizeof(float) * n, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) {
         set_error(std::string(who) + ": " + cudaGetErrorString(e));
@@ -1127,7 +1127,7 @@ void arecgb_ccorr2d(int nx, int ny, float *x, float *y, float *c) {
     std::lock_guard<std::mutex> lk(g_mu);
     const size_t n = (size_t)nx * ny;
     float *d = nullptr;
-    if (cudaMalloc(&d, sizeof(float) * 3 * n) != cudaSuccess) {
+    if (arecgb::dev_malloc(&d, sizeof(float) * 3 * n) != cudaSuccess) {
         set_error("ccorr2d: device allocation failed");
         report_void("ccorr2d");
         return;
@@ -1146,7 +1146,7 @@ void arecgb_fshift2d(int nx, int ny, float *in, float *out, float sx, float sy) 
     std::lock_guard<std::mutex> lk(g_mu);
     const size_t n = (size_t)nx * ny;
     float *d = nullptr;
-    if (cudaMalloc(&d, sizeof(float) * (2 * n + 2)) != cudaSuccess) {
+    if (arecgb::dev_malloc(&d, sizeof(float) * (2 * n + 2)) != cudaSuccess) {
         set_error("fshift2d: device allocation failed");
         report_void("fshift2d");
         return;
@@ -1166,7 +1166,7 @@ void arecgb_speak(int nx, int ny, float *data, float *xt, float *yt) {
     std::lock_guard<std::mutex> lk(g_mu);
     const size_t n = (size_t)nx * ny;
     float *d = nullptr;
-    if (cudaMalloc(&d, sizeof(float) * (n + 2)) != cudaSuccess) {
+    if (arecgb::dev_malloc(&d, sizeof(float) * (n + 2)) != cudaSuccess) {
         set_error("speak: device allocation failed");
         report_void("speak");
         return;

@@ -740,7 +740,7 @@ static int line_plan(int N, LinePlan *lp) {
         std::vector<float2> h(2 * N, make_float2(0.f, 0.f));
         fill_twiddles(N, h.data());
         float2 *d = nullptr;
-        ARECGB_CUDA(cudaMalloc(&d, sizeof(float2) * 2 * N));
+        ARECGB_CUDA(dev_malloc(&d, sizeof(float2) * 2 * N));
         cudaError_t e = cudaMemcpy(d, h.data(), sizeof(float2) * 2 * N, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
             cudaFree(d);
@@ -757,8 +757,9 @@ static int line_plan(int N, LinePlan *lp) {
 // kPoolBytes between calls: cudaMalloc and cudaFree of 256 MB took a third of a shift
 // search on 30 pairs of 750 x 1000 (0.84 ms, 0.59 with the pool).  The pool hands memory
 // out in stream order, to any thread and stream; what a call holds beyond the limit
-// goes back when its stream is waited for, the rest when a plan is created
-// (scratch_trim).  A capturing stream gets cudaMalloc's refusal, as before.
+// goes back when its stream is waited for, the rest when a plan is created or an
+// allocation of the library fails (scratch_trim).  A capturing stream gets cudaMalloc's
+// refusal, as before.
 constexpr size_t kPoolBytes = (size_t)512 << 20;
 static std::mutex g_pool_mu;
 static std::map<int, cudaMemPool_t> g_pool;
@@ -812,7 +813,7 @@ struct Scratch {
             cudaGetLastError();
             p = nullptr;
         }
-        ARECGB_CUDA(cudaMalloc(&p, bytes));
+        ARECGB_CUDA(dev_malloc(&p, bytes));
         return 0;
     }
     // Waits for the stream, as the calls do before they return.

@@ -144,7 +144,7 @@ static int ramp_taps(Plan *p, int *doff, cudaStream_t st) {
         cudaFree(p->d_ramp);
         p->d_ramp = nullptr;
         p->ramp_n = 0;
-        ARECGB_CUDA(cudaMalloc(&p->d_ramp, sizeof(float) * n));
+        ARECGB_CUDA(dev_malloc(&p->d_ramp, sizeof(float) * n));
         k_ramp_taps<<<(n + 255) / 256, 256, 0, st>>>(p->d_ramp, n, off,
                                                      3.14159265358979323846 / p->na);
         ARECGB_CUDA(cudaGetLastError());

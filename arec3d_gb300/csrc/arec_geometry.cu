@@ -221,9 +221,9 @@ int plan_create(Plan **out, int weighting, double radius, int ny, int nangles,
 
     // Upload.
     cudaError_t e = cudaSuccess;
-    e = cudaMalloc(&p->d_groups, sizeof(int4) * groups.size());
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_tiles, sizeof(int2) * tiles.size());
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_err, sizeof(int));
+    e = dev_malloc(&p->d_groups, sizeof(int4) * groups.size());
+    if (e == cudaSuccess) e = dev_malloc(&p->d_tiles, sizeof(int2) * tiles.size());
+    if (e == cudaSuccess) e = dev_malloc(&p->d_err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(p->d_err, 0, sizeof(int));
     if (e == cudaSuccess)
         e = cudaMemcpy(p->d_groups, groups.data(), sizeof(int4) * groups.size(),
@@ -231,11 +231,11 @@ int plan_create(Plan **out, int weighting, double radius, int ny, int nangles,
     if (e == cudaSuccess)
         e = cudaMemcpy(p->d_tiles, tiles.data(), sizeof(int2) * tiles.size(),
                        cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_ray, sizeof(float4) * nr);
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_ang, sizeof(AngleParams) * nangles);
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_rows, sizeof(RowInfo) * nx);
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_cols, sizeof(ColInfo) * nx);
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_kinv, sizeof(int) * std::max(nr, 1));
+    if (e == cudaSuccess) e = dev_malloc(&p->d_ray, sizeof(float4) * nr);
+    if (e == cudaSuccess) e = dev_malloc(&p->d_ang, sizeof(AngleParams) * nangles);
+    if (e == cudaSuccess) e = dev_malloc(&p->d_rows, sizeof(RowInfo) * nx);
+    if (e == cudaSuccess) e = dev_malloc(&p->d_cols, sizeof(ColInfo) * nx);
+    if (e == cudaSuccess) e = dev_malloc(&p->d_kinv, sizeof(int) * std::max(nr, 1));
     if (e == cudaSuccess)
         e = cudaMemcpy(p->d_ray, ray.data(), sizeof(float4) * nr, cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
@@ -254,7 +254,7 @@ int plan_create(Plan **out, int weighting, double radius, int ny, int nangles,
         const int hv = std::max(1, p->vec / 2);
         const int bp_max = p->ntiles * ((p->ys + 32 * hv - 1) / (32 * hv));
         p->n_partials = std::max(bp_grid_blocks(p), bp_max);
-        e = cudaMalloc(&p->d_partials,
+        e = dev_malloc(&p->d_partials,
                        sizeof(double) * ((size_t)fp_grid_blocks(p) + std::max(p->n_partials, kNormBlocks)));
         if (e == cudaSuccess) p->d_bp_partials = p->d_partials + fp_grid_blocks(p);
     }

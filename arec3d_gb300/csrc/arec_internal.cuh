@@ -176,6 +176,14 @@ void plan_destroy(Plan *p);
 int set_smem(const void *kernel, size_t bytes);
 void scratch_trim();  // arec_ccorr.cu: gives unused alignment scratch back
 void graph_memory_trim();  // arec_project_mma.cu: and what graphs that are gone held
+
+// cudaMalloc; when the device is full, again after giving back what the library keeps
+// between calls.
+cudaError_t dev_malloc_bytes(void **p, size_t bytes);
+template <typename T>
+cudaError_t dev_malloc(T **p, size_t bytes) {
+    return dev_malloc_bytes(reinterpret_cast<void **>(p), bytes);
+}
 size_t vol_floats(const Plan *p);
 size_t sin_floats(const Plan *p);
 

@@ -284,7 +284,7 @@ int periodic_decomp(float *d, int nz, int ny, int nx, float *s_out, cudaStream_t
     const size_t off_t = off_w + ((sizeof(float2) * (size_t)ny * nh * batch + 255) / 256) * 256;
     const size_t bytes = off_t + sizeof(float2) * (size_t)ny * nh * batch;
     DevBuf buf;
-    ARECGB_CUDA(cudaMalloc(&buf.p, bytes));
+    ARECGB_CUDA(dev_malloc(&buf.p, bytes));
     char *b0 = (char *)buf.p;
     double2 *d_ex = (double2 *)b0, *d_ey = d_ex + nx;
     float2 *d_fx = (float2 *)(d_ey + ny), *d_fy = d_fx + nx;

@@ -112,6 +112,17 @@ __global__ void __launch_bounds__(256) k_zero_unless(float4 *q, size_t n4, const
         q[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
+cudaError_t dev_malloc_bytes(void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();  // not sticky
+        scratch_trim();
+        graph_memory_trim();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
 int set_smem(const void *kernel, size_t bytes) {
     static RaisedLimits limits;
     int dev = 0;
@@ -288,8 +299,8 @@ static int plan_build_lin_index(Plan *p) {
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
     if ((double)(b_off + b_list) > 0.4 * (double)free_b) return 0;
-    if (cudaMalloc(&p->d_lin_off, b_off) != cudaSuccess ||
-        cudaMalloc(&p->d_lin_list, b_list) != cudaSuccess) {
+    if (dev_malloc(&p->d_lin_off, b_off) != cudaSuccess ||
+        dev_malloc(&p->d_lin_list, b_list) != cudaSuccess) {
         cudaGetLastError();  // not sticky: run with the scatter
         cudaFree(p->d_lin_off);
         cudaFree(p->d_lin_list);
@@ -322,10 +333,10 @@ int plan_build_tables(Plan *p) {
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
     const size_t work = p->mma ? mma_work_bytes(p->nx, p->na, p->ys) : 0;  // in use already
     if ((double)(work + b_taps + b_bpw + b_bpf) > 0.4 * (double)(work + free_b)) return 0;
-    cudaError_t e = mma ? cudaMalloc(&p->d_ptaps, b_recs) : cudaMalloc(&p->d_taps, b_recs);
-    if (e == cudaSuccess && !mma) e = cudaMalloc(&p->d_xT, sizeof(float) * (size_t)p->nrays * p->ys);
-    if (e == cudaSuccess && !mma) e = cudaMalloc(&p->d_bpw, b_bpw);
-    if (e == cudaSuccess && !mma) e = cudaMalloc(&p->d_bpf, b_bpf);
+    cudaError_t e = mma ? dev_malloc(&p->d_ptaps, b_recs) : dev_malloc(&p->d_taps, b_recs);
+    if (e == cudaSuccess && !mma) e = dev_malloc(&p->d_xT, sizeof(float) * (size_t)p->nrays * p->ys);
+    if (e == cudaSuccess && !mma) e = dev_malloc(&p->d_bpw, b_bpw);
+    if (e == cudaSuccess && !mma) e = dev_malloc(&p->d_bpf, b_bpf);
     if (e != cudaSuccess) {
         cudaGetLastError();  // an allocation failure is not sticky; run without tables
         cudaFree(p->d_taps);

@@ -1010,7 +1010,7 @@ Seg make_segments(const std::vector<AngleParams> &ang, int a0, int n, int orient
 
 template <typename T>
 int upload(T **d, const std::vector<T> &h) {
-    ARECGB_CUDA(cudaMalloc(d, sizeof(T) * std::max<size_t>(h.size(), 1)));
+    ARECGB_CUDA(dev_malloc(d, sizeof(T) * std::max<size_t>(h.size(), 1)));
     ARECGB_CUDA(cudaMemcpy(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
     return 0;
 }
@@ -1123,8 +1123,8 @@ int mma_plan_create(Plan *p, const std::vector<int4> &g4, const std::vector<Angl
     // written), and the slices' maxima
     const size_t bytes[2] = {sizeof(float) * (size_t)p->nx * p->nx * p->ys, sizeof(float) * sin_floats(p)};
     for (int d = 0; d < 2; d++) {
-        if (cudaMalloc(&p->d_half[d], bytes[d]) != cudaSuccess ||
-            cudaMalloc(&p->d_smax[d], mma_stats_bytes(p->ys)) != cudaSuccess) {
+        if (dev_malloc(&p->d_half[d], bytes[d]) != cudaSuccess ||
+            dev_malloc(&p->d_smax[d], mma_stats_bytes(p->ys)) != cudaSuccess) {
             cudaGetLastError();  // not sticky: run without
             mma_plan_destroy(p);
             return 0;
@@ -1349,7 +1349,7 @@ void *graph_memory(cudaGraph_t graph, size_t bytes) {
         m->bytes = bytes;
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // this capture is no bar
         const bool relaxed = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
-        if (!relaxed || cudaMalloc(&m->ptr, bytes) != cudaSuccess) m->ptr = nullptr;
+        if (!relaxed || dev_malloc(&m->ptr, bytes) != cudaSuccess) m->ptr = nullptr;
         if (relaxed) cudaThreadExchangeStreamCaptureMode(&mode);
     }
     cudaUserObject_t obj = nullptr;

@@ -491,7 +491,7 @@ int rot_cc_angles(const float *d1, const float *d2, int nz, int ny, int nx, int 
     }
     const size_t prof_bytes = ((sizeof(float) * 2 * (size_t)nz * n + 255) / 256) * 256;
     DevBuf buf;
-    ARECGB_CUDA(cudaMalloc(&buf.p, prof_bytes + sizeof(double) * cs.size()));
+    ARECGB_CUDA(dev_malloc(&buf.p, prof_bytes + sizeof(double) * cs.size()));
     float *prof = (float *)buf.p;                              // [2][nz][n]
     double *d_cs = (double *)((char *)buf.p + prof_bytes);     // cos, sin tables
     ARECGB_CUDA(cudaMemcpyAsync(d_cs, cs.data(), sizeof(double) * cs.size(), cudaMemcpyHostToDevice, st));
@@ -528,7 +528,7 @@ int profile_shifts(const float *d_prof, int prof_y, int prof_x, int pad, int suc
         return ARECGB_ERR_ARG;
     }
     DevBuf buf;
-    ARECGB_CUDA(cudaMalloc(&buf.p, sizeof(double) * prof_y + sizeof(float) * prof_x));
+    ARECGB_CUDA(dev_malloc(&buf.p, sizeof(double) * prof_y + sizeof(float) * prof_x));
     double *d_out = (double *)buf.p;
     float *d_mean = (float *)(d_out + prof_y);
     if (!successive) {
@@ -579,7 +579,7 @@ int ncc_filtered(const float *d_a, const float *d_a2, const float *d_b, int nz, 
     tukey_table(ny, 0.3, h);
     tab.insert(tab.end(), h.begin(), h.end());
     DevBuf buf;
-    ARECGB_CUDA(cudaMalloc(&buf.p, sizeof(double) * tab.size()));
+    ARECGB_CUDA(dev_malloc(&buf.p, sizeof(double) * tab.size()));
     double *d_h = (double *)buf.p;
     ARECGB_CUDA(cudaMemcpyAsync(d_h, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, st));
     for (int z0 = 0; z0 < nz; z0 += 65535) {
@@ -628,7 +628,7 @@ int rotate_stack(float *d_img, const float *d_ref, int nz, int ny, int nx, float
                                                   sizeof(double) * tab.size() + sizeof(int) * nz
                                             : 0;
     DevBuf buf;
-    ARECGB_CUDA(cudaMalloc(&buf.p, bytes_t + bytes_p + bytes_s));
+    ARECGB_CUDA(dev_malloc(&buf.p, bytes_t + bytes_p + bytes_s));
     float *t1 = (float *)buf.p, *t2 = t1 + slice * batch;
     RotParam *par = (RotParam *)((char *)buf.p + bytes_t);
     double *cc = (double *)((char *)buf.p + bytes_t + bytes_p);

@@ -151,7 +151,7 @@ int arecgb_solve_uneven(const arecgb_problem *probs, int n, size_t budget_bytes,
     };
     if (n_nets > 0) {
         for (auto &p : img) {
-            cudaError_t e = cudaMalloc(&p, sizeof(float) * img_floats);
+            cudaError_t e = dev_malloc(&p, sizeof(float) * img_floats);
             if (e != cudaSuccess) {
                 free_img();
                 set_error(std::string("arecgb_solve_uneven: ") + cudaGetErrorString(e));
@@ -201,7 +201,7 @@ int arecgb_solve_uneven(const arecgb_problem *probs, int n, size_t budget_bytes,
                 // the filtered sinogram goes to the sinogram scratch CGLS uses next
                 if (!p->d_sin[0]) {
                     const size_t ns = sin_floats(p);
-                    cudaError_t e = cudaMalloc(&p->d_sin[0], sizeof(float) * ns);
+                    cudaError_t e = dev_malloc(&p->d_sin[0], sizeof(float) * ns);
                     if (e == cudaSuccess) e = cudaMemsetAsync(p->d_sin[0], 0, sizeof(float) * ns, st);
                     if (e != cudaSuccess) {
                         set_error(std::string("arecgb_solve_uneven: ") + cudaGetErrorString(e));

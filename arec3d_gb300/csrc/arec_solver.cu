@@ -449,12 +449,12 @@ static int ensure_workspace(Plan *p, int nvol, int nsin) {
     const size_t nv = vol_floats(p), ns = sin_floats(p);
     for (int i = 0; i < nvol; i++)
         if (!p->d_vol[i]) {
-            ARECGB_CUDA(cudaMalloc(&p->d_vol[i], sizeof(float) * nv));
+            ARECGB_CUDA(dev_malloc(&p->d_vol[i], sizeof(float) * nv));
             ARECGB_CUDA(cudaMemset(p->d_vol[i], 0, sizeof(float) * nv));
         }
     for (int i = 0; i < nsin; i++)
         if (!p->d_sin[i]) {
-            ARECGB_CUDA(cudaMalloc(&p->d_sin[i], sizeof(float) * ns));
+            ARECGB_CUDA(dev_malloc(&p->d_sin[i], sizeof(float) * ns));
             ARECGB_CUDA(cudaMemset(p->d_sin[i], 0, sizeof(float) * ns));
         }
     return ARECGB_OK;
@@ -463,7 +463,7 @@ static int ensure_workspace(Plan *p, int nvol, int nsin) {
 constexpr int kRedBlocks = kSredBlocks;
 
 int ensure_red(Plan *p) {
-    if (!p->d_sred) ARECGB_CUDA(cudaMalloc(&p->d_sred, sizeof(double) * (2 * kSredBlocks + 2)));
+    if (!p->d_sred) ARECGB_CUDA(dev_malloc(&p->d_sred, sizeof(double) * (2 * kSredBlocks + 2)));
     if (!p->h_sred && cudaMallocHost(&p->h_sred, sizeof(double) * 2) != cudaSuccess) {
         p->h_sred = nullptr;
         set_error("pinned allocation failed");
@@ -562,7 +562,7 @@ int cgls_batch(Plan *const *plans, const float *const *d_b, float *const *d_x, c
         if (q0->h_cstate) cudaFreeHost(q0->h_cstate);
         q0->d_cstate = q0->h_cstate = nullptr;
         q0->cstate_bytes = 0;
-        e = cudaMalloc(&q0->d_cstate, s_bytes);
+        e = dev_malloc(&q0->d_cstate, s_bytes);
         if (e == cudaSuccess) e = cudaMallocHost(&q0->h_cstate, s_bytes);
         if (e == cudaSuccess) q0->cstate_bytes = s_bytes;
     }
@@ -570,7 +570,7 @@ int cgls_batch(Plan *const *plans, const float *const *d_b, float *const *d_x, c
         cudaFree(q0->d_chist);
         q0->d_chist = nullptr;
         q0->chist_bytes = 0;
-        e = cudaMalloc(&q0->d_chist, h_bytes);
+        e = dev_malloc(&q0->d_chist, h_bytes);
         if (e == cudaSuccess) q0->chist_bytes = h_bytes;
     }
     if (e == cudaSuccess && !q0->solve_stream)
@@ -742,7 +742,7 @@ int cgls(Plan *p, const float *d_b, float *d_x, int warm, int maxit, float tol, 
 int cgls_stat(Plan *p, const float *d_b, float *d_x, int warm, int maxit, float tol,
               double *hist_host, arecgb_solve_info *info, cudaStream_t st) {
     const size_t ns = sin_floats(p);
-    if (!p->d_w) ARECGB_CUDA(cudaMalloc(&p->d_w, sizeof(float) * ns));
+    if (!p->d_w) ARECGB_CUDA(dev_malloc(&p->d_w, sizeof(float) * ns));
     std::vector<double> hx(p->nx);
     const double alpha = 0.5, pi = std::atan(1.0) * 4.0;
     const double xa = 0.5 * alpha * (p->nx - 1), xb = (1.0 - 0.5 * alpha) * (p->nx - 1);

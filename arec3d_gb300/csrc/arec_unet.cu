@@ -79,7 +79,7 @@ static constexpr int kLossBlocks = 512;
 template <typename T>
 static int alloc(Net *n, T **p, size_t count) {
     void *q = nullptr;
-    ARECGB_CUDA(cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T)));
+    ARECGB_CUDA(dev_malloc(&q, std::max<size_t>(count, 1) * sizeof(T)));
     n->blocks.push_back(q);
     *p = reinterpret_cast<T *>(q);
     return 0;
