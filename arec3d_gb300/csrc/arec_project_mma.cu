@@ -50,15 +50,19 @@ constexpr uint32_t kMmaWait = 1u << 22;
 constexpr int kTakers = 8, kBuilders = 8, kLoadWarp = 16, kMmaWarp = 17;
 constexpr int kMmaThreads = 32 * 20;
 // The tensor core's rounding toward zero takes part of every sum: at 129 to 512 pixels
-// 8.8e-8 of a forward projection of data of one sign, 6.9e-8 with both signs, 3.8e-8 at
-// 5 % of the rays (back 4.9e-8, 4.5e-8, 3.6e-8), nothing of sums that are exact.  The
-// conversion adds this share of a value to its low half: the same for every ray and
-// angle, so A and A^T stay transposes of each other but for their scale.  Errors
-// against FP64 at 256 pixels, 64 angles: dense 6.5e-8 and 4.3e-8 back (1.09e-7 and 6.4e-8
-// without, FP32 kernels 1.34e-7 and 1.66e-7), 5 % of the rays 6.4e-8 and 5.2e-8 (7.0e-8,
-// 6.3e-8; 4.8e-8, 5.2e-8), single rays 8.6e-8 and 5.3e-8 (5.4e-8, 5.3e-8; 4.3e-8, 4.0e-8):
+// 8.4e-8 to 9.3e-8 of a forward projection of data of one sign (random values, spheres,
+// a reconstruction), 7.0e-8 with both signs, 3.8e-8 at 5 % of the rays (back 4.5e-8 to
+// 5.3e-8, 4.7e-8, 3.6e-8), nothing of sums that are exact.  The conversion adds this share
+// of a value to its low half (where some of it is rounded away again): the same for
+// every ray and angle, so A and A^T stay transposes of each other but for their scale,
+// and set for data of one sign, whose projections lose or gain 0.5e-8 at most: b - A x0
+// of a warm start multiplies that (4 steps of Kaiser-Bessel CGLS from there at 65 bins:
+// 3.7e-7 from FP64; 3.2e-6 with factors on some of the sums, 3.0e-5 with none).  Errors
+// against FP64 at 256 pixels, 64 angles: dense 6.5e-8 and 4.1e-8 back (1.09e-7 and 6.4e-8
+// without, FP32 kernels 1.34e-7 and 1.66e-7), 5 % of the rays 7.5e-8 and 5.3e-8 (7.0e-8,
+// 6.3e-8; 4.8e-8, 5.2e-8), single rays 9.4e-8 and 6.4e-8 (5.4e-8, 5.3e-8; 4.3e-8, 4.0e-8):
 // what lost nothing is off by the share and its rounding, less than one last place.
-constexpr float kLostForward = 8e-8f, kLostBack = 4.5e-8f;
+constexpr float kLostForward = 9e-8f, kLostBack = 5.5e-8f;
 constexpr int kSegBlocks = 64;  // line blocks of a segment at most
 
 // ---------------------------------------------------------------------------
@@ -364,7 +368,7 @@ struct FpMma {
 // 8 angles and 256 slices the MMAs read 24 x 8 KB and the loads and builders
 // write 64 + 32 KB: 2300 clocks, against 1536 of tensor work (measured: 3000, and
 // a segment's end, adds to q, about a fifth of the whole).  A projection at
-// 1024^2 x 1200 angles x 512 slices takes 46.0 ms, 159.6 with the FP32 kernels,
+// 1024^2 x 1200 angles x 512 slices takes 44.3 ms, 159.6 with the FP32 kernels,
 // which the FMA pipes bound.
 template <int W, int MT>
 __global__ void __launch_bounds__(kMmaThreads, 1)
@@ -729,7 +733,7 @@ __device__ __forceinline__ void two_sum(unsigned long long *acc, uint32_t *va, u
 //
 // What bounds it: two angles' 24 MMAs read 24 x 6 KB of shared memory, 1300
 // clocks; they take 2460 alone, 2900 beside the takers' traffic with TMEM.  A
-// back projection at 1024^2 x 1200 angles x 512 slices takes 76.0 ms, 209.1 with
+// back projection at 1024^2 x 1200 angles x 512 slices takes 72.3 ms, 209.1 with
 // the FP32 kernels as a plan comes (110.7 with tuned shapes).
 template <int W>
 __global__ void __launch_bounds__(kMmaThreads, 1)
