@@ -199,8 +199,7 @@ __global__ void __launch_bounds__(fft::kThreads, 2)
     };
     if constexpr (N > 0) {
         using L2 = Pow2<N>;
-        constexpr int TPL = L2::TPL, CT = L2::G;
-        constexpr int Ra = L2::template radix<false>(0), Rl = L2::template radix<false>(L2::P - 1);
+        constexpr int TPL = L2::TPL, CT = L2::G, Ra = L2::template radix<false>(0);
         const int c = threadIdx.x % CT, b = threadIdx.x / CT;
         float2 v[2][16];
 #pragma unroll
@@ -218,7 +217,6 @@ __global__ void __launch_bounds__(fft::kThreads, 2)
         __syncthreads();  // the lines' layout changes
         fft::transform<N, true, false, 1>(w, sm2 + c * LS2, b, twr);
         if (c0 + c >= H) return;
-        (void)Rl;
 #pragma unroll
         for (int i = 0; i < 16 / Ra; i++)
 #pragma unroll
@@ -1065,9 +1063,10 @@ int peak_search(const float *dc, int nz, int ny, int nx, float *sx, float *sy, i
 //
 // For callers that must not allocate device memory while they run: an
 // alignment loop that interleaves shift searches with a reconstruction running
-// on another stream (cc_shifts' cudaFree synchronises the whole device and
-// would stall that solve), or a host whose memory is owned by another
-// allocator (a caching allocator that already holds the free HBM).
+// on another stream (cc_shifts waits for its own stream before it returns, and for the
+// whole device where its pool cannot serve it and cudaFree takes its place), or a
+// host whose memory is owned by another allocator (a caching allocator that already
+// holds the free HBM).
 //
 // Scratch: one file-scope device array of kStaticBytes (3.5 MiB), carved into
 //   S       float4 [kStaticSpec]   half spectra of both images; then the

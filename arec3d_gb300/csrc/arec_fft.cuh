@@ -210,8 +210,8 @@ __device__ __forceinline__ void exchange_sync() {
 // One pass boundary: v holds pass p's outputs (radix R, stride Ns); leaves in
 // v the inputs of the next pass (radix RN, stride Ns * R), twiddled.
 // b: the thread's index in its line; L: the line in shared memory.
-template <int N, int R, int RN, int Ns, bool WARP, int K, typename T, typename TW>
-__device__ __forceinline__ void exchange(float2 (&v)[K][16], T *L, int b, const float2 *tw, TW) {
+template <int N, int R, int RN, int Ns, bool WARP, int K, typename T>
+__device__ __forceinline__ void exchange(float2 (&v)[K][16], T *L, int b, const float2 *tw) {
     constexpr int TPL = N / 16;
     exchange_sync<WARP>();  // earlier reads of the buffer
 #pragma unroll
@@ -253,8 +253,6 @@ __device__ __forceinline__ void butterflies(float2 (&v)[K][16]) {
         for (int i = 0; i < 16 / R; i++) dft<R>(&v[c][i * R]);
 }
 
-struct NoTag {};
-
 // Forward transforms of K lines' worth of points per thread, in step (K = 1:
 // T = float2; K = 2: T = float4, the two lines interleaved).  In: v[c][i * R +
 // r] = point (b + i TPL) + r N / R with R the first radix; out: the same with
@@ -266,11 +264,11 @@ __device__ __forceinline__ void transform(float2 (&v)[K][16], T *L, int b, const
     butterflies<Ra, K>(v);
     if constexpr (P::P > 1) {
         constexpr int Rb = P::template radix<REV>(1);
-        exchange<N, Ra, Rb, 1, WARP, K, T>(v, L, b, tw, NoTag{});
+        exchange<N, Ra, Rb, 1, WARP, K, T>(v, L, b, tw);
         butterflies<Rb, K>(v);
         if constexpr (P::P > 2) {
             constexpr int Rc = P::template radix<REV>(2);
-            exchange<N, Rb, Rc, Ra, WARP, K, T>(v, L, b, tw, NoTag{});
+            exchange<N, Rb, Rc, Ra, WARP, K, T>(v, L, b, tw);
             butterflies<Rc, K>(v);
         }
     }

@@ -1036,10 +1036,11 @@ static const int kMinBlocks = 10;
 // more for Kaiser-Bessel, whose taps cost more to compute): 160^2 x 90 x 16 0.094
 // against 0.107 ms, forward 0.20 against 0.36; 1024^2 x 600 x 8 10.7 against 17.8,
 // forward 11.5 against 36.6; at 96^2 x 24 x 8 it would be 0.043 against 0.029.  A long
-// CGLS solve amplifies rounding (its residual goes its own way after about six steps);
-// on slabs of a few slices, where solves are compared step by step with the reference,
-// it stays on the FP32 kernels, which sum in the reference's order: these do not, and
-// end closer to FP64 than to it.  4096 angles fill the back projector's table.
+// CGLS solve amplifies rounding (every float solve leaves FP64's trajectory after six
+// to eight steps, the reference's too).  With fewer than 48 slices it stays on the FP32
+// kernels, which sum in the reference's order, and small solves keep its residual
+// trace; that is a choice, not a matter of time.  From 48 slices on it ends 2 to 10
+// times nearer FP64 here.  4096 angles fill the back projector's table.
 int mma_takes(int weighting, int nx, int ys, int na) {
     if (weighting == ARECGB_LIN || nx < 32 || na > BpMma::MAX_NA) return 0;
     const double px = (double)nx * nx;

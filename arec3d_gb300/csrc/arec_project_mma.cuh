@@ -5,7 +5,7 @@
 // Taken 8 x 8 pixels at a time the matrix is dense enough for the tensor cores:
 // at any angle the 64 rays of a block reach at most 13 neighbouring bins, so
 // with windows of 16 bins a block's product with one angle is a 64 x 16 matrix
-// per slice, 16/3 of the multiply-adds of the sparse one, at 28 times the FP32
+// per slice, 16/3 of the multiply-adds of the sparse one, at 24 times the FP32
 // rate.  Both factors are split into two FP16 numbers each: three products
 // hi*hi, hi*lo, lo*hi carry 22 bits.  The tensor core's FP32 accumulation rounds
 // toward zero, so a sum stays in TMEM for one block only; FP32 registers take

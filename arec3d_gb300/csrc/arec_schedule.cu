@@ -9,7 +9,7 @@
 // the plan's operands and geometry tables) does not fit for all of them at once, so the
 // problems are packed into waves whose workspace fits a byte budget (first
 // fit, largest first).  Per wave: one plan per problem (without the optional
-// projector tables: they would cost 32 B per ray and angle), the optional
+// projector tables: they would cost 16 or 32 B per ray and angle), the optional
 // learned warm start per problem (SIRT -> U-Net), then one batched CGLS in
 // which every iteration of all the wave's problems is one CUDA graph launch
 // (each problem a parallel branch; a converged problem's kernels become

@@ -599,6 +599,8 @@ int conv3x3_bf16(const void *X, const void *Wt, const float *bias, void *Y, int 
     rc = launch_conv_pipe<C, R, BAND, KC, ST>(x, w, bias, y, N, H, Wd, Cin, LW, relu, ystride, err, st)
         const int lw = conv_tile(H, Wd);
         const bool wide = Cin % 64 == 0;
+        // Bands need widths of 128.  They would run at any height; taking them at multiples
+        // of 4 and 2 keeps the order of every size's products, and so its last places.
         // Two tiles share a chunk's weights (48 KB loaded for them instead of 64 at
         // 128 channels) where that leaves every SM a pair.  Bands: as many rows as
         // two stages of their chunks leave room for.

@@ -188,7 +188,7 @@ FP64_SLICES = (137, 388)
 def fp64_check(gb, plan, b_s, x_s, slices):
     """||A^T (b - A x)|| / ||A^T b|| over `slices` of the headline result,
     recomputed with the oracle's FP64 projectors (the checker), beside the same
-    quantity evaluated by the GPU projectors in FP32.  b_s: [na][nx][k] and x_s:
+    quantity evaluated by the GPU projectors.  b_s: [na][nx][k] and x_s:
     [nrays][k] float32 host arrays of those slices."""
     import torch
 
@@ -204,7 +204,7 @@ def fp64_check(gb, plan, b_s, x_s, slices):
         atr = oracle.backproject64(3, radius, r, plan.angles)
     rel64 = float(np.linalg.norm(atr) / np.linalg.norm(atb))
     secs = time.perf_counter() - t0
-    # the GPU's FP32 evaluation of the same quantity (a plan of k slices)
+    # the GPU's evaluation of the same quantity (a plan of k slices)
     k = len(slices)
     old = os.environ.get("ARECGB_PLAN_TABLES")
     os.environ["ARECGB_PLAN_TABLES"] = "0"  # same results without the tables
@@ -231,7 +231,8 @@ def fp64_check(gb, plan, b_s, x_s, slices):
             "abs_diff": abs(rel64 - rel32), "oracle_seconds": secs,
             "note": "normal-equation residual of the last timed solve over these slices "
                     "(numerator and denominator restricted to them), FP64 oracle projectors "
-                    "vs the GPU's FP32 projectors"}
+                    "vs the GPU's projectors (operands as FP16 pairs of 22 bits, FP32 "
+                    "sums)"}
 
 
 def make_problem(gb, seed, device="cuda"):
@@ -611,8 +612,9 @@ def main():
     ap.add_argument("--ref-angle-step", type=int, default=CPU_ANGLE_STEP,
                     help="reference arm: keep every k-th angle in each step's CPU sample")
     ap.add_argument("--ref-iters", type=int, default=32,
-                    help="iterations to extrapolate the reference arm to (plain CGLS needs 32 "
-                         "on this problem)")
+                    help="iterations to extrapolate the reference arm to (plain CGLS on FP32 "
+                         "projectors, whose sums are the reference's, needs 32 on this problem; "
+                         "on the tensor-core projectors, nearer FP64, 29)")
     ap.add_argument("--kernels-only", action="store_true",
                     help="run only the forward and back projectors (for profiling)")
     ap.add_argument("--slices", type=int, default=NY, help="slices for --kernels-only")
@@ -894,6 +896,8 @@ def main():
                          "note": "created once per geometry, outside the timed region"})
         cfg["fp64_check"] = fp64
         cfg["error_vs_phantom"] = err_headline
+        cfg["arithmetic"] = ("FP32 volumes, sinograms and sums; projector operands as FP16 pairs "
+                             "(22 bits)" + ("; network BF16" if net is not None else ""))
         if net is not None:
             first = "filtered back projection" if sirt_iters == 0 else "SIRT-%d" % sirt_iters
             cfg.update(warm_start=True, network_input=first, stage_ms=stages,

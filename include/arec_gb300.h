@@ -65,8 +65,8 @@ int arecgb_version(void);
  * AREC3D/AREC3D/arecImage.cpp:29), ny slices, nangles float radians (copied).
  * Allocates device tables on the current device, and for square-pixel and
  * Kaiser-Bessel plans of more than a few angles and slices (those whose projections
- * run on the tensor cores; with fewer than 48 slices CGLS keeps to FP32 kernels) room for one volume (of all nx nx pixels) and one sinogram as FP16 pairs,
- * unless that takes more than 40 % of the free memory or leaves no room for a solve's
+ * run on the tensor cores; with fewer than 48 slices CGLS keeps to FP32 kernels) room
+ * for one volume (of all nx nx pixels) and one sinogram as FP16 pairs, unless that takes more than 40 % of the free memory or leaves no room for a solve's
  * workspace (the FP32 projectors then).
  * The first call captured into a graph on a stream allocates this room again, for the
  * graph, its clones and instances (freed with a later plan_create or plan_destroy once
@@ -156,7 +156,8 @@ int arecgb_plan_timing(arecgb_plan *plan, int mode, double *fp_ms, long long *fp
  * which it overwrites, and keeps the fastest; reports the band and the chunks
  * (either pointer may be NULL; arecgb_plan_shapes reports all four).  Results
  * do not depend on the choice beyond float summation order across bands.
- * Plans all of whose projections run on the tensor cores have one shape: the call reports their defaults and leaves the buffers alone.  No
+ * Plans all of whose projections run on the tensor cores have one shape: the call
+ * reports their defaults and leaves the buffers alone.  No
  * counterpart in the reference. */
 int arecgb_plan_autotune(arecgb_plan *plan, float *d_x, float *d_q, int *fp_band, int *bp_nsc,
                          void *stream);
