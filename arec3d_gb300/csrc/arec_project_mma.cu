@@ -368,7 +368,7 @@ struct FpMma {
 // 8 angles and 256 slices the MMAs read 24 x 8 KB and the loads and builders
 // write 64 + 32 KB: 2300 clocks, against 1536 of tensor work (measured: 3000, and
 // a segment's end, adds to q, about a fifth of the whole).  A projection at
-// 1024^2 x 1200 angles x 512 slices takes 44.3 ms, 159.6 with the FP32 kernels,
+// 1024^2 x 1200 angles x 512 slices takes 43.8 ms, 159.6 with the FP32 kernels,
 // which the FMA pipes bound.
 template <int W, int MT>
 __global__ void __launch_bounds__(kMmaThreads, 1)
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
     using C = FpMma<MT>;
     extern __shared__ unsigned char sm_raw[];
     __shared__ __align__(8) uint64_t xfull[C::STAGES][C::NSUB], xempty[C::STAGES][C::NSUB];
-    __shared__ __align__(8) uint64_t bfull[C::STAGES], bempty[C::STAGES], accfull[2], accfree[2];
+    __shared__ __align__(8) uint64_t bfull[C::STAGES], bempty[C::STAGES], accfull[2], accfree[2], drained;
     __shared__ uint32_t tmem_base;
     // per line block of the segment and line: ray of the strip's first pixel
     // (of pixel p: that plus p), and the pixels that are rays, first | last << 8
@@ -443,6 +443,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
             umma::mbar_init(&accfull[b], 1);
             umma::mbar_init(&accfree[b], kTakers);
         }
+        umma::mbar_init(&drained, 1);
         umma::mbar_fence_init();
     }
     __syncthreads();
@@ -471,11 +472,12 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
             // ---- loads (pixels outside the disk or the image are zeros)
             if (lane == 0) {
                 bool ok = true;
-                for (int it = 0; it < nb && ok; it++) {
+                int it = 0, i = 0;
+                for (; it < nb && ok; it += ok) {
                     const int s = it % C::STAGES, lb = sg.x + blist[it], P0 = j8 + shear[lb];
                     const int ix = orient ? 8 * lb : P0, iz = orient ? P0 : 8 * lb;
 #pragma unroll 1
-                    for (int i = 0; i < C::NSUB && ok; i++) {
+                    for (i = 0; i < C::NSUB; i++) {
                         if (it >= C::STAGES)
                             ok = umma::mbar_wait(&xempty[s][i], (uint32_t)(it / C::STAGES - 1) & 1u,
                                                  kMmaWait);
@@ -487,7 +489,14 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
                         umma::tma_load_4d(d + 8192, &tmx, y + 64, ix, iz, 1 - (i & 1), &xfull[s][i]);
                     }
                 }
-                if (!ok) atomicOr(A.err, 16);
+                if (!ok) {
+                    atomicOr(A.err, 16);
+                    // copies in flight: the last line blocks' and the first i of this one's
+                    for (int u = max(0, it - C::STAGES); u <= it; u++)
+                        for (int j = 0; j < (u < it ? C::NSUB : i); j++)
+                            umma::mbar_wait(&xfull[u % C::STAGES][j], (uint32_t)(u / C::STAGES) & 1u,
+                                            kMmaWait);
+                }
             }
         } else if (warp == kMmaWarp) {
             // ---- MMAs: low-order products first (their sums are small), then
@@ -534,7 +543,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
                 umma::mma_commit_warp(&bempty[s]);
                 umma::mma_commit_warp(&accfull[b]);
             }
-            if (!ok && lane == 0) atomicOr(A.err, 16);
+            if (!ok) {
+                if (lane == 0) atomicOr(A.err, 16);
+                umma::mma_drain_warp(&drained, kMmaWait);  // half a block of rays, uncommitted
+            }
         }
         __syncwarp();
     } else if (warp >= kTakers) {
@@ -733,7 +745,7 @@ __device__ __forceinline__ void two_sum(unsigned long long *acc, uint32_t *va, u
 //
 // What bounds it: two angles' 24 MMAs read 24 x 6 KB of shared memory, 1300
 // clocks; they take 2460 alone, 2900 beside the takers' traffic with TMEM.  A
-// back projection at 1024^2 x 1200 angles x 512 slices takes 72.3 ms, 209.1 with
+// back projection at 1024^2 x 1200 angles x 512 slices takes 72.4 ms, 209.1 with
 // the FP32 kernels as a plan comes (110.7 with tuned shapes).
 template <int W>
 __global__ void __launch_bounds__(kMmaThreads, 1)
@@ -796,7 +808,8 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
         regs_dec<C::REGS_LOW>();
         if (warp == kLoadWarp && lane == 0) {
             bool ok = true;
-            for (int it = 0; it < ns && ok; it++) {
+            int it = 0;
+            for (; it < ns && ok; it++) {
                 const int s = it % C::STAGES, a = a_lo + 2 * it, n = min(2, na - a);
                 if (it >= C::STAGES)
                     ok = umma::mbar_wait(&empty[s], (uint32_t)(it / C::STAGES - 1) & 1u, kMmaWait);
@@ -809,7 +822,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
                     umma::tma_load_4d(d + C::PART, &tms, 8 * f, yb / 8, a + i, 1, &afull[s]);
                 }
             }
-            if (!ok) atomicOr(A.err, 16);
+            if (!ok) {
+                atomicOr(A.err, 16);
+                umma::ring_drain(afull, C::STAGES, it, kMmaWait);
+            }
         } else if (warp == kMmaWarp) {
             // FP16, A MN-major (bit 15), B K-major, N = 64
             const uint32_t idesc = (1u << 4) | (1u << 15) | (8u << 17) | ((128u >> 4) << 24);
@@ -854,6 +870,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
                 umma::mma_commit_warp(&empty[s]);
                 umma::mma_commit_warp(&accfull[b]);
             }
+            // (the takers wait for every set of MMAs issued, each of which is committed)
             if (!ok && lane == 0) atomicOr(A.err, 16);
         }
         __syncwarp();

@@ -211,6 +211,18 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t *mbar, uint32_t parity, 
     return false;
 }
 
+// Where a wait has given up, before the block returns: the last use of each of a ring's
+// stages has landed (`used` uses in all), or this wait has given up too.
+__device__ __forceinline__ void ring_drain(uint64_t *full, int stages, int used, uint32_t limit) {
+    for (int i = used > stages ? used - stages : 0; i < used; i++)
+        mbar_wait(&full[i % stages], (uint32_t)(i / stages) & 1u, limit);
+}
+// The MMAs this warp has issued are done (`done`: a barrier of its own, not used before).
+__device__ __forceinline__ void mma_drain_warp(uint64_t *done, uint32_t limit) {
+    mma_commit_warp(done);
+    mbar_wait_warp(done, 0u, limit);
+}
+
 // Plain arrival (release semantics) on an mbarrier.
 __device__ __forceinline__ void mbar_arrive(uint64_t *mbar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_addr(mbar)) : "memory");

@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1)
                   "TMEM columns: a power of two in [32, 512]");
     static_assert(Cfg::STAGE % 1024 == 0, "stages stay 1024-byte aligned");
     extern __shared__ unsigned char sm_raw[];
-    __shared__ __align__(8) uint64_t full[ST], empty[ST], accfull[2], accfree[2];
+    __shared__ __align__(8) uint64_t full[ST], empty[ST], accfull[2], accfree[2], drained;
     __shared__ __align__(16) float s_bias[COUT];
     __shared__ uint32_t tmem_base;
     const uint32_t raw = umma::smem_addr(sm_raw);
@@ -261,6 +261,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1)
             umma::mbar_init(&accfull[b], 1);
             umma::mbar_init(&accfree[b], 4);
         }
+        umma::mbar_init(&drained, 1);
         umma::mbar_fence_init();
     }
     for (int i = tid; i < COUT; i += kPipeThreads) s_bias[i] = bias ? bias[i] : 0.f;
@@ -297,7 +298,10 @@ __global__ void __launch_bounds__(kPipeThreads, 1)
                     }
                 }
             }
-            if (!ok) atomicOr(err, 4);
+            if (!ok) {
+                atomicOr(err, 4);
+                umma::ring_drain(full, ST, it, kWaitLimit);
+            }
         }
         __syncwarp();
     } else if (warp == kPipeMma) {
@@ -354,7 +358,10 @@ __global__ void __launch_bounds__(kPipeThreads, 1)
             }
             if (ok) umma::mma_commit_warp(&accfull[i & 1]);
         }
-        if (!ok && lane == 0) atomicOr(err, 4);
+        if (!ok) {
+            if (lane == 0) atomicOr(err, 4);
+            umma::mma_drain_warp(&drained, kWaitLimit);
+        }
         __syncwarp();
     } else {
         // TMEM lane = pixel of a tile, this warp's from 32 warp on

@@ -132,6 +132,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
                 if (it >= J.stages &&
                     !umma::mbar_wait(&empty[s], (uint32_t)(it / J.stages - 1) & 1u, kWgWait)) {
                     atomicOr(err, 4);
+                    umma::ring_drain(full, J.stages, it, kWgWait);
                     break;
                 }
                 const int w0 = c % J.wt * kPix, h0 = c / J.wt % J.ht * kPix, n = c / (J.wt * J.ht);
@@ -172,6 +173,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
                     umma::mma_commit_warp(&accfull[b][t]);
                 }
             }
+            // (the epilogue waits for every tile's MMAs, each of which is committed)
             if (!ok && lane == 0) atomicOr(err, 4);
         }
         __syncwarp();
