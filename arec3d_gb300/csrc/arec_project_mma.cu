@@ -1075,8 +1075,10 @@ int mma_plan_create(Plan *p, const std::vector<int4> &g4, const std::vector<Angl
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
     const size_t work = mma_work_bytes(p->nx, p->na, p->ys);
     if (spare && (double)work > 0.4 * (double)free_b) return 0;
-    // a solve (up to four volumes and three sinograms) must still fit beside them
-    if (work + sizeof(float) * (4 * vol_floats(p) + 3 * sin_floats(p)) > free_b) return 0;
+    // a solve must still fit beside them: the caller's volume and sinogram and CGLS's three
+    // and two; only these where the caller budgets its memory (spare is false)
+    const size_t extra = spare ? 1 : 0;
+    if (work + sizeof(float) * ((3 + extra) * vol_floats(p) + (2 + extra) * sin_floats(p)) > free_b) return 0;
     const int nlb = (p->nx + 7) / 8;
     std::vector<int4> groups;
     std::vector<int2> strips;
