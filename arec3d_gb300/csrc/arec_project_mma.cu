@@ -1348,13 +1348,22 @@ struct GraphMemory {
     void *ptr = nullptr;
     size_t bytes = 0;
 };
-std::mutex g_graph_mu;
-std::vector<GraphMemory> g_graph_free;  // of graphs that are gone
+// Memory of graphs that are gone.  Never destroyed: graphs may go after this library's
+// static objects, at the end of the process.
+struct FreeGraphMemory {
+    std::mutex mu;
+    std::vector<GraphMemory> list;
+};
+FreeGraphMemory &graph_free() {
+    static FreeGraphMemory *f = new FreeGraphMemory;
+    return *f;
+}
 
 // May not call into CUDA: the memory is taken again, or freed by graph_memory_trim.
 void graph_memory_drop(void *m) {
-    std::lock_guard<std::mutex> lk(g_graph_mu);
-    g_graph_free.push_back(*static_cast<GraphMemory *>(m));
+    FreeGraphMemory &f = graph_free();
+    std::lock_guard<std::mutex> lk(f.mu);
+    f.list.push_back(*static_cast<GraphMemory *>(m));
     delete static_cast<GraphMemory *>(m);
 }
 
@@ -1362,11 +1371,12 @@ void graph_memory_drop(void *m) {
 void *graph_memory(cudaGraph_t graph, size_t bytes) {
     GraphMemory *m = new GraphMemory;
     if (cudaGetDevice(&m->device) == cudaSuccess) {
-        std::lock_guard<std::mutex> lk(g_graph_mu);
-        for (size_t i = 0; i < g_graph_free.size() && !m->ptr; i++)
-            if (g_graph_free[i].device == m->device && g_graph_free[i].bytes == bytes) {
-                *m = g_graph_free[i];
-                g_graph_free.erase(g_graph_free.begin() + i);
+        FreeGraphMemory &f = graph_free();
+        std::lock_guard<std::mutex> lk(f.mu);
+        for (size_t i = 0; i < f.list.size() && !m->ptr; i++)
+            if (f.list[i].device == m->device && f.list[i].bytes == bytes) {
+                *m = f.list[i];
+                f.list.erase(f.list.begin() + i);
             }
     }
     if (!m->ptr) {
@@ -1396,11 +1406,12 @@ void *graph_memory(cudaGraph_t graph, size_t bytes) {
 void graph_memory_trim() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return;
-    std::lock_guard<std::mutex> lk(g_graph_mu);
-    for (size_t i = g_graph_free.size(); i-- > 0;)
-        if (g_graph_free[i].device == dev) {
-            cudaFree(g_graph_free[i].ptr);
-            g_graph_free.erase(g_graph_free.begin() + i);
+    FreeGraphMemory &f = graph_free();
+    std::lock_guard<std::mutex> lk(f.mu);
+    for (size_t i = f.list.size(); i-- > 0;)
+        if (f.list[i].device == dev) {
+            cudaFree(f.list[i].ptr);
+            f.list.erase(f.list.begin() + i);
         }
 }
 
