@@ -204,7 +204,8 @@ class Turn {
     cudaStream_t st = nullptr;
 };
 
-// Operators (arec_project.cu); fp32: on the FP32 kernels in any case
+// Operators (arec_project.cu); fp32: on the FP32 kernels in any case, without a turn (for
+// solvers, which have the plan to themselves)
 int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2,
                     const int *d_skip, cudaStream_t st, bool fp32 = false);
 int back_project(const Plan *p, const float *d_s, float *d_g, double *d_norm2,

@@ -161,7 +161,7 @@ int forward_project(const Plan *p, const float *d_x, float *d_q, double *d_norm2
     const size_t nq = sin_floats(p);
     Turn turn;
     int rc = 0;
-    if (mma || d_norm2 || (A.taps && p->ngroups_o[1])) rc = turn.begin(p, 0, st);
+    if (mma || (!fp32 && (d_norm2 || (A.taps && p->ngroups_o[1])))) rc = turn.begin(p, 0, st);
     if (!rc) rc = timing_mark(p, true, false, st);
     if (rc) return rc;
     if (p->weighting == ARECGB_LIN) {
@@ -237,7 +237,7 @@ int back_project(const Plan *p, const float *d_s, float *d_g, double *d_norm2,
         mma = op.half != nullptr;
     }
     Turn turn;
-    if (mma || d_norm2)
+    if (mma || (!fp32 && d_norm2))
         if (int rc = turn.begin(p, 1, st)) return rc;
     if (mma) {
         int rc = timing_mark(p, false, false, st);
